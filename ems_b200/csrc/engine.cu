@@ -85,7 +85,8 @@ struct ems_gpu {
     float* co[12] = {};
     double* partials = nullptr;   // energy partial sums per block
     size_t n_partials = 0;
-    double* d_energy = nullptr;   // [0] field part, [1] operator part
+    double* d_energy = nullptr;   // [0] field part, [1 + q] the q-th operator that holds energy
+    double* shares = nullptr;     // first pass of a long sum (kSumBlocks)
     int* diverged = nullptr;      // set on the device where a marching step writes a non-finite value
     uint64_t test_wait_ns = 0;    // ems_gpu_test_wait_timeout: the next marching step's waits run out
     struct CpmlDev {
@@ -401,6 +402,18 @@ ems_status make_side(ems_gpu* h, const ems_pole_side& t, PoleSideDev& d) {
 }
 
 unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
+
+// Sums n energy shares into *out: one block up to 16384 of them (16 loads per
+// thread), two passes beyond. The caller counts the last launch.
+void sum_shares(ems_gpu* h, const double* partials, size_t n, double* out) {
+    if (n > 16384) {
+        k_sum_shares<<<kSumBlocks, kSumThreads, 0, h->stream>>>(partials, n, h->shares);
+        ++h->launches;
+        partials = h->shares;
+        n = kSumBlocks;
+    }
+    k_reduce_partials<<<1, 1024, 0, h->stream>>>(partials, n, out);
+}
 
 // Fused kernel instances: rows per tile × the thread bound of the launch.
 template <int TJ, int MAXT>
@@ -722,7 +735,7 @@ ems_status run_step_fused(ems_gpu* h, bool energy) {
     h->prof_end(2, ev);
     h->launches += 2;
     if (energy) {
-        k_reduce_partials<<<1, 1024, 0, s>>>(h->fpartials, h->fused_grid, h->d_energy);
+        sum_shares(h, h->fpartials, h->fused_grid, h->d_energy);
         ++h->launches;
     }
     for (int a = 0; a < 3; ++a) {
@@ -765,7 +778,7 @@ ems_status run_step_two(ems_gpu* h, bool energy) {
     h->prof_end(0, ev);
     ++h->launches;
     if (energy) {
-        k_reduce_partials<<<1, 1024, 0, s>>>(h->spartials, h->n_spartials, h->d_energy);
+        sum_shares(h, h->spartials, h->n_spartials, h->d_energy);
         ++h->launches;
     }
     ems_status st = serial_post_h(h, f);
@@ -877,7 +890,7 @@ ems_status run_step_sweep(ems_gpu* h, bool energy) {
             if (pf) { pole(0, ch); shell(1, ch); } else { shell(1, ch); pole(0, ch); }
         }
         if (energy) {
-            k_reduce_partials<<<1, 1024, 0, s>>>(h->qpartials, h->n_qpartials, h->d_energy);
+            sum_shares(h, h->qpartials, h->n_qpartials, h->d_energy);
             ++h->launches;
         }
         if (check(h, cudaStreamEndCapture(s, &graph), "sweep capture")) return EMS_ERR_CUDA;
@@ -1307,9 +1320,9 @@ ems_status run_step(ems_gpu* h, bool energy) {
     ++h->launches;
     if (energy) {
         if (split) {
-            k_reduce_partials<<<1, 1024, 0, s>>>(h->qpartials, h->n_qpartials, h->d_energy);
+            sum_shares(h, h->qpartials, h->n_qpartials, h->d_energy);
         } else {
-            k_reduce_partials<<<1, 1024, 0, s>>>(h->partials, h->n_partials, h->d_energy);
+            sum_shares(h, h->partials, h->n_partials, h->d_energy);
         }
         ++h->launches;
     }
@@ -1659,9 +1672,10 @@ ems_status ems_gpu_create(const ems_engine_desc* d, int device, ems_gpu** out) {
     }
     h->n_partials = (size_t)blocks_for(g.nz, kRowThreads) * g.ny * g.nx;
     h->partials = h->alloc<double>(h->n_partials);
-    h->d_energy = h->alloc<double>(2);
+    h->d_energy = h->alloc<double>(1 + d->n_ops);
+    h->shares = h->alloc<double>(kSumBlocks);
     h->diverged = h->alloc<int>(1);
-    if (!h->partials || !h->d_energy || !h->diverged) return EMS_ERR_NOMEM;
+    if (!h->partials || !h->d_energy || !h->shares || !h->diverged) return EMS_ERR_NOMEM;
     if (check(h.get(), cudaMemsetAsync(h->diverged, 0, sizeof(int), h->stream), "divergence flag")) return EMS_ERR_CUDA;
     for (size_t k = 0; k < d->n_ops; ++k) {
         ems_gpu::Op op;
@@ -2263,37 +2277,37 @@ static ems_status device_status(ems_gpu* h) {
 ems_status ems_gpu_step_with_energy(ems_gpu* h, double* energy) {
     if (!h || !energy) return EMS_ERR_INVALID;
     cudaSetDevice(h->device);
-    // Operator energies of the state before the step (src/engine/mod.rs:819-823).
-    double w_ops = 0.0;
+    // Operator energies of the state before the step (src/engine/mod.rs:819-823),
+    // read back with the field part after it.
+    size_t n_ops = 0;
     for (auto& op : h->ops) {
-        double x = 0.0;
+        double* at = h->d_energy + 1 + n_ops;
         if (op.kind == EMS_OP_POLES) {
-            k_pole_energy<<<1, 1024, 0, h->stream>>>(op.poles.e, op.poles.h, h->d_energy + 1);
+            k_pole_energy<<<kSumBlocks, kSumThreads, 0, h->stream>>>(op.poles.e, op.poles.h, h->shares);
             ++h->launches;
+            sum_shares(h, h->shares, kSumBlocks, at);
         } else if (op.kind == EMS_OP_LUMPED && op.lumped.has_branch) {
-            k_branch_energy<<<1, 1, 0, h->stream>>>(op.lumped.d, h->dt, h->d_energy + 1);
-            ++h->launches;
+            k_branch_energy<<<1, 1, 0, h->stream>>>(op.lumped.d, h->dt, at);
         } else if (op.kind == EMS_OP_MUR && op.mur_energy) {
-            k_mur_energy<<<1, 1024, 0, h->stream>>>(op.mur, h->d_energy + 1);
-            ++h->launches;
+            k_mur_energy<<<1, 1024, 0, h->stream>>>(op.mur, at);
         } else if (op.kind == EMS_OP_SHEET && op.sheet.n_edges) {
-            k_sheet_energy<<<1, 1024, 0, h->stream>>>(op.sheet, h->dt, h->d_energy + 1);
-            ++h->launches;
+            k_sheet_energy<<<1, 1024, 0, h->stream>>>(op.sheet, h->dt, at);
         } else {
             continue;
         }
-        if (check(h, cudaMemcpyAsync(&x, h->d_energy + 1, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "energy"))
-            return EMS_ERR_CUDA;
-        if (check(h, cudaStreamSynchronize(h->stream), "energy")) return EMS_ERR_CUDA;
-        w_ops += x;
+        ++h->launches;
+        ++n_ops;
     }
     ems_status st = step_dumped(h, true);
     if (st) return st;
-    double w = 0.0;
-    if (check(h, cudaMemcpyAsync(&w, h->d_energy, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "energy"))
+    std::vector<double> w(1 + n_ops);
+    if (check(h, cudaMemcpyAsync(w.data(), h->d_energy, w.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
+              "energy"))
         return EMS_ERR_CUDA;
     if (check(h, cudaStreamSynchronize(h->stream), "energy")) return EMS_ERR_CUDA;
-    *energy = 0.25 * h->dt * w + w_ops;
+    double w_ops = 0.0;
+    for (size_t q = 0; q < n_ops; ++q) w_ops += w[1 + q];
+    *energy = 0.25 * h->dt * w[0] + w_ops;
     return device_status(h);
 }
 

@@ -144,6 +144,19 @@ __global__ void __launch_bounds__(1024) k_reduce_partials(const double* partials
     if (threadIdx.x == 0) out[0] = t;
 }
 
+// Blocks of a large energy sum: the first pass leaves one share per block.
+constexpr unsigned kSumBlocks = 1184, kSumThreads = 256;
+
+// First pass of a long sum of shares (k_reduce_partials over its output ends
+// it): one block takes 160 us for the 280 000 shares of a 512^3 grid.
+__global__ void __launch_bounds__(kSumThreads) k_sum_shares(const double* partials, size_t n, double* out) {
+    double s = 0.0;
+    for (size_t q = (size_t)blockIdx.x * kSumThreads + threadIdx.x; q < n; q += (size_t)gridDim.x * kSumThreads)
+        s = __dadd_rn(s, partials[q]);
+    const double t = block_sum<kSumThreads>(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = t;
+}
+
 // E update of every edge (src/engine/kernel.rs:624-697); OE: openEMS's
 // summation order.
 template <bool OE = false>
@@ -406,19 +419,22 @@ __device__ __forceinline__ double pole_energy_block(const PoleSideDev& e, const 
     return block_sum<THREADS>(s);
 }
 
-__global__ void __launch_bounds__(1024) k_pole_energy(PoleSideDev e, PoleSideDev h, double* out) {
+// The poles' energy, one share per block (k_reduce_partials ends it): the
+// state is read once, 33 bytes per pole, by the whole chip.
+__global__ void __launch_bounds__(kSumThreads) k_pole_energy(PoleSideDev e, PoleSideDev h, double* out) {
     double s = 0.0;
     for (int side = 0; side < 2; ++side) {
         const PoleSideDev& p = side == 0 ? e : h;
-        for (size_t q = threadIdx.x; q < p.n_poles; q += blockDim.x) {
-            if (p.kind[q] >= 2) continue;  // openEMS's poles hold no energy
-            const double a = __dmul_rn(__dmul_rn(p.half_l[q], p.j[q]), p.j[q]);
-            const double b = __dmul_rn(__dmul_rn(__dmul_rn(0.5, p.inv_c[q]), p.q[q]), p.q[q]);
-            s = __dadd_rn(s, __dadd_rn(a, b));
+        for (size_t q = (size_t)blockIdx.x * kSumThreads + threadIdx.x; q < p.n_poles;
+             q += (size_t)gridDim.x * kSumThreads) {
+            const double l = p.half_l[q], j = p.j[q], c = p.inv_c[q], x = p.q[q];
+            const double a = __dmul_rn(__dmul_rn(l, j), j);
+            const double b = __dmul_rn(__dmul_rn(__dmul_rn(0.5, c), x), x);
+            if (p.kind[q] < 2) s = __dadd_rn(s, __dadd_rn(a, b));  // openEMS's poles hold no energy
         }
     }
-    const double t = block_sum<1024>(s);
-    if (threadIdx.x == 0) out[0] = t;
+    const double t = block_sum<kSumThreads>(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // Σ ½·L_e·j² + ½·q²/C_e of a lumped branch (src/engine/lumped.rs:1066-1077).
