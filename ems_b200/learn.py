@@ -20,10 +20,13 @@ Layers (channels-last activations, weights W[out][fan_in]):
     dense 64→2·T_OUT                       (V then I)
 
 about 0.38 M parameters. Every layer runs on the kernels of
-libems_learn.so (include/ems_learn.h): im2col, the bf16 tcgen05
-tensor-core GEMM (f32 accumulator in tensor memory), bias + activation, their adjoints, MSE and Adam; the
-f32 master weights are copied to bf16 for the GEMMs. torch only holds the
-device buffers and the stream.
+libems_learn.so (include/ems_learn.h): the bf16 tcgen05 tensor-core GEMM
+(f32 accumulator in tensor memory; a convolution's rows read in place from
+its channels-last input, bias and activation in the epilogue), the
+activations' adjoints with the bias gradients, MSE and Adam; the f32 master
+weights are copied to bf16 for the GEMMs. A pass is a list of launches built
+once per batch size and issued by one call. torch only holds the device
+buffers and the stream.
 """
 from __future__ import annotations
 
@@ -43,6 +46,16 @@ STRIDE = 16      # spacing of the predicted samples, in DT_REF (102.4 ps; 39 ns 
 WINDOW = 4 * STRIDE  # verification window after the input, in DT_REF
 CONVS = [(2, 32, 8, 4), (32, 64, 8, 4), (64, 128, 8, 4)]  # (c_in, c_out, kernel, stride)
 HIDDEN = 64
+
+TO_BF16, GEMM, DY, MSE = 0, 1, 2, 3  # kinds of Cmd
+WS_FLOATS = 4 << 20  # workspace of the split GEMMs (shares of the largest gradient: 0.5 M floats)
+
+
+class Cmd(C.Structure):
+    """``ems_learn_cmd``: one launch of a pass."""
+
+    _fields_ = [("kind", C.c_int32), ("i", C.c_int32 * 7), ("s", C.c_int64 * 8), ("p", C.c_void_p * 7)]
+
 
 _lib = None
 
@@ -66,6 +79,7 @@ def learn_lib() -> C.CDLL:
             "ems_learn_bias_grad": [p, p, i, i, p],
             "ems_learn_mse": [p, p, p, p, sz, p],
             "ems_learn_adam": [p, p, p, p, p, sz, f, f, f, f, i, p],
+            "ems_learn_run": [p, sz, p],
             "ems_learn_check": [],
         }
         for name, args in sig.items():
@@ -137,6 +151,8 @@ class Net:
         self.W = param_views(self.p, k_in, t_out)
         self.Wb = param_views(self.pb, k_in, t_out)
         self.G = param_views(self.g, k_in, t_out)
+        self.shares = []  # shares of the bias gradients
+        self.ws = torch.empty(WS_FLOATS, dtype=torch.float32, device=self.dev)
         self._buf_b = -1
 
     # -- plumbing
@@ -151,106 +167,104 @@ class Net:
         if st != 0:
             raise RuntimeError(f"ems_learn call failed ({st})")
 
-    def _gemm(self, A, sa0, sa1, B, sb0, sb1, Cm, ldc, M, N, K, beta=0.0):
-        self._ck(self.lib.ems_learn_gemm_bf16(A, sa0, sa1, B, sb0, sb1, Cm, ldc, M, N, K, 1.0, beta, self._s()))
+    def _cmd(self, kind, i=(), s=(), p=()):
+        """A launch of a pass; p: tensors (None: null)."""
+        c = Cmd(kind)
+        for q, v in enumerate(i):
+            c.i[q] = v
+        for q, v in enumerate(s):
+            c.s[q] = v
+        for q, t in enumerate(p):
+            c.p[q] = None if t is None else t.data_ptr()
+        return c
+
+    def _gemm(self, A, sa, B, sb, M, N, K, C=None, ldc=None, bias=None, act=0, outb=None, outf=None, rows_a=None,
+              rows_b=None):
+        """C (or act(C + bias)) = A·B; sa, sb: strides of (i, k) and (k, j); rows_a, rows_b: (inner count, outer
+        stride) of a two-level row index."""
+        pa, ba = rows_a or (0, 0)
+        pb, bb = rows_b or (0, 0)
+        return self._cmd(GEMM, (M, N, K, act, pa, pb), (*sa, *sb, N if ldc is None else ldc, ba, bb, WS_FLOATS),
+                         (A, B, C, bias, outb, outf, self.ws))
+
+    def _dy(self, y, da, dyb, db, rows, cols, act, conv=None):
+        """bf16(da·act'(y)) and the bias gradient; conv (T, k, s): da through the adjoint of im2col."""
+        per = 16 * max(1, 256 // cols)  # 16 rows per thread of a block
+        T, k, st = conv or (0, 0, 0)
+        n = (rows + per - 1) // per * cols
+        self.shares.append(self.torch.empty(n, dtype=self.torch.float32, device=self.dev))
+        return self._cmd(DY, (rows, cols, act, T, k, st, per), (), (y, da, dyb, self.shares[-1], db))
 
     def _bufs(self, B: int):
-        """Activation buffers for batch size B."""
+        """Activation buffers and the launch lists for batch size B."""
         if self._buf_b == B:
             return
         t = self.torch
         f32, bf = dict(dtype=t.float32, device=self.dev), dict(dtype=t.int16, device=self.dev)
-        self.cols, self.ys, self.acts, self.dys, self.dcols, self.das = [], [], [], [], [], []
-        for q, (ci, co, k, s) in enumerate(CONVS):
-            rows = B * self.T[q + 1]
-            self.cols.append(t.empty(rows * k * ci, **bf))
-            self.ys.append(t.empty(rows * co, **f32))
-            self.acts.append(t.empty(rows * co, **f32))
-            self.dys.append(t.empty(rows * co, **f32))
-            self.dcols.append(t.empty(rows * k * ci, **f32))
-            self.das.append(t.empty(B * self.T[q] * ci, **f32))
-        flat = self.shapes[3][2]
-        self.flat_b = t.empty(B * flat, **bf)
-        self.y4 = t.empty(B * HIDDEN, **f32)
-        self.a4 = t.empty(B * HIDDEN, **f32)
-        self.a4_b = t.empty(B * HIDDEN, **bf)
-        self.y5 = t.empty(B * 2 * self.t_out, **f32)
-        self.out = t.empty(B * 2 * self.t_out, **f32)
-        self.dy5 = t.empty(B * 2 * self.t_out, **f32)
-        self.dy5_b = t.empty(B * 2 * self.t_out, **bf)
-        self.da4 = t.empty(B * HIDDEN, **f32)
-        self.dy4 = t.empty(B * HIDDEN, **f32)
-        self.dy4_b = t.empty(B * HIDDEN, **bf)
-        self.da3 = t.empty(B * flat, **f32)
-        self.dy_b = [t.empty(B * self.T[q + 1] * CONVS[q][1], **bf) for q in range(len(CONVS))]
-        self.loss = t.zeros(1, **f32)
+        T, flat, no = self.T, self.shapes[3][2], 2 * self.t_out
+        rows = [B * T[q + 1] for q in range(3)]
+        self.shares = []
+        # The layers' bf16 inputs, pre-activations and the bf16 gradients of these.
+        self.xb = [t.empty(B * T[0] * 2, **bf)] + [t.empty(rows[q] * CONVS[q][1], **bf) for q in range(3)]
+        self.ys = [t.empty(rows[q] * CONVS[q][1], **f32) for q in range(3)]
+        self.dyb = [t.empty(rows[q] * CONVS[q][1], **bf) for q in range(3)]
+        self.dcols = [None] + [t.empty(rows[q] * CONVS[q][2] * CONVS[q][0], **f32) for q in (1, 2)]
+        self.y4, self.a4_b, self.out = t.empty(B * HIDDEN, **f32), t.empty(B * HIDDEN, **bf), t.empty(B * no, **f32)
+        self.dy5_b, self.da4 = t.empty(B * no, **bf), t.empty(B * HIDDEN, **f32)
+        self.dy4_b, self.da3 = t.empty(B * HIDDEN, **bf), t.empty(B * flat, **f32)
+        self.grad = t.empty(B * no, **f32)
+        self.loss, self.loss_shares = t.zeros(1, **f32), t.empty(64, **f32)
+
+        fwd = [self._cmd(TO_BF16, s=(B * T[0] * 2,), p=(None, self.xb[0]))]
+        for q, (ci, co, k, st) in enumerate(CONVS):
+            fwd.append(self._gemm(self.xb[q], (st * ci, 1), self.Wb[q][0], (1, k * ci), rows[q], co, k * ci, self.ys[q],
+                                  bias=self.W[q][1], act=1, outb=self.xb[q + 1], rows_a=(T[q + 1], T[q] * ci)))
+        fwd.append(self._gemm(self.xb[3], (flat, 1), self.Wb[3][0], (1, flat), B, HIDDEN, flat, self.y4,
+                              bias=self.W[3][1], act=1, outb=self.a4_b))
+        fwd.append(self._gemm(self.a4_b, (HIDDEN, 1), self.Wb[4][0], (1, HIDDEN), B, no, HIDDEN, bias=self.W[4][1],
+                              outf=self.out))
+
+        # fc2 (identity activation): dW5 = dy5ᵀ a4, db5, da4 = dy5 W5; fc1; the convolutions, last to first.
+        bwd = [self._dy(None, None, self.dy5_b, self.G[4][1], B, no, 0),
+               self._gemm(self.dy5_b, (1, no), self.a4_b, (HIDDEN, 1), no, HIDDEN, B, self.G[4][0]),
+               self._gemm(self.dy5_b, (no, 1), self.Wb[4][0], (HIDDEN, 1), B, HIDDEN, no, self.da4),
+               self._dy(self.y4, self.da4, self.dy4_b, self.G[3][1], B, HIDDEN, 1),
+               self._gemm(self.dy4_b, (1, HIDDEN), self.xb[3], (flat, 1), HIDDEN, flat, B, self.G[3][0]),
+               self._gemm(self.dy4_b, (HIDDEN, 1), self.Wb[3][0], (flat, 1), B, flat, HIDDEN, self.da3)]
+        da, conv = self.da3, None
+        for q in range(len(CONVS) - 1, -1, -1):
+            ci, co, k, st = CONVS[q]
+            bwd.append(self._dy(self.ys[q], da, self.dyb[q], self.G[q][1], rows[q], co, 1, conv))
+            bwd.append(self._gemm(self.dyb[q], (1, co), self.xb[q], (st * ci, 1), co, k * ci, rows[q], self.G[q][0],
+                                  rows_b=(T[q + 1], T[q] * ci)))
+            if q:
+                bwd.append(self._gemm(self.dyb[q], (co, 1), self.Wb[q][0], (k * ci, 1), rows[q], k * ci, co,
+                                      self.dcols[q]))
+                da, conv = self.dcols[q], (T[q], k, st)
+        mse = self._cmd(MSE, s=(B * no,), p=(self.out, None, self.grad, self.loss, self.loss_shares))
+        self._fwd = (Cmd * len(fwd))(*fwd)
+        self._mse = (Cmd * 1)(mse)
+        self._bwd = (Cmd * len(bwd))(*bwd)
         self._buf_b = B
+
+    def _run(self, cmds) -> None:
+        self._ck(self.lib.ems_learn_run(cmds, len(cmds), self._s()))
 
     # -- forward / backward
     def forward(self, x):
         """x: (B, k_in, 2) f32 on the device → (B, 2·t_out)."""
         B = x.shape[0]
         self._bufs(B)
-        L, s = self.lib, self._s()
-        inp = x.contiguous()
-        for q, (ci, co, k, st) in enumerate(CONVS):
-            T = self.T[q]
-            rows, fi = B * self.T[q + 1], k * ci
-            self._ck(L.ems_learn_im2col(self._ptr(inp), self._ptr(self.cols[q]), B, T, ci, k, st, s))
-            Wb, _ = self.Wb[q]
-            self._gemm(self._ptr(self.cols[q]), fi, 1, self._ptr(Wb), 1, fi, self._ptr(self.ys[q]), co, rows, co, fi)
-            self._ck(L.ems_learn_bias_act(self._ptr(self.ys[q]), self._ptr(self.W[q][1]), self._ptr(self.acts[q]),
-                                          rows, co, 1, s))
-            inp = self.acts[q]
-        flat = self.shapes[3][2]
-        self._ck(L.ems_learn_to_bf16(self._ptr(inp), self._ptr(self.flat_b), B * flat, s))
-        self._gemm(self._ptr(self.flat_b), flat, 1, self._ptr(self.Wb[3][0]), 1, flat, self._ptr(self.y4), HIDDEN,
-                   B, HIDDEN, flat)
-        self._ck(L.ems_learn_bias_act(self._ptr(self.y4), self._ptr(self.W[3][1]), self._ptr(self.a4), B, HIDDEN, 1, s))
-        self._ck(L.ems_learn_to_bf16(self._ptr(self.a4), self._ptr(self.a4_b), B * HIDDEN, s))
-        no = 2 * self.t_out
-        self._gemm(self._ptr(self.a4_b), HIDDEN, 1, self._ptr(self.Wb[4][0]), 1, HIDDEN, self._ptr(self.y5), no, B,
-                   no, HIDDEN)
-        self._ck(L.ems_learn_bias_act(self._ptr(self.y5), self._ptr(self.W[4][1]), self._ptr(self.out), B, no, 0, s))
-        return self.out.view(B, no)
+        x = x.contiguous()
+        self._fwd[0].p[0] = x.data_ptr()
+        self._run(self._fwd)
+        return self.out.view(B, 2 * self.t_out)
 
     def backward(self, dout):
         """Gradients of the last forward's output dout (B, 2·t_out) → self.g."""
-        B = dout.shape[0]
-        L, s = self.lib, self._s()
-        no, flat = 2 * self.t_out, self.shapes[3][2]
-        # fc2 (identity activation): dW5 = dy5ᵀ a4, db5, da4 = dy5 W5.
-        self.dy5.copy_(dout.reshape(-1))
-        self._ck(L.ems_learn_to_bf16(self._ptr(self.dy5), self._ptr(self.dy5_b), B * no, s))
-        self._gemm(self._ptr(self.dy5_b), 1, no, self._ptr(self.a4_b), HIDDEN, 1, self._ptr(self.G[4][0]), HIDDEN, no,
-                   HIDDEN, B)
-        self._ck(L.ems_learn_bias_grad(self._ptr(self.dy5), self._ptr(self.G[4][1]), B, no, s))
-        self._gemm(self._ptr(self.dy5_b), no, 1, self._ptr(self.Wb[4][0]), HIDDEN, 1, self._ptr(self.da4), HIDDEN, B,
-                   HIDDEN, no)
-        # fc1.
-        self._ck(L.ems_learn_act_grad(self._ptr(self.y4), self._ptr(self.da4), self._ptr(self.dy4), B, HIDDEN, 1, s))
-        self._ck(L.ems_learn_to_bf16(self._ptr(self.dy4), self._ptr(self.dy4_b), B * HIDDEN, s))
-        self._gemm(self._ptr(self.dy4_b), 1, HIDDEN, self._ptr(self.flat_b), flat, 1, self._ptr(self.G[3][0]), flat,
-                   HIDDEN, flat, B)
-        self._ck(L.ems_learn_bias_grad(self._ptr(self.dy4), self._ptr(self.G[3][1]), B, HIDDEN, s))
-        self._gemm(self._ptr(self.dy4_b), HIDDEN, 1, self._ptr(self.Wb[3][0]), flat, 1, self._ptr(self.da3), flat, B,
-                   flat, HIDDEN)
-        # convolutions, last to first.
-        da = self.da3
-        for q in range(len(CONVS) - 1, -1, -1):
-            ci, co, k, st = CONVS[q]
-            rows, fi = B * self.T[q + 1], k * ci
-            self._ck(L.ems_learn_act_grad(self._ptr(self.ys[q]), self._ptr(da), self._ptr(self.dys[q]), rows, co, 1, s))
-            self._ck(L.ems_learn_to_bf16(self._ptr(self.dys[q]), self._ptr(self.dy_b[q]), rows * co, s))
-            self._gemm(self._ptr(self.dy_b[q]), 1, co, self._ptr(self.cols[q]), fi, 1, self._ptr(self.G[q][0]), fi, co,
-                       fi, rows)
-            self._ck(L.ems_learn_bias_grad(self._ptr(self.dys[q]), self._ptr(self.G[q][1]), rows, co, s))
-            if q == 0:
-                break
-            self._gemm(self._ptr(self.dy_b[q]), co, 1, self._ptr(self.Wb[q][0]), fi, 1, self._ptr(self.dcols[q]), fi,
-                       rows, fi, co)
-            self._ck(L.ems_learn_col2im(self._ptr(self.dcols[q]), self._ptr(self.das[q]), B, self.T[q], ci, k, st, s))
-            da = self.das[q]
+        dout = dout.to(self.torch.float32).contiguous()
+        self._bwd[0].p[1] = dout.data_ptr()
+        self._run(self._bwd)
 
     def adam(self, lr: float = 1e-3, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8) -> None:
         self.t += 1
@@ -259,11 +273,10 @@ class Net:
 
     def train_step(self, x, y, lr: float = 1e-3) -> float:
         """One Adam step on a minibatch; returns the loss (MSE)."""
-        out = self.forward(x)
-        grad = self.torch.empty_like(out)
-        self._ck(self.lib.ems_learn_mse(self._ptr(out), self._ptr(y), self._ptr(grad), self._ptr(self.loss),
-                                        out.numel(), self._s()))
-        self.backward(grad)
+        self.forward(x)
+        self._mse[0].p[1] = self._ptr(y)
+        self._run(self._mse)
+        self.backward(self.grad)
         self.adam(lr)
         return self.loss
 

@@ -33,6 +33,34 @@ extern "C" {
 int ems_learn_gemm_bf16(const uint16_t* A, int64_t sa0, int64_t sa1, const uint16_t* B, int64_t sb0, int64_t sb1,
                         float* C, int64_t ldc, int M, int N, int K, float alpha, float beta, void* stream);
 
+/* A list of launches issued by one call, in order on one stream: a network's
+ * pass is a fixed list per batch size, which a host builds once. Returns the
+ * first nonzero status. Per kind (s: 64-bit values, i: 32-bit, p: pointers):
+ *  TO_BF16  p src, dst; s n.
+ *  GEMM     C (p[2], row stride s[4]) = A (p[0]; strides s[0] of i, s[1] of k) x
+ *           B (p[1]; strides s[2] of k, s[3] of j), M N K in i[0..2]. With a
+ *           bias (p[3]): y = C + bias[j] is kept in p[2] (if not null) and
+ *           act(y) (i[3]: 0 identity, 1 SiLU) written as bf16 to p[4] and f32 to
+ *           p[5] (each if not null, row stride s[4]). i[4] > 0: A's row index is
+ *           two-level, r -> (r / i[4])*s[5] + (r mod i[4])*s[0]; i[5] > 0: the
+ *           same for B's k index with s[6] (the rows of a valid convolution of
+ *           x[b][T][c] with stride d: i = T_out, outer stride T*c, inner d*c).
+ *           p[6], s[7]: workspace of that many floats (16-byte aligned) for a
+ *           reduction split over the chip; NULL: not split.
+ *  DY       dy = da (p[1]) * act'(y (p[0])) (i[2] as above), bf16(dy) to p[2] and
+ *           its column sums to p[4]; rows i[0], cols i[1]. i[4] > 0: da is the
+ *           adjoint of im2col of p[1] (kernel i[4], stride i[5], T = i[3]; rows =
+ *           B*T). p[3]: ceil(rows / i[6]) * cols floats, i[6] rows per share.
+ *  MSE      as ems_learn_mse: p out, target, grad, loss, shares (64 floats); s n. */
+enum { EMS_LEARN_TO_BF16 = 0, EMS_LEARN_GEMM = 1, EMS_LEARN_DY = 2, EMS_LEARN_MSE = 3 };
+typedef struct {
+    int32_t kind;
+    int32_t i[7];
+    int64_t s[8];
+    void* p[7];
+} ems_learn_cmd;
+int ems_learn_run(const ems_learn_cmd* cmds, size_t n, void* stream);
+
 /* 0, or 4 (and clears the flag) if a GEMM's bounded wait for its tensor-core
  * work ran out since the last call; 2 if the flag cannot be read. */
 int ems_learn_check(void);
