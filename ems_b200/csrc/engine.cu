@@ -35,6 +35,7 @@
 #include "interior.cuh"
 #include "march.cuh"
 #include "batch.cuh"
+#include "resident.cuh"
 #include "sheet.cuh"
 
 #include <cudaTypedefs.h>
@@ -92,6 +93,13 @@ struct ems_gpu {
     struct CpmlDev {
         SlabDev s;
     };
+    // The device copy of a source's amplitudes (resident steps): `cap` values,
+    // zero beyond the host table; host entries [lo, hi) are not yet in it.
+    template <class T>
+    struct AmpDev {
+        T* p = nullptr;
+        size_t cap = 0, lo = 0, hi = 0;
+    };
     struct PoleDev {
         PoleSideDev e, h;
     };
@@ -101,6 +109,7 @@ struct ems_gpu {
         size_t n_edges = 0;
         size_t n_amp = 0;
         std::vector<double> amp;   // host copy of the source values (activity test)
+        AmpDev<double> amp_dev;
         bool has_src = false, record = false, has_branch = false;
         uint64_t columns = 0;
         size_t count = 0, cap = 0, vcap = 0, icap = 0;
@@ -115,6 +124,7 @@ struct ems_gpu {
         uint8_t* axis = nullptr;
         float* weight = nullptr;
         std::vector<float> amp;
+        AmpDev<float> amp_dev;
     };
     struct ProbeDev {
         ProbeDevT d;
@@ -188,12 +198,41 @@ struct ems_gpu {
     }
     // The split schedule: CPML layer shell segments per side (0 H, 1 E).
     ShellDev shell[2] = {};
+    bool cpml_first = false;  // a CPML, registered before every other slab operator
+    // Quads with and without CPML slabs per side (cpml_quads), made for
+    // resident steps.
+    const uint2* cpml_layer[2] = {};
+    const uint32_t* cpml_inner[2] = {};
+    uint32_t n_layer[2] = {};
     // The split schedule's row CPML (split.cuh row_cpml): every slab's
     // correction inside the update kernels' CPML variant over the quads that
     // hold layer nodes, no shell kernel; used when switched on
     // (ems_gpu_set_row_cpml) and the plan applies.
     RowCpml rowc;
     bool row_cpml_on = false;
+    // The serial hooks small enough for one block (resident.cuh ResOp), in
+    // registration order, and the newest samples mirrored in host memory.
+    struct Hooks {
+        ResOp* dev = nullptr;
+        std::vector<unsigned char> held;  // what the device table holds
+        std::vector<int> place;           // per operator its place, -1: not in the table
+        uint64_t ready = ~0ull;           // buffers and amplitudes hold the steps before this one
+        bool late_h = false;              // no hook writes i: current probes wait for the electric hooks
+        double* mail = nullptr;           // pinned, 3 per operator
+    } hooks;
+    // Resident steps (resident.cuh): the automatic schedule's form of the
+    // split schedule on small grids, many steps per launch.
+    struct Resident {
+        bool ok = false;
+        std::vector<unsigned char> model;  // what the device table holds
+        ResModel* d_model = nullptr;
+        uint4* blocks = nullptr;
+        uint2* gangs = nullptr;
+        uint32_t* list = nullptr;
+        uint32_t* bars = nullptr;  // two sets of one counter
+        int flip = 0;
+        unsigned grid = 0;
+    } res;
     // The sweep schedule: x chunks of sweep_planes planes, each chunk's
     // shell boxes (first box, first node) and pole edges (first edge) per
     // side; entry [chunks] closes the last range.
@@ -619,6 +658,7 @@ ems_status setup_fused(ems_gpu* h, const ems_engine_desc* d) {
         }
         const uint64_t nodes3[3] = {g.nx, g.ny, g.nz};
         h->rowc = (seen_cpml && cpml_first) ? row_cpml_plan(h->slab_geo, nodes3) : RowCpml{};
+        h->cpml_first = seen_cpml && cpml_first;
     }
     // The sweep needs no magnetic sources or conducting sheets (their serial
     // post_h hooks would sit between a chunk's H and E updates) and no
@@ -1216,8 +1256,6 @@ ems_status run_step_march(ems_gpu* h) {
     return EMS_OK;
 }
 
-// One step through the per-operator kernels; energy: record the
-// invariant's field part into d_energy[0].
 // One update of the split schedule with the row CPML (h->rowc): the CPML
 // variant of the update kernel over every quad that holds a layer node of
 // the side (the x-layer planes whole; in the other planes the y-layer rows
@@ -1261,6 +1299,356 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
     go(false, xl, mid, QuadMap{1u, 0u, yl, inner, 0u, zl, rows * inner});
 }
 
+// ---- Resident steps (resident.cuh).
+
+// Most bytes of fields, dense coefficients, CPML and pole state a resident
+// model touches per step, and most edges of a source (or lumped element) that
+// one block applies alone. Measured on cubes, us per step resident / split:
+// vacuum with CPML 40 cells 22/35, 96 37/50, 160 (110 MB) 106/123, 200 (230
+// MB) 187/216; coefficients of every node 160 (260 MB) 129/141, 240 370/364.
+// The poles' correction runs better in its own kernel (trapezoidal media 64
+// cells 28/46, 96 (27 MB) 55/64, 128 (70 MB) 121/115), and so does the
+// openEMS PML's at nearly every size (24 34/26, 64 28/33, 96 68/59).
+constexpr size_t kResidentBytes = 256u << 20, kResidentPoleBytes = 32u << 20;
+constexpr size_t kResidentEdges = 4096;
+constexpr uint64_t kResidentSteps = 4096;  // most steps per launch
+
+size_t resident_bytes(const ems_gpu* h) {
+    size_t b = 24 * h->g.np;
+    for (int l = 0; l < 12; ++l)
+        if (h->fp.lane[l].dense) b += 4 * h->g.np;
+    for (const auto& op : h->ops) {
+        for (const SlabDev& s : op.cpml)
+            b += 4 * (size_t)(s.hi[0] - s.lo[0]) * (s.hi[1] - s.lo[1]) * (s.hi[2] - s.lo[2]);
+        for (const PoleSideDev* p : {&op.poles.e, &op.poles.h}) b += 16 * p->n_poles + 21 * p->n_edges;
+    }
+    return b;
+}
+
+// Whether the model's operators can run resident: every hook one of those
+// resident.cuh runs, and the serial ones small enough for one block.
+bool resident_ops(const ems_gpu* h) {
+    if (!h->tables_ok) return false;
+    for (const auto& op : h->ops) {
+        if (op.kind == EMS_OP_MUR || op.kind == EMS_OP_SHEET || op.kind == EMS_OP_UPML) return false;
+        if (op.kind == EMS_OP_SOURCE && op.source.n > kResidentEdges) return false;
+        if (op.kind == EMS_OP_LUMPED && op.lumped.n_edges > kResidentEdges) return false;
+        if (op.kind == EMS_OP_PROBE && op.probe.interval >= (1ull << 31)) return false;
+    }
+    return true;
+}
+
+// The quad lists of a model whose CPML the resident updates apply.
+ems_status resident_quads(ems_gpu* h) {
+    if (!h->cpml_first || h->cpml_inner[0]) return EMS_OK;
+    const uint64_t nodes[3] = {h->g.nx, h->g.ny, h->g.nz};
+    for (int side = 0; side < 2; ++side) {
+        std::vector<uint2> layer;
+        std::vector<uint32_t> inner;
+        cpml_quads(h->slab_geo, nodes, side, layer, inner);
+        h->n_layer[side] = (uint32_t)layer.size();
+        h->cpml_layer[side] = h->upload(layer.data(), layer.size());
+        h->cpml_inner[side] = h->upload(inner.data(), inner.size());
+        if (!h->cpml_layer[side] || !h->cpml_inner[side]) return fail(h, EMS_ERR_NOMEM, "resident steps");
+        if (check(h, cudaStreamSynchronize(h->stream), "resident steps")) return EMS_ERR_CUDA;
+    }
+    return EMS_OK;
+}
+
+// Blocks of `threads` threads of the resident kernel that fit the device at
+// once; 0 without cooperative launches.
+unsigned resident_blocks(int device, int threads) {
+    int coop = 0, sms = 0, per = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resident<false>, threads, 0) != cudaSuccess)
+        return 0;
+    int oe = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oe, k_resident<true>, threads, 0) != cudaSuccess) return 0;
+    return (unsigned)(sms * std::min(per, oe));
+}
+
+// The model's tables for the resident kernel (all but its ops).
+void resident_model(ems_gpu* h, ResModel& R) {
+    const Grid& g = h->g;
+    BatchModel& M = R.m;
+    M.P = h->fp;
+    for (int a = 0; a < 3; ++a) {
+        M.P.uo[a] = M.P.un[a] = M.f.u[a] = h->u[a];
+        M.P.io[a] = M.P.in[a] = M.f.i[a] = h->i[a];
+    }
+    for (size_t q = 0; q < h->psi_h.size(); ++q) {
+        FSlab& fs = M.P.slab[0][h->psi_h_at[q].first][h->psi_h_at[q].second];
+        fs.psi_old = fs.psi_new = h->psi_h[q].first;
+    }
+    for (int l = 0; l < 12; ++l) M.c.c[l] = h->co[l];
+    int n = 0;
+    R.order[0] = R.order[1] = -1;
+    for (auto& op : h->ops) {
+        if (op.kind == EMS_OP_CPML) {
+            R.order[n++] = 0;
+        } else if (op.kind == EMS_OP_POLES) {
+            R.order[n++] = 1;
+            M.pe = op.poles.e;
+            M.ph = op.poles.h;
+        } else {
+            const bool h_side = (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)) ||
+                                (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_CURRENT);
+            if (!h_side) R.serial_e = 1;
+            else if (op.kind == EMS_OP_SOURCE) R.serial_h = 1;
+        }
+    }
+    for (int side = 0; side < 2; ++side) {
+        M.shell[side] = h->shell[side];
+        M.run_of[side] = h->run_of[side];
+        R.units[side] = shell_blocks(h->shell[side]);
+    }
+    // Electric hooks in order: writers, then probes.
+    bool seen_probe = false, late = false;
+    R.late_probes = 1;
+    for (auto& op : h->ops) {
+        const bool w = op.kind == EMS_OP_LUMPED || (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_E || op.source.kind == EMS_HARD_E));
+        if (w) R.writes_e = 1;
+        if (w && seen_probe) late = true;
+        if (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_VOLTAGE) seen_probe = true;
+    }
+    if (late || !seen_probe) R.late_probes = 0;
+    for (int side = 0; side < 2; ++side) {
+        R.layer[side] = h->cpml_layer[side];
+        R.inner[side] = h->cpml_inner[side];
+        R.n_layer[side] = h->n_layer[side];
+    }
+    R.quad_cpml = h->cpml_first;
+    M.dt = h->dt;
+    M.bx = split_blocks_x(g);
+    R.div_q = fast_div((g.nz + 3u) / 4u);
+    R.div_j = fast_div(g.ny);
+    R.quads = g.nx * g.ny * ((g.nz + 3u) / 4u);
+}
+
+// One of the operators as a serial hook; false if it is none.
+bool resident_op(const ems_gpu::Op& op, ResOp& o) {
+    if (op.kind == EMS_OP_SOURCE) {
+        const auto& s = op.source;
+        o.kind = ResOp::SOURCE;
+        o.electric = s.kind == EMS_SOFT_E || s.kind == EMS_HARD_E;
+        o.hard = s.kind == EMS_HARD_E || s.kind == EMS_HARD_H;
+        o.n = (uint32_t)s.n;
+        o.node = s.node;
+        o.axis = s.axis;
+        o.weight = s.weight;
+    } else if (op.kind == EMS_OP_PROBE) {
+        const auto& p = op.probe;
+        o.kind = ResOp::PROBE;
+        o.electric = p.quantity == EMS_PROBE_VOLTAGE;
+        o.probe = p.d;
+        o.interval = (uint32_t)std::min<uint64_t>(p.interval, ~0u);
+    } else if (op.kind == EMS_OP_LUMPED) {
+        const auto& l = op.lumped;
+        o.kind = ResOp::LUMPED;
+        o.electric = 1;
+        o.lumped = l.d;
+        o.axis_l = (uint32_t)l.axis;
+        o.has_src = l.has_src;
+    } else {
+        return false;
+    }
+    return true;
+}
+
+// Brings a source's device amplitudes up to date for steps [step, step + n).
+template <class T>
+ems_status sync_amp(ems_gpu* h, const std::vector<T>& amp, ems_gpu::AmpDev<T>& d, uint64_t step, uint64_t n) {
+    if (amp.size() > d.cap || !d.p) {
+        const size_t cap = std::max<size_t>(std::max<size_t>(amp.size(), 2 * d.cap), 16384);
+        T* p = h->alloc<T>(cap);
+        if (!p) return fail(h, EMS_ERR_NOMEM, "source amplitudes");
+        if (d.p) {
+            cudaStreamSynchronize(h->stream);
+            h->release(d.p);
+        }
+        d.p = p;
+        d.cap = cap;
+        d.lo = 0;
+        d.hi = amp.size();
+    }
+    d.hi = std::min(d.hi, amp.size());
+    if (d.lo >= d.hi || d.lo >= step + n || d.hi <= step) return EMS_OK;
+    if (check(h, cudaMemcpyAsync(d.p + d.lo, amp.data() + d.lo, (d.hi - d.lo) * sizeof(T), cudaMemcpyHostToDevice, h->stream),
+              "source amplitudes"))
+        return EMS_ERR_CUDA;
+    d.lo = d.hi = 0;
+    return EMS_OK;
+}
+
+// Uploads a host table if it differs from what the device holds.
+ems_status put_table(ems_gpu* h, std::vector<unsigned char>& held, void* dev, const void* host, size_t bytes) {
+    if (held.size() == bytes && !std::memcmp(held.data(), host, bytes)) return EMS_OK;
+    held.assign((const unsigned char*)host, (const unsigned char*)host + bytes);
+    return check(h, cudaMemcpyAsync(dev, held.data(), bytes, cudaMemcpyHostToDevice, h->stream), "resident tables");
+}
+
+// Makes the serial hooks ready for steps [step, step + n): room for their
+// samples (counted here), amplitudes on the device, and the table of hooks
+// uploaded again if a buffer has moved.
+ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
+    auto& k = h->hooks;
+    if (k.ready == h->step + n) return EMS_OK;
+    if (!k.mail && check(h, cudaHostAlloc((void**)&k.mail, (h->ops.size() + 1) * 3 * sizeof(double), cudaHostAllocMapped),
+                         "serial hooks"))
+        return EMS_ERR_CUDA;
+    bool moved = k.held.empty();
+    for (auto& op : h->ops) {
+        ems_status st = EMS_OK;
+        if (op.kind == EMS_OP_SOURCE && op.source.n <= kResidentEdges) {
+            const float* was = op.source.amp_dev.p;
+            st = sync_amp(h, op.source.amp, op.source.amp_dev, h->step, n);
+            moved |= was != op.source.amp_dev.p;
+        } else if (op.kind == EMS_OP_PROBE) {
+            auto& p = op.probe;
+            const uint64_t end = (h->step + n + p.interval - 1) / p.interval;
+            moved |= end > p.cap;
+            st = grow(h, &p.values, p.count, &p.cap, end);
+            p.count = end;
+        } else if (op.kind == EMS_OP_LUMPED) {
+            auto& l = op.lumped;
+            if (l.has_src) {
+                const double* was = l.amp_dev.p;
+                st = sync_amp(h, l.amp, l.amp_dev, h->step, n);
+                moved |= was != l.amp_dev.p;
+            }
+            if (!st && l.record) {
+                const uint64_t end = h->step + n;
+                moved |= end > l.cap;
+                st = grow(h, &l.rec, l.count, &l.cap, end);
+                if (!st && l.columns) st = grow(h, &l.pv, l.count, &l.vcap, end);
+                if (!st && l.columns) st = grow(h, &l.pi, l.count, &l.icap, end);
+                l.count = end;
+            }
+        }
+        if (st) return st;
+    }
+    k.ready = h->step + n;
+    if (!moved) return EMS_OK;
+    std::vector<unsigned char> ops;
+    for (size_t q = 0; q < h->ops.size(); ++q) {
+        if (k.place[q] < 0) continue;
+        auto& op = h->ops[q];
+        alignas(16) unsigned char raw[sizeof(ResOp)];
+        std::memset(raw, 0, sizeof raw);
+        ResOp& o = *new (raw) ResOp();
+        resident_op(op, o);
+        o.mail = k.mail + 3 * q;
+        if (op.kind == EMS_OP_SOURCE) {
+            o.amp = op.source.amp_dev.p;
+            o.n_amp = (uint32_t)op.source.amp_dev.cap;
+        } else if (op.kind == EMS_OP_PROBE) {
+            o.values = op.probe.values;
+            o.cap = (uint32_t)std::min<size_t>(op.probe.cap, ~0u);
+        } else {
+            const auto& l = op.lumped;
+            o.amp_l = l.amp_dev.p;
+            o.n_amp = (uint32_t)l.amp_dev.cap;
+            o.rec = l.record ? l.rec : nullptr;
+            o.pv = l.columns ? l.pv : nullptr;
+            o.pi = l.columns ? l.pi : nullptr;
+            o.cap = (uint32_t)std::min<size_t>(l.cap, ~0u);
+        }
+        ops.insert(ops.end(), raw, raw + sizeof(ResOp));
+    }
+    return ops.empty() ? EMS_OK : put_table(h, k.held, k.dev, ops.data(), ops.size());
+}
+
+void launch_resident(const ResArgs& A, bool oe, unsigned grid, unsigned threads, cudaStream_t s, cudaError_t* e) {
+    ResArgs a = A;
+    void* args[] = {&a};
+    *e = cudaLaunchCooperativeKernel(oe ? (const void*)k_resident<true> : (const void*)k_resident<false>, dim3(grid),
+                                     dim3(threads), args, 0, s);
+}
+
+// The table of the serial hooks one block can run (every probe; sources and
+// lumped elements of few edges), and the host mirror of the newest samples.
+ems_status setup_hooks(ems_gpu* h) {
+    auto& k = h->hooks;
+    int n = 0;
+    k.late_h = true;
+    for (const auto& op : h->ops) {
+        const bool fits = (op.kind == EMS_OP_SOURCE && op.source.n <= kResidentEdges) ||
+                          (op.kind == EMS_OP_LUMPED && op.lumped.n_edges <= kResidentEdges) ||
+                          op.kind == EMS_OP_PROBE;
+        k.place.push_back(fits ? n++ : -1);
+        if (op.kind == EMS_OP_SHEET || (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)))
+            k.late_h = false;
+    }
+    k.dev = h->alloc<ResOp>(n);
+    return k.dev ? EMS_OK : fail(h, EMS_ERR_NOMEM, "serial hooks");
+}
+
+// The engine's gang: as many blocks as there are quads for, at most those
+// that fit the device.
+ems_status setup_resident(ems_gpu* h) {
+    auto& r = h->res;
+    bool poles = false;
+    for (const auto& op : h->ops) poles |= op.poles.e.n_edges || op.poles.h.n_edges;
+    if (!resident_ops(h) || resident_bytes(h) > (poles ? kResidentPoleBytes : kResidentBytes)) return EMS_OK;
+    const unsigned fit = resident_blocks(h->device, kResThreads);
+    if (!fit) return EMS_OK;
+    const uint64_t quads = (uint64_t)h->g.nx * h->g.ny * ((h->g.nz + 3u) / 4u);
+    if (ems_status st = resident_quads(h)) return st;
+    r.grid = (unsigned)std::min<uint64_t>(fit, std::max<uint64_t>(1, (quads + kResThreads - 1) / kResThreads));
+    if (r.grid >= kHookGang) r.grid = std::min(fit, r.grid + 1u);  // one more for the hooks
+    std::vector<uint4> blocks(r.grid);
+    for (unsigned b = 0; b < r.grid; ++b) blocks[b] = uint4{0, b, r.grid, 0};
+    const uint2 gang{0, 1};
+    const uint32_t list = 0;
+    r.blocks = h->upload(blocks.data(), blocks.size());
+    r.gangs = h->upload(&gang, 1);
+    r.list = h->upload(&list, 1);
+    r.bars = h->alloc<uint32_t>(64);
+    r.d_model = h->alloc<ResModel>(1);
+    if (!h->status) h->status = h->alloc<int>(1);
+    if (!r.blocks || !r.gangs || !r.list || !r.bars || !r.d_model || !h->status)
+        return fail(h, EMS_ERR_NOMEM, "resident steps");
+    r.ok = true;
+    return check(h, cudaStreamSynchronize(h->stream), "resident steps");
+}
+
+// Whether the next steps (no energy, no dumps) run resident: the automatic
+// schedule, the plain step, and the step counter within the kernel's range.
+bool use_resident(const ems_gpu* h) {
+    return h->res.ok && h->schedule == 0 && !h->row_cpml_on && !h->profiling && !h->tune.active && h->dumps.empty() &&
+           h->tdumps.empty() && h->step < (1ull << 30);
+}
+
+ems_status run_resident(ems_gpu* h, uint64_t n) {
+    auto& r = h->res;
+    alignas(16) unsigned char raw[sizeof(ResModel)];
+    std::memset(raw, 0, sizeof raw);
+    ResModel& R = *new (raw) ResModel();
+    resident_model(h, R);
+    R.fold_e = h->fold_prev[0];
+    R.fold_h = h->fold_prev[1];
+    R.capture_first = !h->prev_e_valid;
+    ems_status st = prepare_hooks(h, n);
+    if (st) return st;
+    R.ops = h->hooks.dev;
+    R.n_ops = (uint32_t)(h->hooks.held.size() / sizeof(ResOp));
+    st = put_table(h, r.model, r.d_model, raw, sizeof raw);
+    if (st) return st;
+    ResArgs A{r.d_model, r.blocks, r.gangs, r.list, r.bars + 32 * r.flip, r.bars + 32 * (r.flip ^ 1), 1u, (uint32_t)n,
+              (uint32_t)h->step, nullptr, h->status, kWaitNs};
+    r.flip ^= 1;
+    cudaError_t e;
+    launch_resident(A, h->oe_curl, r.grid, kResThreads, h->stream, &e);
+    if (check(h, e, "resident steps")) return EMS_ERR_CUDA;
+    ++h->launches;
+    h->step += n;
+    h->prev_e_valid = h->fold_prev[0];
+    return EMS_OK;
+}
+
+// One step through the per-operator or split kernels; energy: record the
+// invariant's field part into d_energy[0].
 ems_status run_step(ems_gpu* h, bool energy) {
     const int sch = active_schedule(h);
     // Only the per-operator, split and sweep steps keep the electric saved values.
@@ -1530,45 +1918,84 @@ ems_status setup_sheet(ems_gpu* h, const ems_sheet* t, ems_gpu::Op& op) {
     return EMS_OK;
 }
 
+// Runs the pending hooks [lo, hi) of the table, if any acts in this step:
+// sides bit 0 the magnetic ones, bit 1 the electric ones.
+void run_hooks(ems_gpu* h, const Fields& f, int& lo, int hi, int sides, bool& acts) {
+    if (acts && hi > lo) {
+        k_hooks<<<1, 256, 0, h->stream>>>(f, h->dt, h->hooks.dev + lo, (uint32_t)(hi - lo), (uint32_t)h->step, sides);
+        ++h->launches;
+    }
+    lo = hi;
+    acts = false;
+}
+
+// Whether a hook of the table has something to do in this step.
+bool hook_acts(const ems_gpu* h, const ems_gpu::Op& op) {
+    if (op.kind == EMS_OP_PROBE) return h->step % op.probe.interval == 0;
+    if (op.kind != EMS_OP_SOURCE) return true;
+    const auto& s = op.source;
+    return s.kind == EMS_HARD_E || s.kind == EMS_HARD_H || (h->step < s.amp.size() && s.amp[h->step] != 0.0f);
+}
+
+void run_source(ems_gpu* h, const ems_gpu::SourceDev& sd, float* const F[3]) {
+    const float a = h->step < sd.amp.size() ? sd.amp[h->step] : 0.0f;
+    const bool hard = sd.kind == EMS_HARD_E || sd.kind == EMS_HARD_H;
+    if (!hard && a == 0.0f) return;
+    k_source<<<blocks_for(sd.n, 256), 256, 0, h->stream>>>(F[0], F[1], F[2], sd.axis, sd.node, sd.weight, sd.n, a, hard);
+    ++h->launches;
+}
+
 // Serial post_h hooks in registration order: magnetic sources, conducting
-// sheets, current probes.
+// sheets, current probes. Where no hook writes i the probes are left to
+// serial_post_e (i does not change before it).
 ems_status serial_post_h(ems_gpu* h, const Fields& f) {
-    cudaStream_t s = h->stream;
-    for (auto& op : h->ops) {
-        if (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)) {
-            const ems_gpu::SourceDev& sd = op.source;
-            float a = h->step < sd.amp.size() ? sd.amp[h->step] : 0.0f;
-            bool hard = sd.kind == EMS_HARD_H;
-            if (!hard && a == 0.0f) continue;
-            k_source<<<blocks_for(sd.n, 256), 256, 0, s>>>(f.i[0], f.i[1], f.i[2], sd.axis, sd.node, sd.weight, sd.n, a, hard);
-            ++h->launches;
+    if (ems_status st = prepare_hooks(h, 1)) return st;
+    if (h->hooks.late_h) return EMS_OK;
+    int lo = 0, hi = 0;
+    bool acts = false;
+    for (size_t q = 0; q < h->ops.size(); ++q) {
+        auto& op = h->ops[q];
+        const bool mine = (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)) ||
+                          (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_CURRENT);
+        if (h->hooks.place[q] >= 0) {
+            hi = h->hooks.place[q] + 1;
+            acts |= mine && hook_acts(h, op);
+        } else if (mine) {
+            run_hooks(h, f, lo, hi, 1, acts);
+            run_source(h, op.source, f.i);
         } else if (op.kind == EMS_OP_SHEET && op.sheet.n_edges) {
+            run_hooks(h, f, lo, hi, 1, acts);
             const SheetDevT& sd = op.sheet;
-            k_sheet_post_h<<<blocks_for(sd.n_targets + sd.n_edges, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], f.i[0],
-                                                                                      f.i[1], f.i[2], sd);
+            k_sheet_post_h<<<blocks_for(sd.n_targets + sd.n_edges, 256), 256, 0, h->stream>>>(f.u[0], f.u[1], f.u[2], f.i[0],
+                                                                                              f.i[1], f.i[2], sd);
             ++h->launches;
-        } else if (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_CURRENT && h->step % op.probe.interval == 0) {
-            ems_gpu::ProbeDev& p = op.probe;
-            ems_status st = grow(h, &p.values, p.count, &p.cap, p.count + 1);
-            if (st) return st;
-            k_probe<<<1, 32, 0, s>>>(f.i[0], f.i[1], f.i[2], p.d, p.values + p.count);
-            ++h->launches;
-            ++p.count;
         }
     }
+    run_hooks(h, f, lo, hi, 1, acts);
     return EMS_OK;
 }
 
 // pre_e: lumped elements and Mur boundaries save u^n.
 ems_status serial_pre_e(ems_gpu* h, const Fields& f) {
-    for (auto& op : h->ops) {
+    if (ems_status st = prepare_hooks(h, 1)) return st;
+    bool acts = false;
+    for (size_t q = 0; q < h->ops.size(); ++q) {
+        auto& op = h->ops[q];
         if (op.kind == EMS_OP_LUMPED && (op.lumped.record || op.lumped.has_branch)) {
+            if (h->hooks.place[q] >= 0) {
+                acts = true;
+                continue;
+            }
             k_lumped_pre_e<<<blocks_for(op.lumped.n_edges, 128), 128, 0, h->stream>>>(f.u[op.lumped.axis], op.lumped.d);
             ++h->launches;
         } else if (op.kind == EMS_OP_MUR && op.mur.n) {
             k_mur_save<<<blocks_for(op.mur.n, 256), 256, 0, h->stream>>>(f.u[0], f.u[1], f.u[2], op.mur);
             ++h->launches;
         }
+    }
+    if (acts) {
+        k_hooks_pre<<<1, 256, 0, h->stream>>>(f, h->hooks.dev, (uint32_t)(h->hooks.held.size() / sizeof(ResOp)));
+        ++h->launches;
     }
     return EMS_OK;
 }
@@ -1577,8 +2004,19 @@ ems_status serial_pre_e(ems_gpu* h, const Fields& f) {
 // boundaries, electric sources, conducting sheets, voltage probes.
 ems_status serial_post_e(ems_gpu* h, const Fields& f) {
     cudaStream_t s = h->stream;
-    for (auto& op : h->ops) {
-        if (op.kind == EMS_OP_MUR) {
+    if (ems_status st = prepare_hooks(h, 1)) return st;
+    int lo = 0, hi = 0;
+    bool acts = false;
+    const int sides = h->hooks.late_h ? 3 : 2;
+    for (size_t q = 0; q < h->ops.size(); ++q) {
+        auto& op = h->ops[q];
+        const bool h_side = (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)) ||
+                            (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_CURRENT);
+        if (h->hooks.place[q] >= 0) {
+            hi = h->hooks.place[q] + 1;
+            acts |= (!h_side || h->hooks.late_h) && hook_acts(h, op);
+        } else if (op.kind == EMS_OP_MUR) {
+            run_hooks(h, f, lo, hi, sides, acts);
             const MurDevT& m = op.mur;
             if (m.n_edges) {
                 k_mur_update<<<blocks_for(m.n_edges, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], m, h->step, 0u, m.n_edges);
@@ -1590,45 +2028,25 @@ ems_status serial_post_e(ems_gpu* h, const Fields& f) {
                 ++h->launches;
             }
         } else if (op.kind == EMS_OP_LUMPED) {
-            ems_gpu::LumpedDev& L = op.lumped;
-            double val = (L.has_src && h->step < L.amp.size()) ? L.amp[h->step] : 0.0;
-            bool active = L.has_src && val != 0.0;
-            size_t idx = L.count;
-            if (L.record) {
-                ems_status st = grow(h, &L.rec, L.count, &L.cap, L.count + 1);
-                if (st) return st;
-                if (L.columns) {
-                    st = grow(h, &L.pv, L.count, &L.vcap, L.count + 1);
-                    if (st) return st;
-                    st = grow(h, &L.pi, L.count, &L.icap, L.count + 1);
-                    if (st) return st;
-                }
-            }
+            run_hooks(h, f, lo, hi, sides, acts);
+            const ems_gpu::LumpedDev& L = op.lumped;
+            const double val = (L.has_src && h->step < L.amp.size()) ? L.amp[h->step] : 0.0;
+            const bool active = L.has_src && val != 0.0;
             k_lumped_post_e<<<1, 256, 0, s>>>(f.u[L.axis], L.d, val, active ? 1 : 0, h->dt,
-                                              L.record ? L.rec + idx : nullptr, L.columns ? L.pv + idx : nullptr,
-                                              L.columns ? L.pi + idx : nullptr);
+                                              L.record ? L.rec + h->step : nullptr, L.columns ? L.pv + h->step : nullptr,
+                                              L.columns ? L.pi + h->step : nullptr, h->hooks.mail + 3 * q);
             ++h->launches;
-            if (L.record) ++L.count;
-        } else if (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_E || op.source.kind == EMS_HARD_E)) {
-            const ems_gpu::SourceDev& sd = op.source;
-            float a = h->step < sd.amp.size() ? sd.amp[h->step] : 0.0f;
-            bool hard = sd.kind == EMS_HARD_E;
-            if (!hard && a == 0.0f) continue;
-            k_source<<<blocks_for(sd.n, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], sd.axis, sd.node, sd.weight, sd.n, a, hard);
-            ++h->launches;
+        } else if (op.kind == EMS_OP_SOURCE && !h_side) {
+            run_hooks(h, f, lo, hi, sides, acts);
+            run_source(h, op.source, f.u);
         } else if (op.kind == EMS_OP_SHEET && op.sheet.n_edges) {
+            run_hooks(h, f, lo, hi, sides, acts);
             const SheetDevT& sd = op.sheet;
             k_sheet_post_e<<<blocks_for(sd.n_edges, 128), 128, 0, s>>>(f.u[0], f.u[1], f.u[2], f.i[0], f.i[1], f.i[2], sd);
             ++h->launches;
-        } else if (op.kind == EMS_OP_PROBE && op.probe.quantity == EMS_PROBE_VOLTAGE && h->step % op.probe.interval == 0) {
-            ems_gpu::ProbeDev& p = op.probe;
-            ems_status st = grow(h, &p.values, p.count, &p.cap, p.count + 1);
-            if (st) return st;
-            k_probe<<<1, 32, 0, s>>>(f.u[0], f.u[1], f.u[2], p.d, p.values + p.count);
-            ++h->launches;
-            ++p.count;
         }
     }
+    run_hooks(h, f, lo, hi, sides, acts);
     return EMS_OK;
 }
 
@@ -1915,6 +2333,8 @@ ems_status ems_gpu_create(const ems_engine_desc* d, int device, ems_gpu** out) {
         ems_status st = setup_fused(h.get(), d);
         if (st) return st;
     }
+    if (ems_status st = setup_hooks(h.get())) return st;
+    if (ems_status st = setup_resident(h.get())) return st;
     if (check(h.get(), cudaStreamSynchronize(h->stream), "create")) return EMS_ERR_CUDA;
     *out = h.release();
     return EMS_OK;
@@ -1929,6 +2349,7 @@ ems_status ems_gpu_destroy(ems_gpu* h) {
     h->prof_collect();
     for (cudaEvent_t e : h->ev_free) cudaEventDestroy(e);
     h->bufs.clear();
+    if (h->hooks.mail) cudaFreeHost(h->hooks.mail);
     cudaStreamDestroy(h->stream);
     delete h;
     return EMS_OK;
@@ -2037,9 +2458,12 @@ static ems_status step_dumped(ems_gpu* h, bool energy) {
 ems_status ems_gpu_run(ems_gpu* h, uint64_t n) {
     if (!h) return EMS_ERR_INVALID;
     cudaSetDevice(h->device);
-    for (uint64_t s = 0; s < n; ++s) {
-        ems_status st = step_dumped(h, false);
+    for (uint64_t s = 0; s < n;) {
+        const bool resident = use_resident(h);
+        const uint64_t k = resident ? std::min(n - s, kResidentSteps) : 1;
+        ems_status st = resident ? run_resident(h, k) : step_dumped(h, false);
         if (st) return st;
+        s += k;
     }
     return check(h, cudaGetLastError(), "run");
 }
@@ -2269,7 +2693,7 @@ static ems_status device_status(ems_gpu* h) {
         cudaMemsetAsync(h->diverged, 0, sizeof(int), h->stream);
         if (check(h, cudaStreamSynchronize(h->stream), "status")) return EMS_ERR_CUDA;
     }
-    if (st[0]) return fail(h, EMS_ERR_TIMEOUT, "a bounded wait of the fused or marching kernel ran out");
+    if (st[0]) return fail(h, EMS_ERR_TIMEOUT, "a bounded wait of the fused, marching or resident kernel ran out");
     if (st[1]) return fail(h, EMS_ERR_DIVERGED, "a marching step wrote a non-finite field value");
     return EMS_OK;
 }
@@ -2391,20 +2815,27 @@ ems_status ems_gpu_last_sample(ems_gpu* h, size_t op, int which, double* out) {
         cnt = o.lumped.count;
     }
     if (!src || !cnt) return fail(h, EMS_ERR_INVALID, "no sample");
-    if (check(h, cudaMemcpyAsync(out, src + cnt - 1, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "sample"))
-        return EMS_ERR_CUDA;
-    return check(h, cudaStreamSynchronize(h->stream), "sample");
+    // The hooks have left the newest samples in host memory.
+    if (check(h, cudaStreamSynchronize(h->stream), "sample")) return EMS_ERR_CUDA;
+    *out = ((volatile double*)h->hooks.mail)[3 * op + which];
+    return EMS_OK;
 }
 
 ems_status ems_gpu_source_amplitude(ems_gpu* h, size_t op, uint64_t first, const double* values, size_t n) {
     if (!h || (!values && n) || op >= h->ops.size()) return EMS_ERR_INVALID;
     auto& o = h->ops[op];
+    auto dirty = [&](auto& d) {
+        d.lo = d.lo < d.hi ? std::min<size_t>(d.lo, first) : first;
+        d.hi = std::max<size_t>(d.hi, first + n);
+    };
     if (o.kind == EMS_OP_SOURCE) {
         if (o.source.amp.size() < first + n) o.source.amp.resize(first + n, 0.0f);
         for (size_t q = 0; q < n; ++q) o.source.amp[first + q] = (float)values[q];
+        dirty(o.source.amp_dev);
     } else if (o.kind == EMS_OP_LUMPED && o.lumped.has_src) {
         if (o.lumped.amp.size() < first + n) o.lumped.amp.resize(first + n, 0.0);
         for (size_t q = 0; q < n; ++q) o.lumped.amp[first + q] = values[q];
+        dirty(o.lumped.amp_dev);
     } else {
         return fail(h, EMS_ERR_INVALID, "not a source");
     }
@@ -2595,6 +3026,22 @@ struct ems_batch {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
     } tune;
     int grid_code = 1;
+    // Resident steps (resident.cuh): a gang of blocks per active model.
+    struct Resident {
+        bool ok = false, stale = true;  // stale: the gangs are not those of the active models
+        unsigned fit = 0, grid = 0;
+        std::vector<uint64_t> quads;    // work of each model
+        ResModel* models = nullptr;
+        uint4* blocks = nullptr;
+        uint2* gangs = nullptr;
+        uint32_t* list = nullptr;
+        uint32_t* bars = nullptr;       // two sets of `fit` counters
+        int* status = nullptr;
+        int flip = 0;
+        std::vector<uint4> h_blocks;
+        std::vector<uint2> h_gangs;
+        std::vector<uint32_t> h_list;
+    } res;
 
     template <class T_>
     T_* alloc(size_t n) {
@@ -2699,6 +3146,82 @@ ems_status batch_capture(ems_batch* b, bool energy, cudaGraphExec_t* out) {
     return EMS_OK;
 }
 
+constexpr unsigned kGangThreads = 256;  // two blocks per SM: gangs of half an SM's grain
+
+// Gangs for the active models: with no more models than blocks, each block in
+// turn goes to the model with the most work per block (so the largest share
+// is as small as it can be); with more, a gang is one block and takes the
+// models one after the other, each model going to the least loaded gang.
+ems_status resident_plan(ems_batch* b) {
+    auto& r = b->res;
+    std::vector<uint32_t> act;
+    for (size_t m = 0; m < b->models.size(); ++m)
+        if (b->active[m]) act.push_back((uint32_t)m);
+    std::sort(act.begin(), act.end(), [&](uint32_t x, uint32_t y) {
+        return r.quads[x] != r.quads[y] ? r.quads[x] > r.quads[y] : x < y;
+    });
+    r.h_blocks.clear();
+    r.h_gangs.clear();
+    r.h_list.clear();
+    if (act.size() <= r.fit) {
+        using Entry = std::pair<double, uint32_t>;  // work per block, place in act
+        std::vector<unsigned> size(act.size(), 1);
+        std::vector<Entry> heap;
+        for (uint32_t q = 0; q < act.size(); ++q) heap.push_back({(double)r.quads[act[q]], q});
+        std::make_heap(heap.begin(), heap.end());
+        for (size_t left = r.fit - act.size(); left && !heap.empty(); --left) {
+            std::pop_heap(heap.begin(), heap.end());
+            const uint32_t q = heap.back().second;
+            heap.pop_back();
+            const uint64_t w = r.quads[act[q]];
+            if ((uint64_t)size[q] * kGangThreads >= w) continue;  // a block without a quad helps nobody
+            ++size[q];
+            heap.push_back({(double)w / size[q], q});
+            std::push_heap(heap.begin(), heap.end());
+        }
+        for (uint32_t q = 0; q < act.size(); ++q) {
+            for (unsigned k = 0; k < size[q]; ++k) r.h_blocks.push_back(uint4{q, k, size[q], 0});
+            r.h_gangs.push_back(uint2{q, q + 1});
+            r.h_list.push_back(act[q]);
+        }
+    } else {
+        std::vector<std::vector<uint32_t>> of(r.fit);
+        std::vector<uint64_t> load(r.fit, 0);
+        for (uint32_t m : act) {
+            const size_t q = std::min_element(load.begin(), load.end()) - load.begin();
+            of[q].push_back(m);
+            load[q] += r.quads[m];
+        }
+        for (uint32_t q = 0; q < r.fit; ++q) {
+            r.h_blocks.push_back(uint4{q, 0, 1, 0});
+            r.h_gangs.push_back(uint2{(uint32_t)r.h_list.size(), (uint32_t)(r.h_list.size() + of[q].size())});
+            r.h_list.insert(r.h_list.end(), of[q].begin(), of[q].end());
+        }
+    }
+    r.grid = (unsigned)r.h_blocks.size();
+    r.stale = false;
+    if (!r.grid) return EMS_OK;
+    if (cudaMemcpyAsync(r.blocks, r.h_blocks.data(), r.grid * sizeof(uint4), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+        cudaMemcpyAsync(r.gangs, r.h_gangs.data(), r.h_gangs.size() * sizeof(uint2), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+        cudaMemcpyAsync(r.list, r.h_list.data(), r.h_list.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
+        return bfail(b, EMS_ERR_CUDA, "resident plan");
+    return EMS_OK;
+}
+
+// Steps every active model n times in one launch.
+ems_status batch_resident(ems_batch* b, uint64_t n) {
+    auto& r = b->res;
+    if (r.stale)
+        if (ems_status st = resident_plan(b)) return st;
+    if (!r.grid) return EMS_OK;
+    ResArgs A{r.models, r.blocks, r.gangs, r.list, r.bars + (size_t)32 * r.fit * r.flip,
+              r.bars + (size_t)32 * r.fit * (r.flip ^ 1), r.fit, (uint32_t)n, 0u, b->d_steps, r.status, kWaitNs};
+    r.flip ^= 1;
+    cudaError_t e;
+    launch_resident(A, false, r.grid, kGangThreads, b->stream, &e);
+    return e == cudaSuccess ? EMS_OK : bfail(b, EMS_ERR_CUDA, std::string("resident steps: ") + cudaGetErrorString(e));
+}
+
 // Checks the operator order a batch can run: per model, the serial post_h
 // hooks are H sources then current probes, the serial post_e hooks lumped
 // elements then E sources then voltage probes (the order the batched
@@ -2768,6 +3291,8 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
     std::vector<BatchSource> src[2];
     std::vector<BatchProbe> prb[2];
     std::vector<BatchLumped> lum;
+    std::vector<ResModel> rm(n_models);
+    bool resident = true;
     for (int k = 0; k < BK_KINDS; ++k) b->start[k].assign(1, 0u);
     int pf = -1;
     for (size_t m = 0; m < n_models; ++m) {
@@ -2832,6 +3357,14 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
             b->start[k].push_back((uint32_t)next);
         }
         b->blocks.push_back({blocks[0], blocks[1], blocks[2], blocks[3], blocks[4]});
+        // Resident steps: the same tables; the saved values of the poles are
+        // captured every step, as the batched kernels do.
+        std::vector<ResOp> rops;
+        resident = resident && resident_ops(h);
+        if (resident)
+            if (ems_status rs = resident_quads(h)) return rs;
+        resident_model(h, rm[m]);
+        b->res.quads.push_back(rm[m].quads);
         // Serial hooks: sources, probes, lumped elements (device tables).
         size_t op_i = 0;
         for (auto& op : h->ops) {
@@ -2845,6 +3378,11 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
                     src[e_side ? 1 : 0].push_back(BatchSource{(uint32_t)m, dev_index(g, sr->node[e]), sr->axis[e],
                                                               hard ? 1u : 0u, sr->weight[e],
                                                               (uint32_t)op.source.amp.size(), amp});
+                ResOp o{};
+                resident_op(op, o);
+                o.amp = amp;
+                o.n_amp = (uint32_t)op.source.amp.size();
+                rops.push_back(o);
             } else if (op.kind == EMS_OP_PROBE) {
                 const ems_gpu::ProbeDev& P = op.probe;
                 const uint32_t interval = (uint32_t)std::min<uint64_t>(P.interval, max_steps);
@@ -2853,6 +3391,12 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
                 if (!v) return EMS_ERR_NOMEM;
                 prb[P.quantity == EMS_PROBE_VOLTAGE ? 1 : 0].push_back(BatchProbe{(uint32_t)m, interval, cap, P.d, v});
                 b->series.push_back({m, op_index, 0, interval, cap, v});
+                ResOp o{};
+                resident_op(op, o);
+                o.interval = interval;
+                o.cap = cap;
+                o.values = v;
+                rops.push_back(o);
             } else if (op.kind == EMS_OP_LUMPED) {
                 const ems_gpu::LumpedDev& L = op.lumped;
                 BatchLumped bl{};
@@ -2876,8 +3420,22 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
                     b->series.push_back({m, op_index, 2, 1, (uint32_t)max_steps, bl.pi});
                 }
                 lum.push_back(bl);
+                ResOp o{};
+                resident_op(op, o);
+                o.amp_l = bl.amp;
+                o.n_amp = bl.n_amp;
+                o.rec = bl.rec;
+                o.pv = bl.pv;
+                o.pi = bl.pi;
+                o.cap = bl.cap;
+                rops.push_back(o);
             }
         }
+        rm[m].n_ops = (uint32_t)rops.size();
+        rm[m].ops = b->upload(rops.data(), rops.size());
+        if (!rm[m].ops) return EMS_ERR_NOMEM;
+        // The copies out of rops end before it goes.
+        if (cudaStreamSynchronize(b->stream) != cudaSuccess) return EMS_ERR_CUDA;
     }
     b->poles_first = pf == 1;
     b->active.assign(n_models, 1);
@@ -2914,6 +3472,18 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
     occ[BK_POLES_H] = occ[BK_POLES_E];
     for (int k = 0; k < BK_KINDS; ++k) b->resident[k] = (uint64_t)sms * std::max(1, occ[k]);
     batch_grids(b, 1);
+    auto& r = b->res;
+    r.fit = resident ? resident_blocks(device, kGangThreads) : 0;
+    if (r.fit) {
+        r.models = b->upload(rm.data(), n_models);
+        r.blocks = b->alloc<uint4>(r.fit);
+        r.gangs = b->alloc<uint2>(r.fit);
+        r.list = b->alloc<uint32_t>(n_models);
+        r.bars = b->alloc<uint32_t>((size_t)64 * r.fit);
+        r.status = b->alloc<int>(1);
+        if (!r.models || !r.blocks || !r.gangs || !r.list || !r.bars || !r.status) return EMS_ERR_NOMEM;
+        r.ok = true;
+    }
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return EMS_ERR_CUDA;
     ems_status st = batch_graphs(b);
     if (st) return st;
@@ -2972,11 +3542,28 @@ static ems_status batch_tune_step(ems_batch* b) {
     return EMS_OK;
 }
 
+// EMS_ERR_TIMEOUT if a wait of the resident kernel ran out since the last check.
+static ems_status batch_status(ems_batch* b) {
+    if (!b->res.ok) return EMS_OK;
+    int v = 0;
+    if (cudaMemcpyAsync(&v, b->res.status, sizeof v, cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
+        cudaStreamSynchronize(b->stream) != cudaSuccess)
+        return bfail(b, EMS_ERR_CUDA, "status");
+    if (!v) return EMS_OK;
+    cudaMemsetAsync(b->res.status, 0, sizeof v, b->stream);
+    return bfail(b, EMS_ERR_TIMEOUT, "a bounded wait of the resident kernel ran out");
+}
+
 ems_status ems_batch_run(ems_batch* b, uint64_t n) {
     if (!b) return EMS_ERR_INVALID;
     cudaSetDevice(b->device);
     for (uint64_t q = 0; q < n; ++q) {
-        if (b->tune.active) {
+        if (b->res.ok && !b->tune.active) {
+            const uint64_t k = std::min(n - q, kResidentSteps);
+            ems_status st = batch_resident(b, k);
+            if (st) return st;
+            q += k - 1;
+        } else if (b->tune.active) {
             ems_status st = batch_tune_step(b);
             if (st) return st;
         } else if (cudaGraphLaunch(b->step_graph, b->stream) != cudaSuccess) {
@@ -3023,13 +3610,14 @@ ems_status ems_batch_step_with_energy(ems_batch* b, double* energies) {
         cudaMemcpyAsync(energies, b->energies, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, EMS_ERR_CUDA, "energy step");
-    return EMS_OK;
+    return batch_status(b);
 }
 
 ems_status ems_batch_set_active(ems_batch* b, size_t model, int active) {
     if (!b || model >= b->models.size()) return EMS_ERR_INVALID;
     cudaSetDevice(b->device);
     b->active[model] = active ? 1 : 0;
+    b->res.stale = true;
     // The packed block table shrinks to the active models (a frozen model's
     // range becomes empty), so the persistent grids walk only live work;
     // the graphs read the table from device memory and need no re-capture.
@@ -3056,7 +3644,7 @@ ems_status ems_batch_timestep(ems_batch* b, size_t model, uint64_t* n) {
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, EMS_ERR_CUDA, "timestep");
     *n = v;
-    return EMS_OK;
+    return batch_status(b);
 }
 
 ems_status ems_batch_samples(ems_batch* b, size_t model, size_t op, int which, double* out, size_t cap, size_t* n) {

@@ -397,6 +397,36 @@ inline RowCpml row_cpml_plan(const std::vector<SlabGeo>& slabs, const uint64_t n
     return R;
 }
 
+// The quads (four z-nodes) of the grid that hold a CPML slab of one side, as
+// (quad, slabs) with the quads numbered row by row ((i·ny + j)·quads per row +
+// k / 4) and the slabs as bits side·12 + component·4 + q, and the others. The
+// resident kernel takes each list with code of its own, so that no warp runs
+// the corrections for a few of its lanes.
+inline void cpml_quads(const std::vector<SlabGeo>& slabs, const uint64_t nodes[3], int side, std::vector<uint2>& layer,
+                       std::vector<uint32_t>& inner) {
+    const uint32_t nx = (uint32_t)nodes[0], ny = (uint32_t)nodes[1], nq = ((uint32_t)nodes[2] + 3u) / 4u;
+    std::vector<uint32_t> bx(nx, 0u), by(ny, 0u), bz(nq, 0u);
+    for (const SlabGeo& s : slabs) {
+        if (s.side != side) continue;
+        const uint32_t bit = 1u << (side * 12 + s.comp * 4 + s.q), lo = s.lo[s.normal], hi = s.hi[s.normal];
+        for (uint32_t v = lo; v < hi; ++v) {
+            if (s.normal == 0 && v < nx) bx[v] |= bit;
+            if (s.normal == 1 && v < ny) by[v] |= bit;
+            if (s.normal == 2 && v / 4u < nq) bz[v / 4u] |= bit;
+        }
+    }
+    layer.clear();
+    inner.clear();
+    uint32_t q = 0;
+    for (uint32_t i = 0; i < nx; ++i)
+        for (uint32_t j = 0; j < ny; ++j)
+            for (uint32_t k = 0; k < nq; ++k, ++q) {
+                const uint32_t b = bx[i] | by[j] | bz[k];
+                if (b) layer.push_back(uint2{q, b});
+                else inner.push_back(q);
+            }
+}
+
 inline std::vector<ShellBox> shell_boxes(const FusedTables& T, const uint64_t nodes[3], int side, uint32_t* total,
                                          const std::vector<uint32_t>& xcuts = {}) {
     return shell_boxes(slab_geometry(T), T.nslab[side], nodes, side, total, xcuts);

@@ -12,6 +12,12 @@
 
 namespace emsk {
 
+#ifdef EMS_HOST_EMULATION
+#define EMS_BLOCK_SHARED static
+#else
+#define EMS_BLOCK_SHARED __shared__
+#endif
+
 constexpr unsigned kRowThreads = 128;  // threads of a z-row block
 constexpr uint32_t kMaxPoles = 16;     // poles per edge held in registers
 constexpr uint32_t kOeDebye = 1u << 31;  // PoleRun::oe: an edge of openEMS Debye poles
@@ -313,11 +319,6 @@ __device__ __forceinline__ void probe_sample(const float* f0, const float* f1, c
     }
 }
 
-__global__ void k_probe(const float* f0, const float* f1, const float* f2, ProbeDevT p, double* out) {
-    if (threadIdx.x != 0) return;
-    probe_sample(f0, f1, f2, p, out);
-}
-
 // Lumped element pre_e: saves u^n (src/engine/lumped.rs:1106-1121).
 __device__ __forceinline__ void lumped_pre_e_edge(const float* u, const LumpedDevT& d, uint32_t e) {
     const double x = (double)u[d.node[e]];
@@ -333,9 +334,12 @@ __global__ void k_lumped_pre_e(const float* u, LumpedDevT d) {
 
 // Lumped element post_e (src/engine/lumped.rs:1123-1236) and, for a port,
 // V = Σu/columns, I = −record (src/engine/port.rs:276-290). One block: the
-// per-edge updates in parallel, the sums in edge order by thread 0.
+// per-edge updates and the terms of the sums in parallel, the sums in edge
+// order by thread 0 from shared memory (from global memory its dependent
+// loads took most of the hook's 6.5 us).
 __device__ __forceinline__ void lumped_post_e_block(float* u, const LumpedDevT& d, double val, int active, double dt,
-                                                    double* rec_out, double* pv_out, double* pi_out) {
+                                                    double* rec_out, double* pv_out, double* pi_out,
+                                                    double* mail = nullptr) {
     for (uint32_t e = threadIdx.x; e < d.n; e += blockDim.x) {
         const uint32_t idx = d.node[e];
         if (d.src_w) d.v[e] = active ? __dadd_rn(0.0, __dmul_rn(d.src_w[e], val)) : 0.0;
@@ -373,33 +377,55 @@ __device__ __forceinline__ void lumped_post_e_block(float* u, const LumpedDevT& 
             if (add != 0.0) u[idx] = (float)__dadd_rn((double)u[idx], add);
         }
     }
-    __syncthreads();
+    if (!(d.record && rec_out) && !pv_out) return;
+    constexpr uint32_t kTerms = 128;  // edges whose terms are held at once
+    EMS_BLOCK_SHARED double term[3][kTerms];
+    double sum = 0.0, s = 0.0;
+    for (uint32_t e0 = 0; e0 < d.n; e0 += kTerms) {
+        const uint32_t m = d.n - e0 < kTerms ? d.n - e0 : kTerms;
+        __syncthreads();
+        for (uint32_t q = threadIdx.x; q < m; q += blockDim.x) {
+            const uint32_t e = e0 + q;
+            const double u1 = (double)u[d.node[e]];
+            term[2][q] = u1;
+            if (!(d.record && rec_out)) continue;
+            const double u0 = d.ru_prev[e], v = (active && !d.src_in_branch) ? d.v[e] : 0.0;
+            const double t1 = __dmul_rn(d.rec_g[e], __dsub_rn(__dmul_rn(0.5, __dadd_rn(u0, u1)), v));
+            const double t2 = __ddiv_rn(__dmul_rn(d.rec_c[e], __dsub_rn(u1, u0)), dt);
+            term[0][q] = __dadd_rn(t1, t2);
+            if (d.has_branch) term[1][q] = d.j_avg[e];
+        }
+        __syncthreads();
+        if (threadIdx.x != 0) continue;
+        for (uint32_t q = 0; q < m; ++q) {
+            if (d.record && rec_out) {
+                sum = __dadd_rn(sum, term[0][q]);
+                if (d.has_branch) sum = __dadd_rn(sum, term[1][q]);
+            }
+            s = __dadd_rn(s, term[2][q]);
+        }
+    }
     if (threadIdx.x != 0) return;
     double rec = 0.0;
     if (d.record && rec_out) {
-        double sum = 0.0;
-        for (uint32_t e = 0; e < d.n; ++e) {
-            const double u0 = d.ru_prev[e], u1 = (double)u[d.node[e]];
-            const double v = (active && !d.src_in_branch) ? d.v[e] : 0.0;
-            const double t1 = __dmul_rn(d.rec_g[e], __dsub_rn(__dmul_rn(0.5, __dadd_rn(u0, u1)), v));
-            const double t2 = __ddiv_rn(__dmul_rn(d.rec_c[e], __dsub_rn(u1, u0)), dt);
-            sum = __dadd_rn(sum, __dadd_rn(t1, t2));
-            if (d.has_branch) sum = __dadd_rn(sum, d.j_avg[e]);
-        }
         rec = __ddiv_rn(sum, d.series);
         rec_out[0] = rec;
+        if (mail) mail[0] = rec;
     }
     if (pv_out) {
+        const double v = __ddiv_rn(s, d.columns);
         pi_out[0] = -rec;
-        double s = 0.0;
-        for (uint32_t e = 0; e < d.n; ++e) s = __dadd_rn(s, (double)u[d.node[e]]);
-        pv_out[0] = __ddiv_rn(s, d.columns);
+        pv_out[0] = v;
+        if (mail) {
+            mail[1] = v;
+            mail[2] = -rec;
+        }
     }
 }
 
 __global__ void __launch_bounds__(256) k_lumped_post_e(float* u, LumpedDevT d, double val, int active, double dt,
-                                                       double* rec_out, double* pv_out, double* pi_out) {
-    lumped_post_e_block(u, d, val, active, dt, rec_out, pv_out, pi_out);
+                                                       double* rec_out, double* pv_out, double* pi_out, double* mail) {
+    lumped_post_e_block(u, d, val, active, dt, rec_out, pv_out, pi_out, mail);
 }
 
 // Σ ½·L·j² + ½·q²/C_p of the electric then the magnetic poles
@@ -471,11 +497,24 @@ struct UpmlSideDev {
     float* v = nullptr;
 };
 
+// The update of layer edge q of a side in the field F from the flux
+// increment the update kernel left there (upml.rs Run::apply):
+// F' = flush(flush(co.x·F) + t), x = flush(flush(flush(co.y·v) − flush(co.w·F)) + flush(co.z·F')).
+__device__ __forceinline__ void upml_apply(float* F, const UpmlSideDev& a, uint32_t q) {
+    const uint32_t idx = a.node[q];
+    const float4 c = a.co[q];
+    const float t = F[idx], f0 = a.f[q], v = a.v[q];
+    const float f1 = flush(__fadd_rn(flush(__fmul_rn(c.x, f0)), t));
+    const float x = flush(__fadd_rn(flush(__fsub_rn(flush(__fmul_rn(c.y, v)), flush(__fmul_rn(c.w, f0)))),
+                                    flush(__fmul_rn(c.z, f1))));
+    a.f[q] = f1;
+    a.v[q] = x;
+    F[idx] = x;
+}
+
 // One slab hook of the layers (upml.rs:443-464): threads [0, r.n) take the
 // start values of side r from the fields `src` (Run::refresh), threads
-// [r.n, r.n + a.n) complete the update of side a in the fields `dst` from
-// the flux increment the update kernel left there (Run::apply):
-// F' = flush(flush(co.x·F) + t), x = flush(flush(flush(co.y·v) − flush(co.w·F)) + flush(co.z·F')).
+// [r.n, r.n + a.n) complete the update of side a in the fields `dst`.
 __global__ void __launch_bounds__(256) k_upml_hook(const float* s0, const float* s1, const float* s2, UpmlSideDev r,
                                                    float* d0, float* d1, float* d2, UpmlSideDev a) {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -488,16 +527,7 @@ __global__ void __launch_bounds__(256) k_upml_hook(const float* s0, const float*
     const uint32_t q = e - r.n;
     if (q >= a.n) return;
     const uint8_t ax = a.axis[q];
-    float* F = ax == 0 ? d0 : (ax == 1 ? d1 : d2);
-    const uint32_t idx = a.node[q];
-    const float4 c = a.co[q];
-    const float t = F[idx], f0 = a.f[q], v = a.v[q];
-    const float f1 = flush(__fadd_rn(flush(__fmul_rn(c.x, f0)), t));
-    const float x = flush(__fadd_rn(flush(__fsub_rn(flush(__fmul_rn(c.y, v)), flush(__fmul_rn(c.w, f0)))),
-                                    flush(__fmul_rn(c.z, f1))));
-    a.f[q] = f1;
-    a.v[q] = x;
-    F[idx] = x;
+    upml_apply(ax == 0 ? d0 : (ax == 1 ? d1 : d2), a, q);
 }
 
 // A Mur boundary on the device (src/engine/boundary/mur.rs:103-139):

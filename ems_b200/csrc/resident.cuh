@@ -1,8 +1,8 @@
 // resident.cuh — many steps in one launch (sm_100a).
 //
-// On grids that fit in L2 a step of the split schedule is not bound by
-// memory but by its launches: a 100^3 box takes ten of them, 62 us for about
-// 15 us of L2 traffic. Here a gang of blocks advances a model by n steps in
+// On small grids a step of the split schedule is not bound by memory but by
+// its launches: a 100^3 box takes ten of them, 62 us for about 15 us of L2
+// traffic (40 us here; a 24^3 box 45 -> 26 us). Here a gang of blocks advances a model by n steps in
 // one cooperative launch: the phases of a step (H update, CPML of the H
 // side, E update, CPML of the E side, poles, serial hooks) are the split
 // schedule's device functions over strided work items, with a barrier of the
@@ -10,7 +10,7 @@
 // a gang of its own, sized by its cells, so the models never wait for one
 // another.
 //
-// The serial hooks run on the gang's first block in registration order, from
+// The serial hooks run on one block of the gang in registration order, from
 // amplitude tables and sample buffers on the device. Fields change within
 // the launch, so they are read through the coherent path, never __ldg.
 //
@@ -49,6 +49,7 @@ struct ResOp {
     const float* amp;
     const double* amp_l;
     double *values, *rec, *pv, *pi;  // series (index: step, or step / interval); null: not recorded
+    double* mail;                    // host copies of the newest samples (probe; or rec, pv, pi), or null
     ProbeDevT probe;
     LumpedDevT lumped;
 };
@@ -56,21 +57,25 @@ struct ResOp {
 // One model as the resident kernel reads it.
 struct ResModel {
     BatchModel m;
-    UpmlSideDev upml[2];
     const ResOp* ops;
     uint32_t n_ops;
-    int32_t order[3];            // slab hooks in registration order: 0 CPML, 1 poles, 2 openEMS PML; -1 end
+    int32_t order[2];            // slab hooks in registration order: 0 CPML, 1 poles, -1 none
     int32_t fold_e, fold_h;      // the pole correction stores the saved values
     int32_t capture_first;       // fold_e, but the saved electric values are not current at the launch
     int32_t serial_h, serial_e;  // whether a post_h hook writes i, a post_e hook exists
     FastDiv div_q, div_j;        // quads per row, rows per plane
     uint32_t quads;              // nx·ny·quads per row
     uint32_t units[2];           // blocks of the shell kernels
-    // The CPML comes first among the slab hooks: each thread applies it to the
-    // quad it has just updated (quad_cpml_all). Per side, quads below z_lo or
-    // reaching past z_hi may hold the slabs normal to z, z_bits.
+    // The CPML comes first among the slab hooks: its corrections are part of
+    // the update of the quads in `layer` (cpml_quads), `inner` the others.
+    // Otherwise layer is empty and every quad inner (null: all of them in order).
     int32_t quad_cpml;
-    uint32_t z_lo[2], z_hi[2], z_bits[2];
+    const uint2* layer[2];
+    const uint32_t* inner[2];
+    uint32_t n_layer[2];
+    // Every voltage probe comes after the hooks that write u: the samples of a
+    // step may be taken during the next H update.
+    int32_t late_probes, writes_e;
 };
 
 struct ResArgs {
@@ -102,7 +107,8 @@ __device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
     if (threadIdx.x == 0) {
         const uint32_t want = G.epoch * G.size;
         uint32_t v;
-        __threadfence();
+        // The release covers the block's writes (ordered before it by the
+        // block barrier), the acquire its reads after the next one.
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(G.bar) : "memory");
         uint64_t t0 = 0;
         for (uint32_t it = 0;; ++it) {
@@ -117,7 +123,6 @@ __device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
                 break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return *ok != 0;
@@ -125,7 +130,7 @@ __device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
 
 // A probe's sample by one warp: the products in parallel, their sum in entry
 // order (src/engine/probe.rs:381-392).
-__device__ __forceinline__ void probe_warp(const Fields& f, bool electric, const ProbeDevT& p, double* out) {
+__device__ __forceinline__ void probe_warp(const Fields& f, bool electric, const ProbeDevT& p, double* out, double* mail) {
     const uint32_t lane = threadIdx.x & 31u;
     double s = 0.0;
     float s32 = 0.0f;
@@ -143,28 +148,31 @@ __device__ __forceinline__ void probe_warp(const Fields& f, bool electric, const
             else s = __dadd_rn(s, __shfl_sync(0xffffffffu, t, q));
         }
     }
-    if (lane == 0) *out = p.f32_sum ? (double)s32 : s;
+    if (lane != 0) return;
+    *out = p.f32_sum ? (double)s32 : s;
+    if (mail) *mail = *out;
 }
 
-// The serial hooks of one field side at step `step`, by the gang's first
-// block, in registration order; consecutive probes take a warp each.
-__device__ __forceinline__ void serial_hooks(const ResModel& R, bool electric, uint32_t step) {
-    const Fields& f = R.m.f;
-    for (uint32_t q = 0; q < R.n_ops;) {
-        const ResOp& o = R.ops[q];
-        const bool mine = o.kind == ResOp::LUMPED ? electric : (o.electric != 0) == electric;
+// The serial hooks of one field side at step `step`, by one block, in
+// registration order (probes: the probes; writers: the others); consecutive
+// probes take a warp each.
+__device__ __forceinline__ void serial_hooks(const Fields& f, double dt, const ResOp* ops, uint32_t n_ops, bool electric,
+                                             uint32_t step, bool probes, bool writers) {
+    for (uint32_t q = 0; q < n_ops;) {
+        const ResOp& o = ops[q];
+        const bool mine = (o.electric != 0) == electric && (o.kind == ResOp::PROBE ? probes : writers);
         if (!mine) {
             ++q;
             continue;
         }
         if (o.kind == ResOp::PROBE) {
             uint32_t end = q;
-            while (end < R.n_ops && R.ops[end].kind == ResOp::PROBE) ++end;
+            while (end < n_ops && ops[end].kind == ResOp::PROBE) ++end;
             for (uint32_t r = q + (threadIdx.x >> 5); r < end; r += blockDim.x >> 5) {
-                const ResOp& p = R.ops[r];
+                const ResOp& p = ops[r];
                 if ((p.electric != 0) != electric || step % p.interval) continue;
                 const uint32_t at = step / p.interval;
-                if (at < p.cap) probe_warp(f, electric, p.probe, p.values + at);
+                if (at < p.cap) probe_warp(f, electric, p.probe, p.values + at, p.mail);
             }
             q = end;
         } else if (o.kind == ResOp::SOURCE) {
@@ -179,13 +187,35 @@ __device__ __forceinline__ void serial_hooks(const ResModel& R, bool electric, u
         } else {
             const double val = o.has_src && step < o.n_amp ? o.amp_l[step] : 0.0;
             const bool room = step < o.cap;
-            lumped_post_e_block(f.u[o.axis_l], o.lumped, val, o.has_src && val != 0.0, R.m.dt,
+            lumped_post_e_block(f.u[o.axis_l], o.lumped, val, o.has_src && val != 0.0, dt,
                                 o.rec && room ? o.rec + step : nullptr, o.pv && room ? o.pv + step : nullptr,
-                                o.pi && room ? o.pi + step : nullptr);
+                                o.pi && room ? o.pi + step : nullptr, o.mail);
             ++q;
         }
         __syncthreads();
     }
+}
+
+// The lumped elements' u^n before an E update (src/engine/lumped.rs:1106-1121).
+__device__ __forceinline__ void serial_pre(const Fields& f, const ResOp* ops, uint32_t n_ops) {
+    for (uint32_t q = 0; q < n_ops; ++q) {
+        const ResOp& o = ops[q];
+        if (o.kind != ResOp::LUMPED || !(o.lumped.record || o.lumped.has_branch)) continue;
+        for (uint32_t e = threadIdx.x; e < o.lumped.n; e += blockDim.x) lumped_pre_e_edge(f.u[o.axis_l], o.lumped, e);
+    }
+}
+
+// The serial hooks of a step that is not resident: one block, one launch for
+// every hook of both sides (sides bit 0: current probes and H sources, bit 1:
+// the electric ones) instead of one each: six launches of 2.5 us on a box with
+// a source and five probes.
+__global__ void __launch_bounds__(256) k_hooks(const __grid_constant__ Fields f, double dt, const ResOp* ops, uint32_t n_ops,
+                                               uint32_t step, int sides) {
+    if (sides & 1) serial_hooks(f, dt, ops, n_ops, false, step, true, true);
+    if (sides & 2) serial_hooks(f, dt, ops, n_ops, true, step, true, true);
+}
+__global__ void __launch_bounds__(256) k_hooks_pre(const __grid_constant__ Fields f, const ResOp* ops, uint32_t n_ops) {
+    serial_pre(f, ops, n_ops);
 }
 
 // One side of the poles: the correction, save_prev as in k_poles_blocks.
@@ -202,12 +232,32 @@ __device__ __forceinline__ void res_capture(const ResModel& R, bool electric, ui
         p.prev[e] = (electric ? R.m.f.u : R.m.f.i)[p.axis[e]][p.node[e]];
 }
 
-// The CPML of one side at the quad a thread has just updated.
-template <int SIDE>
-__device__ __forceinline__ void res_quad_cpml(const ResModel& R, uint32_t i, uint32_t j, uint32_t k0) {
-    uint32_t bits = row_slabs(R.m.P, SIDE, i, j);
-    if (k0 < R.z_lo[SIDE] || k0 + 4u > R.z_hi[SIDE]) bits |= R.z_bits[SIDE];
-    if (bits) quad_cpml_all<SIDE, true, false>(R.m.P, i, j, k0, bits);
+// One update (SIDE 0: H, 1: E) of the model's quads, worker t of `stride`.
+template <int SIDE, bool OE>
+__device__ __forceinline__ void res_update(const ResModel& R, uint32_t t, uint32_t stride) {
+    const uint32_t nl = R.n_layer[SIDE];
+    uint32_t x = t;
+    uint2 next = x < nl ? __ldg(R.layer[SIDE] + x) : make_uint2(0u, 0u);
+    for (; x < nl; x += stride) {
+        const uint2 q = next;
+        if (x + stride < nl) next = __ldg(R.layer[SIDE] + x + stride);
+        const uint32_t row = quotient(R.div_q, q.x), i = quotient(R.div_j, row);
+        const uint32_t j = row - i * R.div_j.d, k0 = (q.x - row * R.div_q.d) * 4u;
+        if (SIDE == 0) split_h_at<false, OE, false, false, true>(R.m.P, i, j, k0, q.y);
+        else split_e_at<OE, false, false, true>(R.m.P, i, j, k0, q.y);
+    }
+    const uint32_t ni = R.quads - nl;
+    x -= nl;
+    const uint32_t* list = R.inner[SIDE];
+    uint32_t nq = list && x < ni ? __ldg(list + x) : x;
+    for (; x < ni; x += stride) {
+        const uint32_t q = nq;
+        nq = list && x + stride < ni ? __ldg(list + x + stride) : x + stride;
+        const uint32_t row = quotient(R.div_q, q), i = quotient(R.div_j, row);
+        const uint32_t j = row - i * R.div_j.d, k0 = (q - row * R.div_q.d) * 4u;
+        if (SIDE == 0) split_h_at<false, OE, false, false>(R.m.P, i, j, k0);
+        else split_e_at<OE, false, false>(R.m.P, i, j, k0);
+    }
 }
 
 // The slab hooks of one side after its update, each followed by a barrier of
@@ -218,24 +268,27 @@ __device__ __forceinline__ bool res_slabs(const ResModel& R, Gang& G, uint32_t r
     // The saved values of the other field's poles: it does not change here.
     if (SIDE == 0 && capture) res_capture(R, true, t, stride);
     if (SIDE == 1 && R.m.ph.n_edges && !R.fold_h) res_capture(R, false, t, stride);
-    for (int q = 0; q < 3 && R.order[q] >= 0; ++q) {
+    for (int q = 0; q < 2 && R.order[q] >= 0; ++q) {
         if (R.order[q] == 0) {
             if (!R.units[SIDE] || R.quad_cpml) continue;
             for (uint32_t b = t >> 8; b < R.units[SIDE]; b += stride >> 8)
                 shell_item<SIDE>(R.m.P, R.m.shell[SIDE], b, threadIdx.x & 255u);
-        } else if (R.order[q] == 1) {
+        } else {
             const PoleSideDev& p = SIDE ? R.m.pe : R.m.ph;
             if (!p.n_edges) continue;
             res_poles(R, SIDE == 1, t, stride);
-        } else {
-            const UpmlSideDev &a = R.upml[SIDE ? 0 : 1], &r = R.upml[SIDE ? 1 : 0];
-            for (uint32_t e = t; e < r.n; e += stride) r.v[e] = (SIDE ? R.m.f.i : R.m.f.u)[r.axis[e]][r.node[e]];
-            for (uint32_t e = t; e < a.n; e += stride) upml_apply((SIDE ? R.m.f.u : R.m.f.i)[a.axis[e]], a, e);
         }
         if (!gang_sync(G, ok)) return false;
     }
     return true;
 }
+
+// Barriers of a step: after the H update, after the E update, one more per
+// slab operator but the CPML (and the CPML where it does not come first), one
+// for hooks that write i and one for those that write u. In a gang of
+// kHookGang blocks or more the last one takes no quads: it runs the hooks, the
+// probes beside the other blocks' updates.
+constexpr uint32_t kHookGang = 8;
 
 template <bool OE>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_constant__ ResArgs A) {
@@ -256,42 +309,37 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             reinterpret_cast<uint32_t*>(raw)[w] = reinterpret_cast<const uint32_t*>(A.models + id)[w];
         __syncthreads();
         const uint32_t step0 = A.steps ? A.steps[id] : A.step0;
-        const uint32_t t = rank * blockDim.x + threadIdx.x, stride = G.size * blockDim.x;
+        const bool apart = R.n_ops && G.size >= kHookGang;
+        const bool hooks = rank == (apart ? G.size - 1u : 0u);
+        const uint32_t stride = (G.size - (apart ? 1u : 0u)) * blockDim.x;
+        const uint32_t t = apart && hooks ? ~0u - 2u * stride : rank * blockDim.x + threadIdx.x;
+        auto hook = [&](bool electric, uint32_t step, bool probes, bool writers) {
+            serial_hooks(R.m.f, R.m.dt, R.ops, R.n_ops, electric, step, probes, writers);
+        };
         for (uint32_t s = 0; s < A.n; ++s) {
             const uint32_t step = step0 + s;
-            // The lumped elements' u^n: the E update is two barriers away.
-            if (rank == 0)
-                for (uint32_t q = 0; q < R.n_ops; ++q) {
-                    const ResOp& o = R.ops[q];
-                    if (o.kind != ResOp::LUMPED || !(o.lumped.record || o.lumped.has_branch)) continue;
-                    for (uint32_t e = threadIdx.x; e < o.lumped.n; e += blockDim.x)
-                        lumped_pre_e_edge(R.m.f.u[o.axis_l], o.lumped, e);
-                }
-            for (uint32_t q = t; q < R.quads; q += stride) {
-                const uint32_t row = quotient(R.div_q, q), i = quotient(R.div_j, row);
-                const uint32_t j = row - i * R.div_j.d, k0 = (q - row * R.div_q.d) * 4u;
-                split_h_at<false, OE, false, false>(R.m.P, i, j, k0);
-                if (R.quad_cpml) res_quad_cpml<0>(R, i, j, k0);
+            if (hooks) {
+                // The lumped elements' u^n and the samples of u^n.
+                serial_pre(R.m.f, R.ops, R.n_ops);
+                if (R.late_probes && s) hook(true, step - 1u, true, false);
             }
+            if (!(apart && hooks)) res_update<0, OE>(R, t, stride);
             if (!gang_sync(G, &ok)) return;
             if (!res_slabs<0>(R, G, rank, &ok, R.m.pe.n_edges && (!R.fold_e || (R.capture_first && s == 0)))) return;
-            // Hooks that write i before the E update; current probes beside it.
-            if (rank == 0) serial_hooks(R, false, step);
+            // Hooks that write i before the E update, in order with the current
+            // probes; else the probes beside it.
+            if (hooks) hook(false, step, true, true);
             if (R.serial_h && !gang_sync(G, &ok)) return;
-            for (uint32_t q = t; q < R.quads; q += stride) {
-                const uint32_t row = quotient(R.div_q, q), i = quotient(R.div_j, row);
-                const uint32_t j = row - i * R.div_j.d, k0 = (q - row * R.div_q.d) * 4u;
-                split_e_at<OE, false, false>(R.m.P, i, j, k0);
-                if (R.quad_cpml) res_quad_cpml<1>(R, i, j, k0);
-            }
+            if (!(apart && hooks)) res_update<1, OE>(R, t, stride);
             if (!gang_sync(G, &ok)) return;
             if (!res_slabs<1>(R, G, rank, &ok, false)) return;
-            if (R.serial_e) {
-                if (rank == 0) serial_hooks(R, true, step);
+            if (R.writes_e || (R.serial_e && !R.late_probes)) {
+                if (hooks) hook(true, step, !R.late_probes, true);
                 if (!gang_sync(G, &ok)) return;
             }
         }
-        if (A.steps && rank == 0 && threadIdx.x == 0) A.steps[id] = step0 + A.n;
+        if (R.late_probes && hooks && A.n) hook(true, step0 + A.n - 1u, true, false);
+        if (A.steps && hooks && threadIdx.x == 0) A.steps[id] = step0 + A.n;
     }
 }
 

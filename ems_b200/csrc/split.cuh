@@ -29,9 +29,17 @@ constexpr unsigned kShellWarps = 8;      // shell segments per block
 struct Q4 {
     float v[4];
 };
+// NC: through the read-only path; false where another block of the same
+// launch may have written the value (the resident kernel).
+template <bool NC = true>
 __device__ __forceinline__ Q4 ldq(const float* p) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    const float4* q = reinterpret_cast<const float4*>(p);
+    const float4 t = NC ? __ldg(q) : *q;
     return Q4{{t.x, t.y, t.z, t.w}};
+}
+template <bool NC>
+__device__ __forceinline__ float ldf(const float* p) {
+    return NC ? __ldg(p) : *p;
 }
 __device__ __forceinline__ Q4 ldq_rw(const float* p) {
     const float4 t = *reinterpret_cast<const float4*>(p);
@@ -122,18 +130,80 @@ __device__ __forceinline__ void row_cpml(const FusedParams& P, uint32_t i, uint3
     }
 }
 
+// One CPML slab at a quad of component C whose update is under way: its ψ,
+// loaded beside the update's own loads, and the nodes it corrects (bits 0-3).
+struct QuadSlab {
+    const FSlab* s;
+    uint32_t at, in;  // ψ index of node 0 of the quad (may lie before the row), nodes
+    float psi[4];
+};
+
+// The first slab of `bits` (bit side·12 + component·4 + q: the slabs that may
+// hold the quad) at component C; returns the others' bits q. in = 0: none.
+template <int SIDE, int C>
+__device__ __forceinline__ uint32_t quad_slab(const FusedParams& P, uint32_t i, uint32_t j, uint32_t k0, uint32_t set,
+                                              QuadSlab& f) {
+    const Grid& g = P.g;
+    f.in = 0u;
+    if (!set) return 0u;
+    // The component exists (the update's conditions); nodes k < kmax have it.
+    const bool has = SIDE == 0 ? (C == 0 || i + 1 < g.nx) && (C == 1 || j + 1 < g.ny)
+                               : (C != 0 || i + 1 < g.nx) && (C != 1 || j + 1 < g.ny);
+    const uint32_t kmax = (SIDE == 0 ? C != 2 : C == 2) ? g.nz - 1u : g.nz;
+    const FSlab& s = P.slab[SIDE][C][__ffs((int)set) - 1];
+    f.s = &s;
+    f.at = ((i - s.lo[0]) * (s.hi[1] - s.lo[1]) + (j - s.lo[1])) * (s.hi[2] - s.lo[2]) + (k0 - s.lo[2]);
+    // A slab spans the other axes up to their padding index.
+    if (has && i < s.hi[0] && j < s.hi[1]) {
+        const uint32_t hi = s.hi[2] < kmax ? s.hi[2] : kmax;
+#pragma unroll
+        for (uint32_t e = 0; e < 4u; ++e) f.in |= (k0 + e >= s.lo[2] && k0 + e < hi ? 1u : 0u) << e;
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < 4u; ++e) f.psi[e] = (f.in >> e) & 1u ? s.psi_old[f.at + e] : 0.0f;
+    return set & (set - 1u);
+}
+
+// The corrections of component C by slab f and then those of `rest`, in
+// order: the chain of shell_node on the curl differences the update formed
+// (A along next(C), B along prev(C)).
+template <int SIDE, int C>
+__device__ __forceinline__ void quad_cpml(const FusedParams& P, uint32_t i, uint32_t j, uint32_t k0, QuadSlab f,
+                                          uint32_t rest, Q4& t, const Q4& cf, const Q4& A, const Q4& B) {
+    constexpr uint32_t na = (C + 1) % 3;
+    for (;;) {
+        if (f.in) {
+            const FSlab& s = *f.s;
+            const uint32_t n = s.normal;
+            const uint32_t d = n == 0u ? i - s.lo[0] : (n == 1u ? j - s.lo[1] : k0 - s.lo[2]), dz = n == 2u ? 1u : 0u;
+#pragma unroll
+            for (uint32_t e = 0; e < 4u; ++e) {
+                if (!((f.in >> e) & 1u)) continue;
+                const uint32_t q = d + e * dz;
+                const float v = n == na ? A.v[e] : __fmul_rn(-1.0f, B.v[e]);
+                const float psi = flush(__fadd_rn(__fmul_rn(__ldg(s.b + q), f.psi[e]), __fmul_rn(__ldg(s.a + q), v)));
+                t.v[e] = flush(__fadd_rn(t.v[e], __fmul_rn(SIDE ? cf.v[e] : -cf.v[e], __fadd_rn(__fmul_rn(__ldg(s.k + q), v), psi))));
+                s.psi_new[f.at + e] = psi;
+            }
+        }
+        if (!rest) return;
+        rest = quad_slab<SIDE, C>(P, i, j, k0, rest, f);
+    }
+}
+
 // H update of every dual edge (src/engine/kernel.rs:447-511, 571-618), four
 // z-nodes per thread; with ENERGY each block writes its share of the energy
 // invariant in units of dt/4 (src/engine/kernel.rs:132-244). Entries the
 // update does not write (edges that do not exist, row padding) are stored
 // back as read. OE: openEMS's summation order. Grid: (quads of a plane /
 // kSplitThreads, nx).
-template <bool ENERGY, bool OE, bool ROWCPML = false>
-__device__ __forceinline__ double split_h_quad(const FusedParams& P, uint32_t i, uint32_t q) {
+// CP: the quad's CPML corrections (`bits` as in quad_slab) before the store,
+// their ψ loaded with the update's operands.
+template <bool ENERGY, bool OE, bool ROWCPML = false, bool NC = true, bool CP = false>
+__device__ __forceinline__ double split_h_at(const FusedParams& P, uint32_t i, uint32_t j, uint32_t k0, uint32_t bits = 0) {
     const Grid& g = P.g;
-    uint32_t j = 0, k0 = 0;
     double w = 0.0;
-    if (quad_of(g, q, j, k0) && !in_interior(P.skip, i, j, k0)) {
+    {
         const uint32_t sj = g.pitch, si = g.ny * g.pitch;
         const uint32_t idx = i * si + j * sj + k0;
         const uint32_t row = i * g.ny + j;
@@ -141,14 +211,21 @@ __device__ __forceinline__ double split_h_quad(const FusedParams& P, uint32_t i,
         // Neighbour offsets; 0 where the neighbour does not exist (the value
         // read is then unused).
         const uint32_t oj = jn ? sj : 0u, oi = in_ ? si : 0u, o4 = k0 + 4 < g.nz ? 4u : 0u;
-        const Q4 ux = ldq(P.uo[0] + idx), uy = ldq(P.uo[1] + idx), uz = ldq(P.uo[2] + idx);
-        const Q4 uzj = ldq(P.uo[2] + idx + oj), uxj = ldq(P.uo[0] + idx + oj);
-        const Q4 uzi = ldq(P.uo[2] + idx + oi), uyi = ldq(P.uo[1] + idx + oi);
-        const float uy4 = __ldg(P.uo[1] + idx + o4), ux4 = __ldg(P.uo[0] + idx + o4);
+        const Q4 ux = ldq<NC>(P.uo[0] + idx), uy = ldq<NC>(P.uo[1] + idx), uz = ldq<NC>(P.uo[2] + idx);
+        const Q4 uzj = ldq<NC>(P.uo[2] + idx + oj), uxj = ldq<NC>(P.uo[0] + idx + oj);
+        const Q4 uzi = ldq<NC>(P.uo[2] + idx + oi), uyi = ldq<NC>(P.uo[1] + idx + oi);
+        const float uy4 = ldf<NC>(P.uo[1] + idx + o4), ux4 = ldf<NC>(P.uo[0] + idx + o4);
         const Q4 hx = ldq_rw(P.io[0] + idx), hy = ldq_rw(P.io[1] + idx), hz = ldq_rw(P.io[2] + idx);
         const Q4 dax = ldq(lane_row(P, 6, row) + k0), dbx = ldq(lane_row(P, 9, row) + k0);
         const Q4 day = ldq(lane_row(P, 7, row) + k0), dby = ldq(lane_row(P, 10, row) + k0);
         const Q4 daz = ldq(lane_row(P, 8, row) + k0), dbz = ldq(lane_row(P, 11, row) + k0);
+        QuadSlab f0, f1, f2;
+        uint32_t r0 = 0, r1 = 0, r2 = 0;
+        if (CP) {
+            r0 = quad_slab<0, 0>(P, i, j, k0, bits & 15u, f0);
+            r1 = quad_slab<0, 1>(P, i, j, k0, (bits >> 4) & 15u, f1);
+            r2 = quad_slab<0, 2>(P, i, j, k0, (bits >> 8) & 15u, f2);
+        }
         Q4 nx_ = hx, ny_ = hy, nz_ = hz;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -212,11 +289,38 @@ __device__ __forceinline__ double split_h_quad(const FusedParams& P, uint32_t i,
             }
             row_cpml<0, 2>(P, i, j, k0, mz, nz_, mdbz, A, B);
         }
+        if (CP) {
+            Q4 A, B;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                A.v[e] = __fsub_rn(uzj.v[e], uz.v[e]);
+                B.v[e] = __fsub_rn(e < 3 ? uy.v[e + 1] : uy4, uy.v[e]);
+            }
+            quad_cpml<0, 0>(P, i, j, k0, f0, r0, nx_, dbx, A, B);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                A.v[e] = __fsub_rn(e < 3 ? ux.v[e + 1] : ux4, ux.v[e]);
+                B.v[e] = __fsub_rn(uzi.v[e], uz.v[e]);
+            }
+            quad_cpml<0, 1>(P, i, j, k0, f1, r1, ny_, dby, A, B);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                A.v[e] = __fsub_rn(uyi.v[e], uy.v[e]);
+                B.v[e] = __fsub_rn(uxj.v[e], ux.v[e]);
+            }
+            quad_cpml<0, 2>(P, i, j, k0, f2, r2, nz_, dbz, A, B);
+        }
         if (jn) stq(P.in[0] + idx, nx_);
         if (in_) stq(P.in[1] + idx, ny_);
         if (in_ && jn) stq(P.in[2] + idx, nz_);
     }
     return w;
+}
+template <bool ENERGY, bool OE, bool ROWCPML = false>
+__device__ __forceinline__ double split_h_quad(const FusedParams& P, uint32_t i, uint32_t q) {
+    uint32_t j = 0, k0 = 0;
+    if (!quad_of(P.g, q, j, k0) || in_interior(P.skip, i, j, k0)) return 0.0;
+    return split_h_at<ENERGY, OE, ROWCPML>(P, i, j, k0);
 }
 
 // Grid: (quads of a plane / kSplitThreads, planes): planes i0 .. i0 +
@@ -239,24 +343,29 @@ __global__ void __launch_bounds__(kSplitThreads, ENERGY ? 1 : (ROWCPML ? 4 : 7))
 // E update of every edge (src/engine/kernel.rs:624-697), four z-nodes per
 // thread; OE: openEMS's summation order. Grid: (quads of a plane /
 // kSplitThreads, nx).
-template <bool OE, bool ROWCPML = false>
-__device__ __forceinline__ void split_e_quad(const FusedParams& P, uint32_t i, uint32_t q) {
+template <bool OE, bool ROWCPML = false, bool NC = true, bool CP = false>
+__device__ __forceinline__ void split_e_at(const FusedParams& P, uint32_t i, uint32_t j, uint32_t k0, uint32_t bits = 0) {
     const Grid& g = P.g;
-    uint32_t j = 0, k0 = 0;
-    if (!quad_of(g, q, j, k0) || in_interior(P.skip, i, j, k0)) return;
     const uint32_t sj = g.pitch, si = g.ny * g.pitch;
     const uint32_t idx = i * si + j * sj + k0;
     const uint32_t row = i * g.ny + j;
-    const Q4 ix = ldq(P.in[0] + idx), iy = ldq(P.in[1] + idx), iz = ldq(P.in[2] + idx);
+    const Q4 ix = ldq<NC>(P.in[0] + idx), iy = ldq<NC>(P.in[1] + idx), iz = ldq<NC>(P.in[2] + idx);
     // Neighbours below the node; zero on the low faces (no edge there).
-    const Q4 izj = j > 0 ? ldq(P.in[2] + idx - sj) : zq(), ixj = j > 0 ? ldq(P.in[0] + idx - sj) : zq();
-    const Q4 izi = i > 0 ? ldq(P.in[2] + idx - si) : zq(), iyi = i > 0 ? ldq(P.in[1] + idx - si) : zq();
-    const float iym = k0 > 0 ? __ldg(P.in[1] + idx - 1) : 0.0f, ixm = k0 > 0 ? __ldg(P.in[0] + idx - 1) : 0.0f;
+    const Q4 izj = j > 0 ? ldq<NC>(P.in[2] + idx - sj) : zq(), ixj = j > 0 ? ldq<NC>(P.in[0] + idx - sj) : zq();
+    const Q4 izi = i > 0 ? ldq<NC>(P.in[2] + idx - si) : zq(), iyi = i > 0 ? ldq<NC>(P.in[1] + idx - si) : zq();
+    const float iym = k0 > 0 ? ldf<NC>(P.in[1] + idx - 1) : 0.0f, ixm = k0 > 0 ? ldf<NC>(P.in[0] + idx - 1) : 0.0f;
     const Q4 ex = ldq_rw(P.uo[0] + idx), ey = ldq_rw(P.uo[1] + idx), ez = ldq_rw(P.uo[2] + idx);
     const Q4 cax = ldq(lane_row(P, 0, row) + k0), cbx = ldq(lane_row(P, 3, row) + k0);
     const Q4 cay = ldq(lane_row(P, 1, row) + k0), cby = ldq(lane_row(P, 4, row) + k0);
     const Q4 caz = ldq(lane_row(P, 2, row) + k0), cbz = ldq(lane_row(P, 5, row) + k0);
     const bool xi = i + 1 < g.nx, yj = j + 1 < g.ny;
+    QuadSlab f0, f1, f2;
+    uint32_t r0 = 0, r1 = 0, r2 = 0;
+    if (CP) {
+        r0 = quad_slab<1, 0>(P, i, j, k0, (bits >> 12) & 15u, f0);
+        r1 = quad_slab<1, 1>(P, i, j, k0, (bits >> 16) & 15u, f1);
+        r2 = quad_slab<1, 2>(P, i, j, k0, (bits >> 20) & 15u, f2);
+    }
     Q4 nx_ = ex, ny_ = ey, nz_ = ez;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -297,9 +406,35 @@ __device__ __forceinline__ void split_e_quad(const FusedParams& P, uint32_t i, u
         }
         row_cpml<1, 2>(P, i, j, k0, mz, nz_, cbz, A, B);
     }
+    if (CP) {
+        Q4 A, B;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            A.v[e] = __fsub_rn(iz.v[e], izj.v[e]);
+            B.v[e] = __fsub_rn(iy.v[e], e > 0 ? iy.v[e - 1] : iym);
+        }
+        quad_cpml<1, 0>(P, i, j, k0, f0, r0, nx_, cbx, A, B);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            A.v[e] = __fsub_rn(ix.v[e], e > 0 ? ix.v[e - 1] : ixm);
+            B.v[e] = __fsub_rn(iz.v[e], izi.v[e]);
+        }
+        quad_cpml<1, 1>(P, i, j, k0, f1, r1, ny_, cby, A, B);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            A.v[e] = __fsub_rn(iy.v[e], iyi.v[e]);
+            B.v[e] = __fsub_rn(ix.v[e], ixj.v[e]);
+        }
+        quad_cpml<1, 2>(P, i, j, k0, f2, r2, nz_, cbz, A, B);
+    }
     if (xi) stq(P.un[0] + idx, nx_);
     if (yj) stq(P.un[1] + idx, ny_);
     stq(P.un[2] + idx, nz_);
+}
+template <bool OE, bool ROWCPML = false>
+__device__ __forceinline__ void split_e_quad(const FusedParams& P, uint32_t i, uint32_t q) {
+    uint32_t j = 0, k0 = 0;
+    if (quad_of(P.g, q, j, k0) && !in_interior(P.skip, i, j, k0)) split_e_at<OE, ROWCPML>(P, i, j, k0);
 }
 
 template <bool OE = false, bool ROWCPML = false>

@@ -337,7 +337,8 @@ ems_status ems_gpu_upload_field(ems_gpu* h, int field, int axis, const float* ho
 ems_status ems_gpu_samples(ems_gpu* h, size_t op, int which, double* out, size_t cap, size_t* n);
 
 /* The latest sample of a series of ems_gpu_samples (EMS_ERR_INVALID if the
- * series is empty): one device-to-host read of 8 bytes. */
+ * series is empty): the steps mirror it in host memory, so this waits for
+ * them and reads it there. */
 ems_status ems_gpu_last_sample(ems_gpu* h, size_t op, int which, double* out);
 
 /* Overwrites amplitudes [first, first + n) of the source table of operator

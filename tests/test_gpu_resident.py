@@ -1,0 +1,117 @@
+"""Resident steps (many steps per launch, the automatic schedule on small
+grids) against the split schedule's kernels, one step at a time: every
+operator they run, odd and tiny grids, short and long runs, energy steps,
+uploads, amplitudes fed while running and schedule switches between them.
+Fields and series must agree bit for bit."""
+import numpy as np
+import pytest
+
+import ems_b200 as E
+from ems_b200 import workloads as W
+from helpers import assert_fields_equal, graded, mixed_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _cavity(n, kappa=0.003, layers=0):
+    m = E.Model(*[graded(q * 1e-3, q, 0.2) for q in n])
+    h = [q // 2 for q in n]
+    m.fill(m.cells().box([0, 0, 0], [n[0], n[1], max(1, h[2])]), m.material(eps_r=3.0, kappa=kappa))
+    m.build(courant=0.99)
+    if layers:
+        m.add_cpml([layers] * 6)
+    amp = np.sin(0.3 * np.arange(400))
+    src = m.add_source_table(E.SOFT_E, [(E.Z, (h[0], h[1], 0), 1.0)], amp)
+    m.add_source_table(E.HARD_E, [(E.X, (0, h[1], h[2]), 0.5)], amp[::-1].copy())
+    ops = [m.add_probe(E.VOLTAGE, [(E.Z, (h[0], j, 0), 0.5 + j) for j in range(1, n[1])], interval=3),
+           m.add_probe(E.CURRENT, [(E.Y, (0, j % n[1], 0), 1.0) for j in range(70)], f32_sum=True),
+           m.add_probe(E.VOLTAGE, [(E.X, (0, 1, 1), 1.0)])]
+    return m, src, [(op, 0) for op in ops]
+
+
+def _mixed(scheme):
+    m, ops = mixed_model(scheme=scheme, steps=400)
+    return m, None, [(ops["pv"], 0), (ops["pi"], 0), (ops["pe"], 0), (ops["port"], 0), (ops["port"], 1),
+                     (ops["port"], 2)]
+
+
+def _lumped():
+    m, src, s = _cavity((14, 9, 11), layers=2)
+    amp = np.cos(0.2 * np.arange(300))
+    a = m.add_lumped(E.Z, [4, 4, 2], [4, 6, 5], r=50.0, l=2e-9, c=1e-12, series=True, record=True, amp=amp)
+    b = m.add_lumped_port_table(E.X, [6, 2, 3], [9, 2, 3], 75.0, amp)
+    return m, src, s + [(a, 0), (b, 0), (b, 1), (b, 2)]
+
+
+CASES = {
+    "mixed_trapezoidal": lambda: _mixed(E.TRAPEZOIDAL), "mixed_leapfrog": lambda: _mixed(E.LEAPFROG),
+    "tiny": lambda: _cavity((2, 2, 2)), "flat": lambda: _cavity((41, 3, 2)), "rows_33": lambda: _cavity((7, 12, 33)),
+    "cpml_overlap": lambda: _cavity((9, 9, 9), layers=4), "cpml_odd": lambda: _cavity((31, 22, 45), layers=5),
+    "lumped": _lumped,
+}
+
+
+@pytest.mark.parametrize("curl", [0, 1])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_resident_equals_split(name, curl):
+    m, src, series = CASES[name]()
+    g, s = E.Engine(m), E.Engine(m)
+    s.set_schedule(4)
+    for e in (g, s):
+        e.set_curl_order(curl)
+    rng = np.random.default_rng(5)
+    before = g.launches
+    for e in (g, s):
+        e.run(60)
+    assert g.launches - before == 1 and g.schedule == 4
+    assert_fields_equal(g, s, f"{name}: 60 steps")
+    for n in (1, 2, 7, 0, 31):
+        if src is not None:
+            v = rng.standard_normal(3)
+            for e in (g, s):
+                e.source_amplitude(src, e.timestep, v)
+        w = [e.step_with_energy() for e in (g, s)]
+        assert abs(w[0] - w[1]) <= 1e-12 * abs(w[1])
+        u = rng.standard_normal(g.nodes).astype(np.float32)
+        for e in (g, s):
+            e.set_field(n % 2, n % 3, u)
+            e.run(n)
+    g.set_schedule(1)
+    g.run(3)
+    g.set_schedule(0)
+    g.run(5)
+    s.run(8)
+    assert g.timestep == s.timestep
+    assert_fields_equal(g, s, name)
+    for op, which in series:
+        x, y = g.samples(op, which), s.samples(op, which)
+        assert x.size == y.size > 0
+        assert np.array_equal(x.view(np.uint64), y.view(np.uint64)), (name, op, which)
+
+
+def test_batch_of_more_models_than_blocks():
+    """More models than resident blocks (two per SM): a block takes several,
+    each for the whole run."""
+    sizes = [(3 + q % 5, 4 + q % 3, 2 + q % 7) for q in range(320)]
+    built = [_cavity(n)[0] for n in sizes]
+    b = E.Batch(built, max_steps=200)
+    b.run(20)
+    for q in (0, 3, 317):
+        b.set_active(q, False)
+    b.run(13)
+    for q in (0, 1, 3, 100, 317, 319):
+        g = E.Engine(built[q])
+        g.set_schedule(4)
+        g.run(20 if q in (0, 3, 317) else 33)
+        assert b.timestep(q) == g.timestep
+        for f in range(2):
+            for a in range(3):
+                assert np.array_equal(b.field(q, f, a).view(np.uint32), g.field(f, a).view(np.uint32)), (q, f, a)
+
+
+def test_large_grids_keep_the_split_kernels():
+    w = W.vacuum_box(n=224, cpml=8, steps=10)
+    g = E.Engine(w.model)
+    before = g.launches
+    g.run(4)
+    assert g.launches - before > 4 * 4
