@@ -1022,8 +1022,7 @@ class Engine:
         n = int(np.prod(dims))
         out = np.empty(n * 6, dtype=np.float64)
         self._ck(self._lib.ems_gpu_freq_dump_read(self._h, dump, k, out.ctypes.data, out.size))
-        c = out[0::2] + 1j * out[1::2]
-        return c.reshape(*dims, 3)
+        return out.view(np.complex128).reshape(*dims, 3)
 
     def autotune(self, cache_path: str) -> None:
         """Schedule autotuning (``ems_gpu_autotune``): cached pick, or timed

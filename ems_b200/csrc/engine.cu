@@ -88,6 +88,7 @@ struct ems_gpu {
     size_t n_partials = 0;
     double* d_energy = nullptr;   // [0] field part, [1 + q] the q-th operator that holds energy
     double* shares = nullptr;     // first pass of a long sum (kSumBlocks)
+    int* flags = nullptr;         // pinned copy of the status and divergence flags
     int* diverged = nullptr;      // set on the device where a marching step writes a non-finite value
     uint64_t test_wait_ns = 0;    // ems_gpu_test_wait_timeout: the next marching step's waits run out
     struct CpmlDev {
@@ -220,6 +221,13 @@ struct ems_gpu {
         bool late_h = false;              // no hook writes i: current probes wait for the electric hooks
         double* mail = nullptr;           // pinned, 3 per operator
     } hooks;
+    // Pinned staging of field downloads, two buffers of `cap` floats, made on
+    // the first download.
+    struct Staging {
+        float* p[2] = {nullptr, nullptr};
+        cudaEvent_t ready[2] = {nullptr, nullptr};
+        size_t cap = 0;
+    } staging;
     // Resident steps (resident.cuh): the automatic schedule's form of the
     // split schedule on small grids, many steps per launch.
     struct Resident {
@@ -2054,7 +2062,9 @@ ems_status serial_post_e(ems_gpu* h, const Fields& f) {
 
 extern "C" {
 
-ems_status ems_gpu_create(const ems_engine_desc* d, int device, ems_gpu** out) {
+// alone: an engine that steps by itself; a batch's models need no tables of
+// their own for it.
+static ems_status create_engine(const ems_engine_desc* d, int device, bool alone, ems_gpu** out) {
     if (!d || !out) return EMS_ERR_INVALID;
     *out = nullptr;
     if (d->nodes[0] < 2 || d->nodes[1] < 2 || d->nodes[2] < 2 || !(d->dt > 0.0)) return EMS_ERR_INVALID;
@@ -2333,13 +2343,20 @@ ems_status ems_gpu_create(const ems_engine_desc* d, int device, ems_gpu** out) {
         ems_status st = setup_fused(h.get(), d);
         if (st) return st;
     }
-    if (ems_status st = setup_hooks(h.get())) return st;
-    if (ems_status st = setup_resident(h.get())) return st;
+    if (alone) {
+        if (ems_status st = setup_hooks(h.get())) return st;
+        if (ems_status st = setup_resident(h.get())) return st;
+    }
     if (check(h.get(), cudaStreamSynchronize(h->stream), "create")) return EMS_ERR_CUDA;
     *out = h.release();
     return EMS_OK;
 }
 
+ems_status ems_gpu_create(const ems_engine_desc* d, int device, ems_gpu** out) {
+    return create_engine(d, device, true, out);
+}
+
+static void release_staging(ems_gpu* h);
 ems_status ems_gpu_destroy(ems_gpu* h) {
     if (!h) return EMS_ERR_INVALID;
     cudaSetDevice(h->device);
@@ -2350,6 +2367,8 @@ ems_status ems_gpu_destroy(ems_gpu* h) {
     for (cudaEvent_t e : h->ev_free) cudaEventDestroy(e);
     h->bufs.clear();
     if (h->hooks.mail) cudaFreeHost(h->hooks.mail);
+    release_staging(h);
+    if (h->flags) cudaFreeHost(h->flags);
     cudaStreamDestroy(h->stream);
     delete h;
     return EMS_OK;
@@ -2681,13 +2700,18 @@ ems_status ems_gpu_autotune(ems_gpu* h, const char* cache_path) {
 // host's next check, as the reference's stepping itself never fails
 // (src/engine/mod.rs:456-458).
 static ems_status device_status(ems_gpu* h) {
-    int st[2] = {0, 0};
-    if (h->status &&
-        check(h, cudaMemcpyAsync(&st[0], h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status"))
+    // Pinned, so that the two copies join the caller's work in the stream and
+    // one wait covers all of it.
+    if (!h->flags && check(h, cudaHostAlloc((void**)&h->flags, 2 * sizeof(int), cudaHostAllocDefault), "status"))
         return EMS_ERR_CUDA;
-    if (check(h, cudaMemcpyAsync(&st[1], h->diverged, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status"))
+    h->flags[0] = 0;
+    if (h->status &&
+        check(h, cudaMemcpyAsync(&h->flags[0], h->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status"))
+        return EMS_ERR_CUDA;
+    if (check(h, cudaMemcpyAsync(&h->flags[1], h->diverged, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status"))
         return EMS_ERR_CUDA;
     if (check(h, cudaStreamSynchronize(h->stream), "status")) return EMS_ERR_CUDA;
+    const int st[2] = {h->flags[0], h->flags[1]};
     if (st[0] || st[1]) {
         if (h->status) cudaMemsetAsync(h->status, 0, sizeof(int), h->stream);
         cudaMemsetAsync(h->diverged, 0, sizeof(int), h->stream);
@@ -2728,11 +2752,11 @@ ems_status ems_gpu_step_with_energy(ems_gpu* h, double* energy) {
     if (check(h, cudaMemcpyAsync(w.data(), h->d_energy, w.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
               "energy"))
         return EMS_ERR_CUDA;
-    if (check(h, cudaStreamSynchronize(h->stream), "energy")) return EMS_ERR_CUDA;
+    st = device_status(h);
     double w_ops = 0.0;
     for (size_t q = 0; q < n_ops; ++q) w_ops += w[1 + q];
     *energy = 0.25 * h->dt * w[0] + w_ops;
-    return device_status(h);
+    return st;
 }
 
 ems_status ems_gpu_timestep(const ems_gpu* h, uint64_t* n) {
@@ -2741,16 +2765,81 @@ ems_status ems_gpu_timestep(const ems_gpu* h, uint64_t* n) {
     return EMS_OK;
 }
 
+// Floats of a staging buffer (2 MiB: pinning takes some 1 ms per MiB, paid by
+// the first download), and the share of a copy below which another thread
+// costs more than it saves (a thread's start takes some 20 us, in which one
+// core copies 0.2 MB into fresh pages). A 36 MB set of fields of 132x118x94
+// nodes: 17 ms with strided copies, 3.6 ms through the staging.
+static constexpr size_t kStageFloats = 512u << 10, kCopyShare = 128u << 10;
+
+static void release_staging(ems_gpu* h) {
+    for (int q = 0; q < 2; ++q) {
+        if (h->staging.p[q]) cudaFreeHost(h->staging.p[q]);
+        if (h->staging.ready[q]) cudaEventDestroy(h->staging.ready[q]);
+        h->staging.p[q] = nullptr;
+        h->staging.ready[q] = nullptr;
+    }
+}
+
+// Copies n floats, on up to four threads: the destination is often memory
+// that the caller has just obtained, whose first touch costs more than the
+// copy.
+static void copy_out(float* dst, const float* src, size_t n) {
+    const size_t parts = std::max<size_t>(1, std::min<size_t>(4, n / kCopyShare)), each = (n + parts - 1) / parts;
+    std::thread th[4];
+    size_t done = each;  // the first part is this thread's
+    try {
+        for (size_t q = 1; q < parts; ++q, done += each)
+            th[q] = std::thread([=] { std::memcpy(dst + q * each, src + q * each, (std::min(n, (q + 1) * each) - q * each) * sizeof(float)); });
+    } catch (...) {
+        // No thread to be had: what is left is copied here.
+        if (done < n) std::memcpy(dst + done, src + done, (n - done) * sizeof(float));
+    }
+    std::memcpy(dst, src, std::min(n, each) * sizeof(float));
+    for (auto& t : th)
+        if (t.joinable()) t.join();
+}
+
 ems_status ems_gpu_download_field(ems_gpu* h, int field, int axis, float* host) {
     if (!h || !host || field < 0 || field > 1 || axis < 0 || axis > 2) return EMS_ERR_INVALID;
     cudaSetDevice(h->device);
     const Grid& g = h->g;
-    float* src = field == 0 ? h->u[axis] : h->i[axis];
-    if (check(h, cudaMemcpy2DAsync(host, g.nz * sizeof(float), src, g.pitch * sizeof(float), g.nz * sizeof(float),
-                                   (size_t)g.nx * g.ny, cudaMemcpyDeviceToHost, h->stream),
-              "download"))
-        return EMS_ERR_CUDA;
-    if (check(h, cudaStreamSynchronize(h->stream), "download")) return EMS_ERR_CUDA;
+    const float* src = field == 0 ? h->u[axis] : h->i[axis];
+    auto& st = h->staging;
+    if (!st.p[0]) {
+        st.cap = std::min<size_t>(g.n, kStageFloats);
+        for (int q = 0; q < 2 && st.cap; ++q)
+            if (cudaHostAlloc((void**)&st.p[q], st.cap * sizeof(float), cudaHostAllocMapped) != cudaSuccess ||
+                cudaEventCreateWithFlags(&st.ready[q], cudaEventDisableTiming) != cudaSuccess)
+                st.cap = 0;
+    }
+    if (!st.cap) {  // no pinned memory to be had
+        cudaGetLastError();
+        release_staging(h);
+        if (check(h, cudaMemcpy2DAsync(host, g.nz * sizeof(float), src, g.pitch * sizeof(float), g.nz * sizeof(float),
+                                       (size_t)g.nx * g.ny, cudaMemcpyDeviceToHost, h->stream),
+                  "download") ||
+            check(h, cudaStreamSynchronize(h->stream), "download"))
+            return EMS_ERR_CUDA;
+        return device_status(h);
+    }
+    // The device fills one buffer while the host empties the other.
+    const uint64_t chunks = (g.n + st.cap - 1) / st.cap;
+    auto size = [&](uint64_t c) { return (size_t)std::min<uint64_t>(st.cap, g.n - c * st.cap); };
+    auto fill = [&](uint64_t c) {
+        const uint64_t e = c * st.cap;
+        const unsigned nb = std::min(blocks_for(size(c), 256), 148u * 8u);
+        k_unpad<<<nb, 256, 0, h->stream>>>(src, g.nz, g.pitch, (uint32_t)(e / g.nz), (uint32_t)(e % g.nz), (uint32_t)size(c),
+                                          st.p[c & 1]);
+        ++h->launches;
+        return check(h, cudaEventRecord(st.ready[c & 1], h->stream), "download");
+    };
+    if (fill(0)) return EMS_ERR_CUDA;
+    for (uint64_t c = 0; c < chunks; ++c) {
+        if (c + 1 < chunks && fill(c + 1)) return EMS_ERR_CUDA;
+        if (check(h, cudaEventSynchronize(st.ready[c & 1]), "download")) return EMS_ERR_CUDA;
+        copy_out(host + c * st.cap, st.p[c & 1], size(c));
+    }
     return device_status(h);
 }
 
@@ -2792,12 +2881,12 @@ ems_status ems_gpu_samples(ems_gpu* h, size_t op, int which, double* out, size_t
         return fail(h, EMS_ERR_INVALID, "no such series");
     }
     *n = cnt;
-    if (out && cnt && cap) {
+    if (!out) return EMS_OK;  // the count alone: known here
+    if (cnt && cap) {
         size_t m = std::min(cap, cnt);
         if (check(h, cudaMemcpyAsync(out, src, m * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "samples"))
             return EMS_ERR_CUDA;
     }
-    if (check(h, cudaStreamSynchronize(h->stream), "samples")) return EMS_ERR_CUDA;
     return device_status(h);
 }
 
@@ -2991,6 +3080,7 @@ struct ems_batch {
     std::vector<std::array<uint32_t, BK_KINDS>> blocks;  // each model's blocks per kernel kind
     BatchTable T{};
     std::vector<int> active;
+    std::vector<uint64_t> done;              // completed steps of each model (d_steps)
     int* d_active = nullptr;
     uint32_t* d_steps = nullptr;
     BatchSource* d_src[2] = {nullptr, nullptr};  // [0] H sources, [1] E sources
@@ -3037,6 +3127,7 @@ struct ems_batch {
         uint32_t* list = nullptr;
         uint32_t* bars = nullptr;       // two sets of `fit` counters
         int* status = nullptr;
+        int* flag = nullptr;            // pinned copy of *status
         int flip = 0;
         std::vector<uint4> h_blocks;
         std::vector<uint2> h_gangs;
@@ -3304,7 +3395,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
             return EMS_ERR_INVALID;
         }
         ems_gpu* h = nullptr;
-        ems_status st = ems_gpu_create(d, device, &h);
+        ems_status st = create_engine(d, device, false, &h);
         if (st) return st;
         b->models.push_back(h);
         if (!h->tables_ok) {
@@ -3439,6 +3530,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
     }
     b->poles_first = pf == 1;
     b->active.assign(n_models, 1);
+    b->done.assign(n_models, 0);
     BatchTable& T = b->T;
     T.n = (uint32_t)n_models;
     T.models = b->upload(hm.data(), n_models);
@@ -3499,6 +3591,7 @@ ems_status ems_batch_destroy(ems_batch* b) {
     if (b->step_graph) cudaGraphExecDestroy(b->step_graph);
     if (b->energy_graph) cudaGraphExecDestroy(b->energy_graph);
     b->bufs.clear();
+    if (b->res.flag) cudaFreeHost(b->res.flag);
     for (ems_gpu* h : b->models) ems_gpu_destroy(h);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -3542,15 +3635,22 @@ static ems_status batch_tune_step(ems_batch* b) {
     return EMS_OK;
 }
 
+static void batch_count(ems_batch* b, uint64_t n) {
+    for (size_t m = 0; m < b->done.size(); ++m)
+        if (b->active[m]) b->done[m] += n;
+}
+
 // EMS_ERR_TIMEOUT if a wait of the resident kernel ran out since the last check.
 static ems_status batch_status(ems_batch* b) {
-    if (!b->res.ok) return EMS_OK;
-    int v = 0;
-    if (cudaMemcpyAsync(&v, b->res.status, sizeof v, cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
+    auto& r = b->res;
+    if (!r.ok) return EMS_OK;
+    if (!r.flag && cudaHostAlloc((void**)&r.flag, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
+        return bfail(b, EMS_ERR_CUDA, "status");
+    if (cudaMemcpyAsync(r.flag, r.status, sizeof(int), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, EMS_ERR_CUDA, "status");
-    if (!v) return EMS_OK;
-    cudaMemsetAsync(b->res.status, 0, sizeof v, b->stream);
+    if (!*r.flag) return EMS_OK;
+    cudaMemsetAsync(r.status, 0, sizeof(int), b->stream);
     return bfail(b, EMS_ERR_TIMEOUT, "a bounded wait of the resident kernel ran out");
 }
 
@@ -3562,13 +3662,17 @@ ems_status ems_batch_run(ems_batch* b, uint64_t n) {
             const uint64_t k = std::min(n - q, kResidentSteps);
             ems_status st = batch_resident(b, k);
             if (st) return st;
+            batch_count(b, k);
             q += k - 1;
-        } else if (b->tune.active) {
+            continue;
+        }
+        if (b->tune.active) {
             ems_status st = batch_tune_step(b);
             if (st) return st;
         } else if (cudaGraphLaunch(b->step_graph, b->stream) != cudaSuccess) {
             return bfail(b, EMS_ERR_CUDA, "graph launch");
         }
+        batch_count(b, 1);
     }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? EMS_OK : bfail(b, EMS_ERR_CUDA, cudaGetErrorString(e));
@@ -3610,6 +3714,7 @@ ems_status ems_batch_step_with_energy(ems_batch* b, double* energies) {
         cudaMemcpyAsync(energies, b->energies, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bfail(b, EMS_ERR_CUDA, "energy step");
+    batch_count(b, 1);
     return batch_status(b);
 }
 
@@ -3638,30 +3743,24 @@ ems_status ems_batch_set_active(ems_batch* b, size_t model, int active) {
 
 ems_status ems_batch_timestep(ems_batch* b, size_t model, uint64_t* n) {
     if (!b || !n || model >= b->models.size()) return EMS_ERR_INVALID;
-    cudaSetDevice(b->device);
-    uint32_t v = 0;
-    if (cudaMemcpyAsync(&v, b->d_steps + model, sizeof(v), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
-        cudaStreamSynchronize(b->stream) != cudaSuccess)
-        return bfail(b, EMS_ERR_CUDA, "timestep");
-    *n = v;
-    return batch_status(b);
+    *n = b->done[model];
+    return EMS_OK;
 }
 
 ems_status ems_batch_samples(ems_batch* b, size_t model, size_t op, int which, double* out, size_t cap, size_t* n) {
     if (!b || !n || model >= b->models.size()) return EMS_ERR_INVALID;
-    uint64_t steps = 0;
-    ems_status st = ems_batch_timestep(b, model, &steps);
-    if (st) return st;
+    cudaSetDevice(b->device);
+    const uint64_t steps = b->done[model];
     for (const auto& sr : b->series) {
         if (sr.model != model || sr.op != op || sr.which != which) continue;
         const uint64_t count = std::min<uint64_t>(steps ? (steps - 1) / sr.interval + 1 : 0, sr.cap);
         *n = (size_t)count;
         if (!out) return EMS_OK;
         const size_t k = std::min<size_t>(cap, (size_t)count);
-        if (k && (cudaMemcpyAsync(out, sr.dev, k * sizeof(double), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
-                  cudaStreamSynchronize(b->stream) != cudaSuccess))
+        if (k && cudaMemcpyAsync(out, sr.dev, k * sizeof(double), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess)
             return bfail(b, EMS_ERR_CUDA, "samples");
-        return EMS_OK;
+        if (b->res.ok) return batch_status(b);
+        return cudaStreamSynchronize(b->stream) == cudaSuccess ? EMS_OK : bfail(b, EMS_ERR_CUDA, "samples");
     }
     return bfail(b, EMS_ERR_INVALID, "no such series");
 }

@@ -692,6 +692,17 @@ __global__ void __launch_bounds__(256) k_snapshot(const __grid_constant__ DumpDe
     out[3 * (size_t)p + 2] = x[2];
 }
 
+// Elements [0, n) of a field from its row row0, place k0 on, without the row
+// padding (reference layout), into host-visible memory: coalesced writes over
+// the bus in place of a strided copy of one short row after another.
+__global__ void __launch_bounds__(256) k_unpad(const float* src, uint32_t nz, uint32_t pitch, uint32_t row0, uint32_t k0,
+                                               uint32_t n, float* dst) {
+    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < n; t += gridDim.x * 256u) {
+        const uint32_t x = k0 + t, r = x / nz;
+        dst[t] = src[(size_t)(row0 + r) * pitch + (x - r * nz)];
+    }
+}
+
 __device__ __forceinline__ double frac_toward_zero(double x) { return x - trunc(x); }
 
 __global__ void __launch_bounds__(256) k_dump(const __grid_constant__ DumpDev d, double m) {
