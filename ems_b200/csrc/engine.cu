@@ -277,6 +277,12 @@ struct ems_gpu {
     // step with no field upload since.
     bool fold_prev[2] = {false, false};
     bool prev_e_valid = false;
+    // openEMS PML layers: nothing but the layers' own update writes their
+    // edges of a side (E, H) after the field update, so the start value that
+    // update leaves is the one the refresh would take (upml_own); the E side's
+    // only after a step with no field upload since.
+    bool upml_fold[2] = {false, false};
+    bool upml_e_valid = false;
     double* qpartials = nullptr;    // energy shares of the split H update
     size_t n_qpartials = 0;
     uint32_t* counter = nullptr;
@@ -1574,6 +1580,44 @@ void launch_resident(const ResArgs& A, bool oe, unsigned grid, unsigned threads,
                                      dim3(threads), args, 0, s);
 }
 
+// Whether nothing but its own layer update writes an edge of side `side` of an
+// openEMS PML after the field update (see upml_fold): one such operator, no
+// other slab operator and no conducting sheet, and no lumped element, source
+// or Mur edge of that field on a layer edge.
+bool upml_own(const ems_engine_desc* d, int side) {
+    const ems_upml* t = nullptr;
+    for (size_t k = 0; k < d->n_ops; ++k) {
+        const int kind = d->ops[k].kind;
+        if (kind == EMS_OP_CPML || kind == EMS_OP_POLES || kind == EMS_OP_SHEET) return false;
+        if (kind != EMS_OP_UPML) continue;
+        if (t) return false;
+        t = (const ems_upml*)d->ops[k].table;
+    }
+    if (!t || !t->n[side]) return false;
+    const uint64_t n = d->nodes[0] * d->nodes[1] * d->nodes[2];
+    std::vector<bool> layer(3 * n, false);
+    for (size_t e = 0; e < t->n[side]; ++e) layer[t->axis[side][e] * n + t->node[side][e]] = true;
+    auto hit = [&](uint64_t axis, uint64_t node) { return axis < 3 && node < n && layer[axis * n + node]; };
+    for (size_t k = 0; k < d->n_ops; ++k) {
+        const int kind = d->ops[k].kind;
+        if (kind == EMS_OP_SOURCE) {
+            const auto* s = (const ems_source*)d->ops[k].table;
+            if ((s->kind == EMS_SOFT_E || s->kind == EMS_HARD_E) != (side == 0)) continue;
+            for (size_t e = 0; e < s->n_edges; ++e)
+                if (hit(s->axis[e], s->node[e])) return false;
+        } else if (kind == EMS_OP_LUMPED && side == 0) {
+            const auto* l = (const ems_lumped*)d->ops[k].table;
+            for (size_t e = 0; e < l->n_edges; ++e)
+                if (hit((uint64_t)l->axis, l->node[e])) return false;
+        } else if (kind == EMS_OP_MUR && side == 0) {
+            const auto* m = (const ems_mur*)d->ops[k].table;
+            for (size_t e = 0; e < m->n; ++e)
+                if (hit(m->axis[e], m->node[e])) return false;
+        }
+    }
+    return true;
+}
+
 // The table of the serial hooks one block can run (every probe; sources and
 // lumped elements of few edges), and the host mirror of the newest samples.
 ems_status setup_hooks(ems_gpu* h) {
@@ -1652,6 +1696,7 @@ ems_status run_resident(ems_gpu* h, uint64_t n) {
     ++h->launches;
     h->step += n;
     h->prev_e_valid = h->fold_prev[0];
+    h->upml_e_valid = true;
     return EMS_OK;
 }
 
@@ -1752,9 +1797,11 @@ ems_status run_step(ems_gpu* h, bool energy) {
             }
         } else if (op.kind == EMS_OP_UPML) {
             // upml.rs:443-454: E start values from u, then the H layer update.
-            if (const uint32_t n = op.upml[0].n + op.upml[1].n) {
-                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], op.upml[0], f.i[0], f.i[1],
-                                                              f.i[2], op.upml[1]);
+            UpmlSideDev fresh = op.upml[0];
+            if (h->upml_fold[0] && h->upml_e_valid) fresh.n = 0;
+            if (const uint32_t n = fresh.n + op.upml[1].n) {
+                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], fresh, f.i[0], f.i[1], f.i[2],
+                                                              op.upml[1]);
                 ++h->launches;
             }
         }
@@ -1805,9 +1852,11 @@ ems_status run_step(ems_gpu* h, bool energy) {
             }
         } else if (op.kind == EMS_OP_UPML) {
             // upml.rs:456-464: H start values from i, then the E layer update.
-            if (const uint32_t n = op.upml[0].n + op.upml[1].n) {
-                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.i[0], f.i[1], f.i[2], op.upml[1], f.u[0], f.u[1],
-                                                              f.u[2], op.upml[0]);
+            UpmlSideDev fresh = op.upml[1];
+            if (h->upml_fold[1]) fresh.n = 0;
+            if (const uint32_t n = fresh.n + op.upml[0].n) {
+                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.i[0], f.i[1], f.i[2], fresh, f.u[0], f.u[1], f.u[2],
+                                                              op.upml[0]);
                 ++h->launches;
             }
         }
@@ -1815,6 +1864,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
     st = serial_post_e(h, f);
     if (st) return st;
     if (split) h->prev_e_valid = h->fold_prev[0];
+    h->upml_e_valid = true;
     ++h->step;
     return EMS_OK;
 }
@@ -2344,7 +2394,9 @@ static ems_status create_engine(const ems_engine_desc* d, int device, bool alone
         if (st) return st;
     }
     if (alone) {
-        if (ems_status st = setup_hooks(h.get())) return st;
+        if (h->has_upml)
+        for (int side = 0; side < 2; ++side) h->upml_fold[side] = upml_own(d, side);
+    if (ems_status st = setup_hooks(h.get())) return st;
         if (ems_status st = setup_resident(h.get())) return st;
     }
     if (check(h.get(), cudaStreamSynchronize(h->stream), "create")) return EMS_ERR_CUDA;
@@ -2847,7 +2899,7 @@ ems_status ems_gpu_upload_field(ems_gpu* h, int field, int axis, const float* ho
     if (!h || !host || field < 0 || field > 1 || axis < 0 || axis > 2) return EMS_ERR_INVALID;
     cudaSetDevice(h->device);
     const Grid& g = h->g;
-    if (field == 0) h->prev_e_valid = false;  // the saved electric values are captured again
+    if (field == 0) h->prev_e_valid = h->upml_e_valid = false;  // the saved electric values are captured again
     // Both buffers of a double-buffered field get the values (the padding
     // entries the kernels read as zero stay equal in both).
     float* dsts[2] = {field == 0 ? h->u[axis] : h->i[axis], field == 0 ? h->u2[axis] : h->i2[axis]};

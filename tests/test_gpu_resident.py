@@ -115,3 +115,43 @@ def test_large_grids_keep_the_split_kernels():
     before = g.launches
     g.run(4)
     assert g.launches - before > 4 * 4
+
+
+def test_engines_on_several_threads():
+    """Resident engines and a batch stepping at once from threads of their
+    own (each launch fills the device): every result as when alone."""
+    import threading
+
+    m, _, series = _cavity((40, 33, 47), layers=5)
+    small = [_cavity((9 + q, 11, 13))[0] for q in range(6)]
+    want = E.Engine(m)
+    want.run(600)
+    alone = [E.Engine(x) for x in small]
+    for e in alone:
+        e.run(600)
+    engines = [E.Engine(m) for _ in range(3)]
+    b = E.Batch(small, max_steps=700)
+    errors = []
+
+    def go(x, n):
+        try:
+            for _ in range(600 // n):
+                x.run(n)
+            if isinstance(x, E.Engine):
+                x.check()
+        except BaseException as err:  # reported below
+            errors.append(err)
+
+    threads = [threading.Thread(target=go, args=(x, n)) for x, n in zip([*engines, b], (1, 20, 300, 5))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for e in engines:
+        assert_fields_equal(e, want, "threads")
+        for op, which in series:
+            assert np.array_equal(e.samples(op, which), want.samples(op, which))
+    for q, e in enumerate(alone):
+        assert b.timestep(q) == 600 and b.samples(q, 2).size == 200
+        assert np.array_equal(b.field(q, 0, 2).view(np.uint32), e.field(0, 2).view(np.uint32))
