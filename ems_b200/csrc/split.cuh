@@ -608,7 +608,14 @@ __device__ __forceinline__ void poles_edge_core(const Fields& f, const Coeffs& c
     float* fld = electric ? f.u[ax] : f.i[ax];
     float u32 = fld[idx];
     const double cb = (double)(electric ? c.c[3 + ax][idx] : c.c[9 + ax][idx]);
+    // The states of the first two poles, loaded together: after the first
+    // pole's stores the compiler could no longer load the second's.
     const double j0 = p.j[p0], q0 = p.q[p0];
+    double j1 = 0.0, q1 = 0.0;
+    if (R.np > 1u) {
+        j1 = p.j[p0 + 1];
+        q1 = p.q[p0 + 1];
+    }
     const double half_prev = __dmul_rn(0.5, prev);
     const double* cs = sets + R.set;
     if (R.oe & kOeDebye) {
@@ -620,7 +627,7 @@ __device__ __forceinline__ void poles_edge_core(const Fields& f, const Coeffs& c
     double s = 0.0;
     for (uint32_t q = 0; q < R.np; ++q) {
         const double a = cs[3 * q], ic = cs[3 * q + 1], iz = cs[3 * q + 2];
-        const double jq = q ? p.j[p0 + q] : j0, qq = q ? p.q[p0 + q] : q0;
+        const double jq = q == 0u ? j0 : (q == 1u ? j1 : p.j[p0 + q]), qq = q == 0u ? q0 : (q == 1u ? q1 : p.q[p0 + q]);
         if ((R.oe >> q) & 1u) {
             u32 = oe_pole_step(a, ic, iz, p.j[p0 + q], p.q[p0 + q], prev32, u32);
         } else if ((R.kinds >> q) & 1u) {
@@ -643,7 +650,7 @@ __device__ __forceinline__ void poles_edge_core(const Fields& f, const Coeffs& c
         for (uint32_t q = 0; q < R.np; ++q) {
             if ((R.kinds >> q) & 1u) continue;
             const double a = cs[3 * q], ic = cs[3 * q + 1], iz = cs[3 * q + 2];
-            const double jq = p.j[p0 + q], qq = p.q[p0 + q];
+            const double jq = q == 0u ? j0 : (q == 1u ? j1 : p.j[p0 + q]), qq = q == 0u ? q0 : (q == 1u ? q1 : p.q[p0 + q]);
             const double kk = __dadd_rn(__dsub_rn(__dmul_rn(a, jq), __dmul_rn(qq, ic)), half_prev);
             const double jb = __dmul_rn(__dadd_rn(kk, half_new), iz);
             p.j[p0 + q] = __dsub_rn(__dmul_rn(2.0, jb), jq);
