@@ -10,6 +10,18 @@
 
 namespace emsk {
 
+// The start of a kernel that may be launched while the one before it in the
+// stream is still running its last blocks (programmatic dependent launch):
+// waits until that one has ended and its writes are visible, then lets the next
+// one be launched in the same way. Nothing is read or written before it.
+// Without the launch attribute both are no-ops.
+__device__ __forceinline__ void after_previous() {
+#ifndef EMS_HOST_EMULATION
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
 // Rounds subnormal results to zero (src/engine/kernel.rs:30-33).
 __device__ __forceinline__ float flush(float x) { return fabsf(x) < FLT_MIN ? 0.0f : x; }
 

@@ -468,6 +468,25 @@ void sum_shares(ems_gpu* h, const double* partials, size_t n, double* out) {
     k_reduce_partials<<<1, 1024, 0, h->stream>>>(partials, n, out);
 }
 
+// Launches a kernel that begins with after_previous(): its blocks may take
+// their places while the kernel before it in the stream ends, which saves the
+// 1 to 2 us between two kernels of a step (157x203x119 box with poles 173 ->
+// 160 us per step, openEMS PML box 74 -> 63, voxel model 156 -> 143, 512^3
+// 2850 -> 2836).
+template <class... K, class... A>
+void launch_next(cudaStream_t s, void (*k)(K...), dim3 grid, unsigned threads, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, static_cast<K>(args)...);
+}
+
 // Fused kernel instances: rows per tile × the thread bound of the launch.
 template <int TJ, int MAXT>
 void launch_fused(const FusedParams& P, unsigned grid, unsigned threads, size_t smem, cudaStream_t s) {
@@ -1747,8 +1766,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
             if (oe) k_split_h<true, true><<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
             else k_split_h<true><<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
         } else {
-            if (oe) k_split_h<false, true><<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
-            else k_split_h<false><<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
+            launch_next(s, oe ? k_split_h<false, true> : k_split_h<false>, qgrd, kSplitThreads, P, 0u);
         }
     } else if (energy) {
         if (oe) k_update_h<true, true><<<grd, blk, 0, s>>>(g, f, c, h->partials);
@@ -1771,7 +1789,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
     for (auto& op : h->ops) {
         if (op.kind == EMS_OP_CPML && split) {
             if (const uint32_t nb = rows ? 0u : shell_blocks(h->shell[0])) {
-                k_shell<0><<<nb, 32 * kShellWarps, 0, s>>>(P, h->shell[0]);
+                launch_next(s, k_shell<0>, nb, 32 * kShellWarps, P, h->shell[0]);
                 ++h->launches;
             }
         } else if (op.kind == EMS_OP_CPML) {
@@ -1783,9 +1801,9 @@ ems_status run_step(ems_gpu* h, bool energy) {
             }
         } else if (op.kind == EMS_OP_POLES) {
             if (op.poles.h.n_edges && split) {
-                k_poles_blocks<<<blocks_for(op.poles.h.n_edges, kPoleBlock), kPoleBlock, 0, s>>>(
-                    f, c, op.poles.h, P.runs_h, P.sets_h, h->run_of[1], 0, h->dt, h->fold_prev[1] ? 1 : 0, 0u,
-                    (uint32_t)op.poles.h.n_edges);
+                launch_next(s, k_poles_blocks<>, blocks_for(op.poles.h.n_edges, kPoleBlock), kPoleBlock, f, c, op.poles.h,
+                            P.runs_h, P.sets_h, h->run_of[1], 0, h->dt, h->fold_prev[1] ? 1 : 0, 0u,
+                            (uint32_t)op.poles.h.n_edges, Fields{});
                 ++h->launches;
             } else if (op.poles.h.n_edges) {
                 k_poles_correct<<<blocks_for(op.poles.h.n_edges, 256), 256, 0, s>>>(g, f, c, op.poles.h, false, h->dt);
@@ -1800,7 +1818,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
             UpmlSideDev fresh = op.upml[0];
             if (h->upml_fold[0] && h->upml_e_valid) fresh.n = 0;
             if (const uint32_t n = fresh.n + op.upml[1].n) {
-                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.u[0], f.u[1], f.u[2], fresh, f.i[0], f.i[1], f.i[2],
+                launch_next(s, k_upml_hook, blocks_for(n, 256), 256, f.u[0], f.u[1], f.u[2], fresh, f.i[0], f.i[1], f.i[2],
                                                               op.upml[1]);
                 ++h->launches;
             }
@@ -1815,8 +1833,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
         launch_split_rows<1>(h, P, oe, s);
         --h->launches;
     } else if (split) {
-        if (oe) k_split_e<true><<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
-        else k_split_e<<<qgrd, kSplitThreads, 0, s>>>(P, 0u);
+        launch_next(s, oe ? k_split_e<true> : k_split_e<>, qgrd, kSplitThreads, P, 0u);
     } else {
         if (oe) k_update_e<true><<<grd, blk, 0, s>>>(g, f, c);
         else k_update_e<<<grd, blk, 0, s>>>(g, f, c);
@@ -1826,7 +1843,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
     for (auto& op : h->ops) {
         if (op.kind == EMS_OP_CPML && split) {
             if (const uint32_t nb = rows ? 0u : shell_blocks(h->shell[1])) {
-                k_shell<1><<<nb, 32 * kShellWarps, 0, s>>>(P, h->shell[1]);
+                launch_next(s, k_shell<1>, nb, 32 * kShellWarps, P, h->shell[1]);
                 ++h->launches;
             }
         } else if (op.kind == EMS_OP_CPML) {
@@ -1838,9 +1855,9 @@ ems_status run_step(ems_gpu* h, bool energy) {
             }
         } else if (op.kind == EMS_OP_POLES) {
             if (op.poles.e.n_edges && split) {
-                k_poles_blocks<<<blocks_for(op.poles.e.n_edges, kPoleBlock), kPoleBlock, 0, s>>>(
-                    f, c, op.poles.e, P.runs, P.sets, h->run_of[0], 1, h->dt, h->fold_prev[0] ? 1 : 0, 0u,
-                    (uint32_t)op.poles.e.n_edges);
+                launch_next(s, k_poles_blocks<>, blocks_for(op.poles.e.n_edges, kPoleBlock), kPoleBlock, f, c, op.poles.e,
+                            P.runs, P.sets, h->run_of[0], 1, h->dt, h->fold_prev[0] ? 1 : 0, 0u,
+                            (uint32_t)op.poles.e.n_edges, Fields{});
                 ++h->launches;
             } else if (op.poles.e.n_edges) {
                 k_poles_correct<<<blocks_for(op.poles.e.n_edges, 256), 256, 0, s>>>(g, f, c, op.poles.e, true, h->dt);
@@ -1855,7 +1872,7 @@ ems_status run_step(ems_gpu* h, bool energy) {
             UpmlSideDev fresh = op.upml[1];
             if (h->upml_fold[1]) fresh.n = 0;
             if (const uint32_t n = fresh.n + op.upml[0].n) {
-                k_upml_hook<<<blocks_for(n, 256), 256, 0, s>>>(f.i[0], f.i[1], f.i[2], fresh, f.u[0], f.u[1], f.u[2],
+                launch_next(s, k_upml_hook, blocks_for(n, 256), 256, f.i[0], f.i[1], f.i[2], fresh, f.u[0], f.u[1], f.u[2],
                                                               op.upml[0]);
                 ++h->launches;
             }
@@ -1980,7 +1997,7 @@ ems_status setup_sheet(ems_gpu* h, const ems_sheet* t, ems_gpu::Op& op) {
 // sides bit 0 the magnetic ones, bit 1 the electric ones.
 void run_hooks(ems_gpu* h, const Fields& f, int& lo, int hi, int sides, bool& acts) {
     if (acts && hi > lo) {
-        k_hooks<<<1, 256, 0, h->stream>>>(f, h->dt, h->hooks.dev + lo, (uint32_t)(hi - lo), (uint32_t)h->step, sides);
+        launch_next(h->stream, k_hooks, 1, 256, f, h->dt, h->hooks.dev + lo, (uint32_t)(hi - lo), (uint32_t)h->step, sides);
         ++h->launches;
     }
     lo = hi;
@@ -2052,7 +2069,7 @@ ems_status serial_pre_e(ems_gpu* h, const Fields& f) {
         }
     }
     if (acts) {
-        k_hooks_pre<<<1, 256, 0, h->stream>>>(f, h->hooks.dev, (uint32_t)(h->hooks.held.size() / sizeof(ResOp)));
+        launch_next(h->stream, k_hooks_pre, 1, 256, f, h->hooks.dev, (uint32_t)(h->hooks.held.size() / sizeof(ResOp)));
         ++h->launches;
     }
     return EMS_OK;
@@ -2508,7 +2525,7 @@ static ems_status dumps_sample(ems_gpu* h, uint64_t m, bool first) {
         if (m % D.interval) continue;
         DumpDev d = D.d;
         for (int a = 0; a < 3; ++a) d.f[a] = D.field ? h->i[a] : h->u[a];
-        k_dump<<<blocks_for(d.npts, 256), 256, 0, h->stream>>>(d, (double)m);
+        launch_next(h->stream, k_dump, blocks_for(d.npts, 256), 256, d, (double)m);
         ++h->launches;
     }
     return EMS_OK;

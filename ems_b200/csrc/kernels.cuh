@@ -517,6 +517,7 @@ __device__ __forceinline__ void upml_apply(float* F, const UpmlSideDev& a, uint3
 // [r.n, r.n + a.n) complete the update of side a in the fields `dst`.
 __global__ void __launch_bounds__(256) k_upml_hook(const float* s0, const float* s1, const float* s2, UpmlSideDev r,
                                                    float* d0, float* d1, float* d2, UpmlSideDev a) {
+    after_previous();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < r.n) {
         const uint8_t ax = r.axis[e];
@@ -706,6 +707,7 @@ __global__ void __launch_bounds__(256) k_unpad(const float* src, uint32_t nz, ui
 __device__ __forceinline__ double frac_toward_zero(double x) { return x - trunc(x); }
 
 __global__ void __launch_bounds__(256) k_dump(const __grid_constant__ DumpDev d, double m) {
+    after_previous();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= d.npts) return;
     double x[3];

@@ -211,10 +211,12 @@ __device__ __forceinline__ void serial_pre(const Fields& f, const ResOp* ops, ui
 // a source and five probes.
 __global__ void __launch_bounds__(256) k_hooks(const __grid_constant__ Fields f, double dt, const ResOp* ops, uint32_t n_ops,
                                                uint32_t step, int sides) {
+    after_previous();
     if (sides & 1) serial_hooks(f, dt, ops, n_ops, false, step, true, true);
     if (sides & 2) serial_hooks(f, dt, ops, n_ops, true, step, true, true);
 }
 __global__ void __launch_bounds__(256) k_hooks_pre(const __grid_constant__ Fields f, const ResOp* ops, uint32_t n_ops) {
+    after_previous();
     serial_pre(f, ops, n_ops);
 }
 

@@ -332,6 +332,7 @@ __device__ __forceinline__ double split_h_quad(const FusedParams& P, uint32_t i,
 template <bool ENERGY, bool OE = false, bool ROWCPML = false>
 __global__ void __launch_bounds__(kSplitThreads, ENERGY ? 1 : (ROWCPML ? 4 : 7)) k_split_h(
     const __grid_constant__ FusedParams P, uint32_t i0) {
+    after_previous();
     const uint32_t i = i0 + (gridDim.y - 1u - blockIdx.y);
     const double w = split_h_quad<ENERGY, OE, ROWCPML>(P, i, mapped_quad(P, blockIdx.x * kSplitThreads + threadIdx.x));
     if (ENERGY) {
@@ -440,6 +441,7 @@ __device__ __forceinline__ void split_e_quad(const FusedParams& P, uint32_t i, u
 template <bool OE = false, bool ROWCPML = false>
 __global__ void __launch_bounds__(kSplitThreads, ROWCPML ? 4 : 7) k_split_e(const __grid_constant__ FusedParams P,
                                                                          uint32_t i0) {
+    after_previous();
     split_e_quad<OE, ROWCPML>(P, i0 + blockIdx.y, mapped_quad(P, blockIdx.x * kSplitThreads + threadIdx.x));
 }
 
@@ -580,6 +582,7 @@ __device__ __forceinline__ void shell_item(const FusedParams& P, const ShellDev&
 template <int SIDE>
 __global__ void __launch_bounds__(32 * kShellWarps) k_shell(const __grid_constant__ FusedParams P,
                                                             const __grid_constant__ ShellDev S) {
+    after_previous();
     shell_item<SIDE>(P, S, blockIdx.x, threadIdx.x);
 }
 
@@ -691,6 +694,7 @@ __global__ void __launch_bounds__(kPoleBlock) k_poles_blocks(const __grid_consta
                                                              double dt, int save_prev, uint32_t e0, uint32_t e1,
                                                              const __grid_constant__ Fields old = Fields{}) {
     EMS_SHARED PoleRun sr[kPoleBlock];
+    after_previous();
     const uint32_t eb = e0 + blockIdx.x * kPoleBlock;
     if (eb >= e1) return;
     const uint32_t el = min(eb + kPoleBlock, e1) - 1;
