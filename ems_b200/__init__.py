@@ -1083,8 +1083,8 @@ class Engine:
 
 class Batch:
     """Many built :class:`Model` s stepping together on one device
-    (``ems_batch_*``): one launch per kernel kind over all models, one CUDA
-    graph per step; a frozen model keeps its state."""
+    (``ems_batch_*``): many steps per launch, a gang of blocks per model; a
+    frozen model keeps its state."""
 
     def __init__(self, models: Sequence[Model], device: int = 0, max_steps: int = 100_000):
         self._lib = gpu_lib()

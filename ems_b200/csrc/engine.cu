@@ -1341,7 +1341,8 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
 // MB) 187/216; coefficients of every node 160 (260 MB) 129/141, 240 370/364.
 // The poles' correction runs better in its own kernel (trapezoidal media 64
 // cells 28/46, 96 (27 MB) 55/64, 128 (70 MB) 121/115), and so does the
-// openEMS PML's at nearly every size (24 34/26, 64 28/33, 96 68/59).
+// openEMS PML's at nearly every size (24 34/26, 64 28/33, 96 68/59). (The
+// split times before launch_next, which takes some 8 us off them.)
 constexpr size_t kResidentBytes = 256u << 20, kResidentPoleBytes = 32u << 20;
 constexpr size_t kResidentEdges = 4096;
 constexpr uint64_t kResidentSteps = 4096;  // most steps per launch

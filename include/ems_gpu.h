@@ -390,7 +390,8 @@ ems_status ems_gpu_profile(ems_gpu* h, int enable);
 ems_status ems_gpu_profile_read(ems_gpu* h, int kernel, double* ms, uint64_t* launches);
 
 /* Selects the step schedule: 0 = automatic (the fastest one the model
- * allows), 1 = one kernel per field update and operator, 2 = the fused
+ * allows; on small grids the split schedule's resident form, many steps per
+ * launch), 1 = one kernel per field update and operator, 2 = the fused
  * single-pass kernel, 3 = two kernels (H with its slab hooks, E with its
  * slab hooks), 4 = split (streaming H and E updates, one CPML shell kernel
  * per side, the other hooks per operator), 5 = sweep (the split kernels
@@ -447,7 +448,7 @@ ems_status ems_gpu_set_interior_planes(ems_gpu* h, uint32_t planes);
 
 /* Synchronises the handle's stream and reports what its device flags hold
  * since the last check (and clears them): EMS_ERR_TIMEOUT if a bounded wait
- * of the fused or marching kernel ran out, EMS_ERR_DIVERGED if a marching
+ * of the fused, marching or resident kernel ran out, EMS_ERR_DIVERGED if a marching
  * step wrote a non-finite field value (NaN or Inf). Field downloads, sample
  * reads and step_with_energy report the same at their end. This is the
  * check at which device errors surface: stepping itself never fails, as in
@@ -569,10 +570,11 @@ ems_status ems_gpu_freq_dump_read(ems_gpu* h, size_t id, size_t k, double* out, 
  * No counterpart in the reference, where a parameter sweep runs
  * Simulation::run (src/sim/mod.rs:1044) once per model. A batch builds
  * every model as ems_gpu_create does and steps them together on one device:
- * each kernel kind of the split schedule runs once per step over all models
- * (a packed per-model block table walked by a persistent grid), the serial
- * hooks run batched from device-side step counters, and a whole step is one
- * CUDA graph. Each model's fields, probe and port series equal those of the
+ * many steps per launch, a gang of blocks per model sized by its cells, or,
+ * for energy steps and models with more edges in a source than one block can
+ * drive, one CUDA graph per step (each kernel kind of the split schedule once
+ * over all models, a packed per-model block table walked by a persistent
+ * grid). The serial hooks run from device-side step counters. Each model's fields, probe and port series equal those of the
  * same model run alone bit for bit. A model needs the split schedule's
  * tables, its post_e hooks in the order lumped elements, E sources, voltage
  * probes and its post_h hooks in the order H sources, current probes, and
