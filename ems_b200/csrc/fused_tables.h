@@ -417,6 +417,8 @@ inline void cpml_quads(const std::vector<SlabGeo>& slabs, const uint64_t nodes[3
     }
     layer.clear();
     inner.clear();
+    layer.reserve((size_t)nx * ny * nq);
+    inner.reserve((size_t)nx * ny * nq);
     uint32_t q = 0;
     for (uint32_t i = 0; i < nx; ++i)
         for (uint32_t j = 0; j < ny; ++j)
