@@ -2494,7 +2494,8 @@ static ems_status tune_step(ems_gpu* h) {
             size_t best = 0;
             for (size_t q = 1; q < T.cand.size(); ++q)
                 if (T.ms[q] < T.ms[best]) best = q;
-            h->schedule = T.cand[best];
+            // The split schedule: its resident form too, where the automatic choice takes it.
+            h->schedule = T.cand[best] == 4 ? 0 : T.cand[best];
             tune_record(T.cache, T.key, T.cand[best], T.ms[best] / (kTuneSteps - 1));
             T.active = false;
             cudaEventDestroy(T.e0);
@@ -2744,7 +2745,7 @@ ems_status ems_gpu_autotune(ems_gpu* h, const char* cache_path) {
     if (tune_lookup(T.cache, T.key, &v) &&
         (v == 1 || ((v == 4 || (v == 3 && !h->oe_curl && !h->has_upml)) && h->tables_ok) ||
          (v == 5 && h->tables_ok && h->sweep_ok))) {
-        h->schedule = v;
+        h->schedule = v == 4 ? 0 : v;
         return EMS_OK;
     }
     // In-place schedules only (the per-operator, two-kernel and split ones
