@@ -1,7 +1,8 @@
 // learn.cu — kernels of the learned early stop (include/ems_learn.h), sm_100a.
 //
-// A small 1-D CNN (convolutions as im2col + GEMM, then two dense layers)
-// trained and run on these kernels. The GEMM runs on the tcgen05 tensor
+// A small 1-D CNN (convolutions as GEMMs over rows read in place from the
+// channels-last input, then two dense layers) trained and run on these
+// kernels. The GEMM runs on the tcgen05 tensor
 // cores (bf16 operands from shared memory, f32 accumulator in tensor
 // memory). The matrices here are small (≤ 10^5 rows, ≤ 2·10^3 columns), so
 // the kernel takes A and B with arbitrary element strides (a transposed
@@ -10,6 +11,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
 #include <cstdint>
 
 #include "../../include/ems_learn.h"
@@ -17,34 +20,43 @@
 namespace {
 
 // The GEMM C = alpha·A·B + beta·C on the fifth-generation tensor cores: one
-// CTA of eight warps per 128×TN tile of C (TN the columns rounded up to 16, at
-// most 128) and per share of K, the f32 accumulator in tensor memory. K runs
-// in chunks of 64 through two stages of shared memory; warps 0-3 stage A,
-// warps 4-7 B, each chunk's loads held in registers while the chunk before
-// it multiplies. The operands lie in the no-swizzle K-major core-matrix
-// layout (8 rows × 8 bf16, 16 bytes per row, per core matrix); the core
-// matrices of neighbouring row groups are 144 bytes apart rather than 128, so
-// that the transposing stores below meet no bank conflict. One elected thread
-// issues the tcgen05.mma (M 128, N TN, K 16, bf16 in, f32 out) of a chunk and
-// commits them to the stage's mbarrier (bounded waits).
+// CTA per 128×TN tile of C (TN the columns rounded up to 16, at most 128), the
+// f32 accumulator in tensor memory, K in chunks of 64 through a ring of stages
+// in shared memory. Warps 0-3 feed A and warps 4-7 B by 16-byte asynchronous
+// copies, several chunks ahead of the one thread of warp 8 that issues the
+// tcgen05.mma (M 128, N TN, K 16, bf16 in, f32 out) of a chunk and commits them
+// to the stage's mbarrier (bounded waits).
 //
-// The matrices are small and most are bound by the latency of one CTA's chunk
-// loop, so K is split over the grid's z dimension until the chip is filled
-// (gemm_plan): every share writes its tile to the workspace and k_gemm_sum
-// adds the shares in order. The weight gradients gain most: 32×16 over 32704
-// rows took 1349 us in the single CTA of a scalar-staged kernel.
+// Every element of C is ONE chain of products over K in order, whatever the
+// other sizes: a batch's rows come out bit for bit as each would alone, and K
+// is not shared out over the chip. Shares added in f32 gave other bits, with an
+// error against f64 up to 3 % larger. The chain of one CTA bounds the small
+// matrices: 0.18 us per chunk for the products, and about as much again for
+// copies and hand-over that they do not hide (32x16 over 32704 rows: 158 us,
+// 64x256 over 8064: 54 us, 32x64 over 3840: 25 us; with two stages filled
+// through registers 1100, 300 and 160 us). The weight gradients therefore share
+// a launch (Jobs).
 //
-// An operand is read in 16-byte vectors along whichever index is contiguous
-// (mode 1: k; mode 2: the row or column, transposed 8×8 in registers), or
-// element by element for strides that allow neither (mode 0). An index may be
-// two-level, r -> (r / per)·big + (r mod per)·stride: the rows of a valid 1-D
-// convolution are overlapping spans of the channels-last input, so the
-// convolutions read it in place, without columns being formed.
-constexpr int TM = 128, TK = 64;
-constexpr uint32_t kGroup = 144;                           // bytes between row groups of 8
-constexpr uint32_t kStageOp = (TM / 8) * kGroup * (TK / 8);  // one operand's stage
-constexpr uint32_t kGemmSmem = 4 * kStageOp + 64;          // three CTAs per SM, 384 of 512 tensor-memory columns
-constexpr uint32_t kSumBytes = 512 * 1024;                 // shares of one tile that k_gemm_sum reads, at most
+// An operand is copied in vectors along whichever index is contiguous (mode 1:
+// k; mode 2: the row or column), into 8×8 core matrices without swizzle that
+// are K-major or MN-major accordingly, or element by element for strides that
+// allow neither (mode 0). Core matrices of neighbouring row groups lie 144
+// bytes apart and those of neighbouring k groups an odd multiple of 16 modulo
+// 128, so that neither mapping of copies to threads meets a bank conflict. An
+// index may be two-level, r -> (r / per)·big + (r mod per)·stride: the rows of
+// a valid 1-D convolution are overlapping spans of the channels-last input, so
+// the convolutions read it in place, without columns being formed.
+constexpr int TM = 128, TK = 64, kFeeders = 256, kGemmThreads = kFeeders + 32;
+constexpr uint32_t kGroup = 144;  // bytes between row groups of 8
+constexpr int kMaxStages = 8;
+constexpr uint32_t kStageBytes = 192 * 1024;         // most shared memory of the ring
+constexpr uint32_t kBarBytes = (2 * kMaxStages + 2) * 8;
+// A tile of 128 columns takes at least a quarter of an SM's shared memory: four
+// of them hold all of its 512 tensor-memory columns.
+constexpr uint32_t kWideBytes = 48 * 1024;
+// Bytes between k groups of 8, and of a chunk, of an operand of `rows` rows.
+__host__ __device__ constexpr uint32_t k_step(int rows) { return (uint32_t)(rows >> 3) * kGroup + 16u; }
+__host__ __device__ constexpr uint32_t chunk_bytes(int rows) { return (TK / 8) * k_step(rows); }
 constexpr uint64_t kGemmWaitNs = 1000000000ull;
 
 __device__ int g_learn_fail = 0;
@@ -57,10 +69,11 @@ __device__ __forceinline__ uint64_t now_ns() {
     return t;
 }
 
-// Waits for phase `parity`; false after kGemmWaitNs.
+// Waits for phase `parity`; false after kGemmWaitNs. The clock is read only
+// once a wait drags on.
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
     uint32_t done = 0;
-    const uint64_t t0 = now_ns();
+    uint64_t t0 = 0;
     for (uint32_t it = 0;; ++it) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -70,7 +83,10 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
             : "r"(smem_addr(bar)), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((it & 63u) == 63u && now_ns() - t0 > kGemmWaitNs) return false;
+        if ((it & 63u) != 63u) continue;
+        const uint64_t now = now_ns();
+        if (!t0) t0 = now;
+        if (now - t0 > kGemmWaitNs) return false;
     }
 }
 
@@ -82,9 +98,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 }
 
 // Instruction descriptor of kind::f16: f32 accumulator (bits 4-5 = 1), A
-// and B bf16 (bits 7-9, 10-12 = 1), both K-major, N/8 at bit 17, M/16 at 24.
-__device__ __forceinline__ uint32_t inst_desc(uint32_t tn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((tn >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+// and B bf16 (bits 7-9, 10-12 = 1), MN-major operands at bits 15 (A) and 16
+// (B), N/8 at bit 17, M/16 at 24.
+__device__ __forceinline__ uint32_t inst_desc(uint32_t tn, bool mn_a, bool mn_b) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_a ? 1u << 15 : 0u) | (mn_b ? 1u << 16 : 0u) | ((tn >> 3) << 17) |
+           ((uint32_t)(TM >> 4) << 24);
 }
 
 // One operand: rows (M or N) by k.
@@ -112,123 +130,244 @@ struct Epilogue {
     int act;
     float* outf;
     uint16_t* outb;
+    bool wide;  // rows of every array begin on 16 bytes
 };
 __device__ __forceinline__ float sigmoid(float y) { return 1.0f / (1.0f + expf(-y)); }
 __device__ __forceinline__ uint16_t bf16_of(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ void finish(const Epilogue& e, int i, int j, float x) {
-    const int64_t at = (int64_t)i * e.ldc + j;
+__device__ __forceinline__ float finish_y(const Epilogue& e, float x, int j) { return e.alpha * x + e.bias[j]; }
+// The elements j0 .. j0 + 15 of row i from the accumulator's values v; `wide`:
+// all of them exist and every array takes 16-byte stores. A lane holds a row, so
+// its stores go out in pieces of 16 bytes rather than 4.
+__device__ __forceinline__ void finish(const Epilogue& e, int i, int j0, int N, bool wide, const uint32_t (&v)[16]) {
+    const int64_t at = (int64_t)i * e.ldc + j0;
     if (!e.bias) {
-        e.C[at] = e.beta != 0.0f ? e.alpha * x + e.beta * e.C[at] : e.alpha * x;
+        if (wide && e.beta == 0.0f) {
+#pragma unroll
+            for (int q = 0; q < 16; q += 4)
+                *reinterpret_cast<float4*>(e.C + at + q) =
+                    make_float4(e.alpha * __uint_as_float(v[q]), e.alpha * __uint_as_float(v[q + 1]),
+                                e.alpha * __uint_as_float(v[q + 2]), e.alpha * __uint_as_float(v[q + 3]));
+            return;
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            if (j0 + q >= N) continue;
+            const float x = __uint_as_float(v[q]);
+            e.C[at + q] = e.beta != 0.0f ? e.alpha * x + e.beta * e.C[at + q] : e.alpha * x;
+        }
         return;
     }
-    const float y = e.alpha * x + e.bias[j];
-    if (e.C) e.C[at] = y;
-    const float a = e.act ? y * sigmoid(y) : y;
-    if (e.outf) e.outf[at] = a;
-    if (e.outb) e.outb[at] = bf16_of(a);
-}
-
-// A thread's part of one chunk of an operand tile of RT rows (rows r0.. of
-// MN, k0.. below K), and its place in the stage. Modes 0 and 1: vector q of
-// the thread holds 8 k of one row; eight lanes take eight rows of the same k
-// (one 128-byte core matrix: no conflict), four groups of lanes 64 contiguous
-// bytes. Mode 2: vector q holds 8 rows of k = 8·k8 + q.
-struct Part {
-    uint4 v[8];
-};
-__device__ __forceinline__ uint4 pack8(const uint16_t (&h)[8]) {
-    return make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16,
-                      h[6] | (uint32_t)h[7] << 16);
-}
-__device__ __forceinline__ void part_load(const Operand& o, int r0, int MN, int k0, int K, int RT, int t, Part& P) {
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    if (o.mode == 2) {
-        const int mg = RT >> 3, m = r0 + (t % mg) * 8, k8 = t / mg;
-        const bool mine = t < RT, whole = m + 8 <= MN;
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) {
+        float y[8], a[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int k = k0 + k8 * 8 + q;
-            P.v[q] = zero;
-            if (!mine || k >= K || m >= MN) continue;
-            const uint16_t* p = o.p + op_k(o, k) + m;
-            if (whole) {
-                P.v[q] = __ldg(reinterpret_cast<const uint4*>(p));
-            } else {
-                uint16_t h[8];
+            const int j = j0 + h + q;
+            y[q] = j < N ? finish_y(e, __uint_as_float(v[h + q]), j) : 0.0f;
+            a[q] = e.act ? y[q] * sigmoid(y[q]) : y[q];
+        }
+        if (wide) {
+            float4* c = reinterpret_cast<float4*>(e.C + at + h);
+            float4* f = reinterpret_cast<float4*>(e.outf + at + h);
+            if (e.C) c[0] = make_float4(y[0], y[1], y[2], y[3]), c[1] = make_float4(y[4], y[5], y[6], y[7]);
+            if (e.outf) f[0] = make_float4(a[0], a[1], a[2], a[3]), f[1] = make_float4(a[4], a[5], a[6], a[7]);
+            if (e.outb) {
+                uint32_t b[4];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) h[e] = m + e < MN ? p[e] : (uint16_t)0;
-                P.v[q] = pack8(h);
+                for (int q = 0; q < 4; ++q) b[q] = bf16_of(a[2 * q]) | (uint32_t)bf16_of(a[2 * q + 1]) << 16;
+                *reinterpret_cast<uint4*>(e.outb + at + h) = make_uint4(b[0], b[1], b[2], b[3]);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (j0 + h + q >= N) continue;
+            if (e.C) e.C[at + h + q] = y[q];
+            if (e.outf) e.outf[at + h + q] = a[q];
+            if (e.outb) e.outb[at + h + q] = bf16_of(a[q]);
+        }
+    }
+}
+
+// 16 bytes global to shared, the first `bytes` of them read, zeros behind.
+// Through L1 (.ca): the copies that pass it by (.cg) took 2.3 times as long.
+__device__ __forceinline__ void copy16(uint32_t dst, const uint16_t* src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// A thread's copies of an operand tile of RT rows (rows r0.. of MN): up to 8
+// vectors of a chunk. Modes 0 and 1: vector q is 8 k (`k` on) of row
+// t / 8 + 16·q, so eight lanes read 128 contiguous bytes. Mode 2: vector q is 8
+// rows of k = `k` + q·dk, the valid row groups (rounded up to a power of two)
+// side by side. Rows beyond MN are left as they are: they reach only rows or
+// columns of the product that are not stored. The vectors' sources are kept and
+// moved on by a chunk: computed anew for each chunk they took 500 clocks, more
+// than the copies and the products.
+struct Feed {
+    const uint16_t* src[8];  // of the coming chunk (mode 0: of k 0)
+    int inner[8];            // two-level k index: k mod per_k of the vector
+    int64_t next, wrap;      // elements to the next chunk; from the end of an inner run to the next one
+    uint32_t dst, step, bytes;
+    int k, dk, n;  // n: vectors of this thread
+};
+__device__ __forceinline__ void feed_init(const Operand& o, int r0, int MN, int RT, int t, Feed& f) {
+    const int valid = min(RT, MN - r0);
+    f.wrap = 0;
+    if (o.mode == 2) {
+        const int groups = (valid + 7) >> 3, lg = 32 - __clz(groups - 1), g = t & ((1 << lg) - 1);  // clz(0) = 32
+        f.k = t >> lg;
+        f.dk = 128 >> lg;
+        f.n = g < groups && f.k < TK ? max(1, (1 << lg) >> 1) : 0;
+        f.bytes = (uint32_t)min(16, 2 * (valid - 8 * g));
+        f.dst = (uint32_t)(f.k >> 3) * k_step(RT) + (uint32_t)g * kGroup + (uint32_t)(f.k & 7) * 16u;
+        f.step = (uint32_t)(f.dk >> 3) * k_step(RT);
+        f.next = TK * o.sk;
+        if (o.per_k) f.wrap = o.big - o.per_k * o.sk;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = f.k + q * f.dk;
+            f.src[q] = o.p + (q < f.n ? r0 + 8 * g + op_k(o, k) : 0);
+            f.inner[q] = o.per_k ? k % o.per_k : 0;
+        }
+        return;
+    }
+    const int r = t >> 3;
+    f.k = (t & 7) * 8;
+    f.dk = 0;
+    f.bytes = 16u;
+    f.n = r < valid ? min(RT >> 4, (valid - r + 15) >> 4) : 0;
+    f.dst = (uint32_t)(t & 7) * k_step(RT) + (uint32_t)(r >> 3) * kGroup + (uint32_t)(r & 7) * 16u;
+    f.step = 2u * kGroup;
+    f.next = o.mode ? TK : 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        f.src[q] = o.p + (q < f.n ? op_row(o, r0 + r + 16 * q) + (o.mode ? f.k : 0) : 0);
+        f.inner[q] = 0;
+    }
+}
+// The copies of the chunk at k0 into the stage at `smem`, and on to the next
+// chunk; k up to the next multiple of 16 beyond K are zeros.
+__device__ __forceinline__ void feed(const Operand& o, Feed& f, uint32_t smem, int k0, int K) {
+    const int left = K - k0;  // k that exist from k0 on
+    if (o.mode && left >= TK) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (q >= f.n) break;
+            copy16(smem + f.dst + q * f.step, f.src[q], f.bytes);
+        }
+        // After all copies are issued: a copy holds its address registers until
+        // it leaves the queue.
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            f.src[q] += f.next;
+            if (o.per_k) {
+                f.inner[q] += TK;
+                while (f.inner[q] >= o.per_k) {
+                    f.inner[q] -= o.per_k;
+                    f.src[q] += f.wrap;
+                }
             }
         }
         return;
     }
-    const int lane = t & 31, w = t >> 5;
+    const int end = (min(TK, left) + 15) & ~15;  // k of the chunk multiplied
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const int tile = w + 4 * q;
-        P.v[q] = zero;
-        if (tile >= (RT >> 2)) continue;
-        const int m = r0 + (tile >> 1) * 8 + (lane & 7), k = k0 + ((tile & 1) * 4 + (lane >> 3)) * 8;
-        if (m >= MN || k >= K) continue;
-        if (o.mode == 1 && k + 8 <= K) {
-            P.v[q] = __ldg(reinterpret_cast<const uint4*>(o.p + op_row(o, m) + k));
+        const int k = f.k + q * f.dk;
+        if (q >= f.n || k >= end) break;
+        const uint32_t dst = smem + f.dst + q * f.step;
+        if (o.mode) {
+            // Mode 1: what is left of the vector's 8 k; mode 2: its one k or none.
+            const uint32_t bytes = o.mode == 2 ? f.bytes : (uint32_t)min(16, 2 * (left - k));
+            copy16(dst, k < left ? f.src[q] : o.p, k < left ? bytes : 0u);
         } else {
-            uint16_t h[8];
+            uint32_t h[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int e = 0; e < 8; ++e) h[e] = k + e < K ? o.p[op_row(o, m) + op_k(o, k + e)] : (uint16_t)0;
-            P.v[q] = pack8(h);
+            for (int e = 0; e < 8; ++e)
+                if (k + e < left) h[e >> 1] |= (uint32_t)f.src[q][op_k(o, k0 + k + e)] << (16 * (e & 1));
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
+                         : "memory");
         }
-    }
-}
-__device__ __forceinline__ uint32_t word(const uint4& v, int q) { return q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w)); }
-__device__ __forceinline__ void part_store(const Operand& o, unsigned char* stage, int RT, int t, const Part& P) {
-    const uint32_t kstep = (uint32_t)(RT >> 3) * kGroup;
-    if (o.mode == 2) {
-        if (t >= RT) return;
-        const int mg = RT >> 3;
-        unsigned char* dst = stage + (t / mg) * kstep + (t % mg) * kGroup;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {  // row e: its 8 k
-            const uint32_t sel = e & 1 ? 0x7632u : 0x5410u;
-            uint4 r;
-            r.x = __byte_perm(word(P.v[0], e >> 1), word(P.v[1], e >> 1), sel);
-            r.y = __byte_perm(word(P.v[2], e >> 1), word(P.v[3], e >> 1), sel);
-            r.z = __byte_perm(word(P.v[4], e >> 1), word(P.v[5], e >> 1), sel);
-            r.w = __byte_perm(word(P.v[6], e >> 1), word(P.v[7], e >> 1), sel);
-            *reinterpret_cast<uint4*>(dst + e * 16) = r;
-        }
-        return;
-    }
-    const int lane = t & 31, w = t >> 5;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int tile = w + 4 * q;
-        if (tile >= (RT >> 2)) continue;
-        *reinterpret_cast<uint4*>(stage + ((tile & 1) * 4 + (lane >> 3)) * kstep + (tile >> 1) * kGroup +
-                                  (lane & 7) * 16) = P.v[q];
     }
 }
 
-// Grid: (column tiles, row tiles, shares of K). ws: null (one share), or the
-// shares' tiles, [tile][share][row][TN].
-__global__ void __launch_bounds__(256, 3) k_gemm_tc(const __grid_constant__ Operand A, const __grid_constant__ Operand B,
-                                                    const __grid_constant__ Epilogue E, int M, int N, int K, int tn,
-                                                    int per, float* ws) {
+// The copies of one operand by its four warps, stage by stage of `deep` chunks:
+// `smem` the operand's part of the first chunk of stage 0, `size` the bytes of
+// a chunk. False once a wait has run out.
+__device__ __forceinline__ bool feeders(const Operand o, int r0, int MN, int RT, int t, uint32_t smem, uint32_t size,
+                                        int K, int stages, int deep, uint64_t* full, uint64_t* empty) {
+    Feed f;
+    feed_init(o, r0, MN, RT, t, f);
+    const int chunks = (K - 1) / TK + 1;
+    int sg = 0;
+    uint32_t round = 0;
+    bool ok = true;
+    for (int ch = 0; ch < chunks;) {
+        if (round && !bar_wait(empty + sg, (round - 1u) & 1u)) {
+            ok = false;
+            break;
+        }
+        for (int d = 0; d < deep && ch < chunks; ++d, ++ch) feed(o, f, smem + (uint32_t)(sg * deep + d) * size, ch * TK, K);
+        // Arrives once the thread's copies so far are done.
+        if (o.mode) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(full + sg)) : "memory");
+        else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(full + sg)) : "memory");
+        if (++sg == stages) {
+            sg = 0;
+            ++round;
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return ok;
+}
+
+// One product of a launch: its tiles are the blocks from `first` on, row by row.
+struct Job {
+    Operand A, B;
+    Epilogue E;
+    int M, N, K, ra, tn, stages, deep, tiles_n;
+};
+constexpr int kJobs = 6;
+struct Jobs {
+    Job job[kJobs];
+    int first[kJobs];  // beyond the last job: INT_MAX
+};
+
+// Grid: the tiles of up to kJobs products that do not depend on one another
+// (the weight gradients: the chain of the longest, one block, hides the
+// others). Dynamic shared memory: `stages` stages of `deep` chunks of A (ra
+// rows) and B (tn rows), then the barriers. The products read 128 rows of A:
+// those beyond ra alias what lies behind them.
+__global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_tc(const __grid_constant__ Jobs P) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 4 * kStageOp);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 4 * kStageOp + 16);
+    __shared__ __align__(16) unsigned char raw[sizeof(Job)];
+    int q = 0;
+    while (q + 1 < kJobs && P.first[q + 1] <= (int)blockIdx.x) ++q;
+    for (unsigned w = threadIdx.x; w < sizeof(Job) / 4; w += kGemmThreads)
+        reinterpret_cast<uint32_t*>(raw)[w] = reinterpret_cast<const uint32_t*>(&P.job[q])[w];
+    __syncthreads();
+    const Job& J = *reinterpret_cast<const Job*>(raw);
+    const Epilogue& E = J.E;
+    const int M = J.M, N = J.N, K = J.K, ra = J.ra, tn = J.tn, stages = J.stages, deep = J.deep;
+    const int tile = (int)blockIdx.x - P.first[q], ty = tile / J.tiles_n;
+    const uint32_t size_a = chunk_bytes(ra), size = size_a + chunk_bytes(tn);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + stages * deep * size);
+    uint64_t* empty = full + kMaxStages;
+    uint64_t* all = empty + kMaxStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(all + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = tid >> 7, t = tid & 127;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * tn;
+    const int m0 = ty * TM, n0 = (tile - ty * J.tiles_n) * tn;
     const uint32_t cols = tn <= 32 ? 32u : (tn <= 64 ? 64u : 128u);
-    if (warp == 0) {
+    if (warp == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
                      "r"(cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar + 1)) : "memory");
+        for (int s = 0; s < stages; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(full + s)), "r"(kFeeders) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(empty + s)) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(all)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -236,59 +375,68 @@ __global__ void __launch_bounds__(256, 3) k_gemm_tc(const __grid_constant__ Oper
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
-    const int chunks = (K + TK - 1) / TK, c0 = blockIdx.z * per, c1 = min(chunks, c0 + per);
-    const Operand& O = half ? B : A;
-    const int r0 = half ? n0 : m0, MN = half ? N : M, RT = half ? tn : TM;
-    const uint32_t lboA = (uint32_t)(TM >> 3) * kGroup, lboB = (uint32_t)(tn >> 3) * kGroup;
-    Part P;
-    part_load(O, r0, MN, c0 * TK, K, RT, t, P);
-    part_store(O, smem + half * kStageOp, RT, t, P);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    for (int ch = c0; ch < c1; ++ch) {
-        const int at = ch - c0, sg = at & 1;
-        if (ch + 1 < c1) part_load(O, r0, MN, (ch + 1) * TK, K, RT, t, P);
-        if (tid == 0) {
+    const int chunks = (K - 1) / TK + 1;
+    // The job comes through shared memory and its operands by value, one branch
+    // each: a copy of the one or the other kernel parameter chosen per warp has
+    // come out as the wrong one (nvcc 12.9), and a reference to the chosen one is
+    // read again after every copy.
+    if (half == 0) {
+        ok = feeders(J.A, m0, M, ra, t, smem_addr(smem), size, K, stages, deep, full, empty);
+    } else if (half == 1) {
+        ok = feeders(J.B, n0, N, tn, t, smem_addr(smem) + size_a, size, K, stages, deep, full, empty);
+    } else if (lane == 0) {
+        const uint32_t id = inst_desc((uint32_t)tn, J.A.mode == 2, J.B.mode == 2);
+        const uint32_t step_a = k_step(ra), step_b = k_step(tn);
+        int sg = 0;
+        uint32_t round = 0;
+        for (int ch = 0; ch < chunks;) {
+            if (!bar_wait(full + sg, round & 1u)) {
+                ok = false;
+                break;
+            }
+            // The copies are writes of the generic proxy, the products read through
+            // the asynchronous one. The fence stands here: a feeder's would wait
+            // for its copies of the stages behind.
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = smem_addr(smem + sg * 2 * kStageOp), b0 = a0 + kStageOp;
-            const uint32_t id = inst_desc((uint32_t)tn);
-            const int steps = min(TK / 16, (K - ch * TK + 15) / 16);
-            for (int s = 0; s < steps; ++s) {
-                const uint64_t da = smem_desc(a0 + s * 2 * lboA, lboA, kGroup);
-                const uint64_t db = smem_desc(b0 + s * 2 * lboB, lboB, kGroup);
-                const uint32_t acc = (at > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(id), "r"(acc)
-                    : "memory");
+            for (int d = 0; d < deep && ch < chunks; ++d, ++ch) {
+                const uint32_t a0 = smem_addr(smem) + (uint32_t)(sg * deep + d) * size, b0 = a0 + size_a;
+                const int steps = (min(TK, K - ch * TK) + 15) / 16;
+                for (int s = 0; s < steps; ++s) {
+                    const uint64_t da = smem_desc(a0 + s * 2 * step_a, step_a, kGroup);
+                    const uint64_t db = smem_desc(b0 + s * 2 * step_b, step_b, kGroup);
+                    const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                        "l"(da), "l"(db), "r"(id), "r"(acc)
+                        : "memory");
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_addr(bar + sg))
+                             smem_addr(empty + sg))
                          : "memory");
+            if (++sg == stages) {
+                sg = 0;
+                ++round;
+            }
         }
-        if (ch + 1 < c1) {
-            // The other stage is free once the chunk before this one has multiplied.
-            if (at > 0 && !bar_wait(bar + (sg ^ 1), (uint32_t)(((at - 1) >> 1) & 1))) ok = false;
-            part_store(O, smem + ((sg ^ 1) * 2 + half) * kStageOp, RT, t, P);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-        }
+        // Follows every product issued, also where a wait ran out.
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(all))
+                     : "memory");
     }
-    // The last chunk's commit follows every earlier one's.
-    const int last = c1 - 1 - c0;
-    if (!bar_wait(bar + (last & 1), (uint32_t)((last >> 1) & 1))) ok = false;
+    __syncwarp();  // warp 8: the lanes beside the issuing one do not poll
+    if ((warp < 8 || lane == 0) && !bar_wait(all, 0u)) ok = false;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The epilogue's tensor-memory loads are warp-collective: every thread
     // takes the same branch.
     ok = __syncthreads_and(ok) != 0;
     if (!ok && tid == 0) atomicExch(&g_learn_fail, 1);
-    if (ok) {
+    if (ok && warp < 8) {
         // Warp w reads tensor-memory lanes 32(w mod 4)..: row 32(w mod 4) + lane
         // of the tile; warps 0-3 the even groups of 16 columns, 4-7 the odd ones.
         const int r = (warp & 3) * 32 + lane, i = m0 + r;
-        float* share = ws ? ws + ((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * gridDim.z + blockIdx.z) * TM * tn : nullptr;
         for (int cb = half * 16; cb < tn; cb += 32) {
             uint32_t v[16];
             const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb;
@@ -301,62 +449,20 @@ __global__ void __launch_bounds__(256, 3) k_gemm_tc(const __grid_constant__ Oper
                 : "r"(taddr)
                 : "memory");
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (i >= M) continue;
-            if (share) {
-#pragma unroll
-                for (int q = 0; q < 16; q += 4)
-                    *reinterpret_cast<uint4*>(share + (size_t)r * tn + cb + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    if (n0 + cb + q < N) finish(E, i, n0 + cb + q, __uint_as_float(v[q]));
-            }
+            if (i < M && n0 + cb < N) finish(E, i, n0 + cb, N, E.wide && n0 + cb + 16 <= N, v);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 8) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     }
 }
 
-// The shares of a split GEMM summed in order, four columns per thread, eight
-// shares' loads in flight.
-__global__ void __launch_bounds__(128) k_gemm_sum(const float* ws, const __grid_constant__ Epilogue E, int M, int N,
-                                                  int tn, int shares, int tiles_n) {
-    const int q4 = tn >> 2;
-    const int q = blockIdx.x * 128 + threadIdx.x, r = q / q4, c = (q - r * q4) * 4;
-    const int tile = blockIdx.y, ty = tile / tiles_n, i = ty * TM + r, j = (tile - ty * tiles_n) * tn + c;
-    if (r >= TM || i >= M || j >= N) return;
-    const float4* p = reinterpret_cast<const float4*>(ws + ((size_t)tile * shares * TM + r) * tn + c);
-    const size_t step = (size_t)TM * q4;
-    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int s = 0; s < shares; s += 8) {
-        float4 y[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (s + e < shares) y[e] = p[(s + e) * step];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (s + e < shares) {
-                x.x += y[e].x;
-                x.y += y[e].y;
-                x.z += y[e].z;
-                x.w += y[e].w;
-            }
-    }
-    finish(E, i, j, x.x);
-    if (j + 1 < N) finish(E, i, j + 1, x.y);
-    if (j + 2 < N) finish(E, i, j + 2, x.z);
-    if (j + 3 < N) finish(E, i, j + 3, x.w);
-}
-
-__device__ __forceinline__ uint16_t bf16_bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
-
 __global__ void k_to_bf16(const float* src, uint16_t* dst, size_t n) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) dst[q] = bf16_bits(src[q]);
+    if (q < n) dst[q] = bf16_of(src[q]);
 }
 
 __global__ void k_im2col(const float* x, uint16_t* col, int B, int T, int C, int k, int s, int To) {
@@ -366,7 +472,7 @@ __global__ void k_im2col(const float* x, uint16_t* col, int B, int T, int C, int
     const size_t r = q / F, f = q - r * F;
     const int b = (int)(r / To), to = (int)(r - (size_t)b * To);
     const int tap = (int)(f / C), ch = (int)(f - (size_t)tap * C);
-    col[q] = bf16_bits(x[((size_t)b * T + (size_t)to * s + tap) * C + ch]);
+    col[q] = bf16_of(x[((size_t)b * T + (size_t)to * s + tap) * C + ch]);
 }
 
 __global__ void k_col2im(const float* dcol, float* dx, int B, int T, int C, int k, int s, int To) {
@@ -422,74 +528,60 @@ __global__ void __launch_bounds__(256) k_bias_grad(const float* dy, float* db, i
     if (threadIdx.x == 0) db[j] = sh[0];
 }
 
-// The adjoint of an activation, with its bf16 copy and the shares of the bias
-// gradient: dy = da·act'(y) (act 0: dy = da), dyb = bf16(dy), and per block
-// and column the sum of dy over the block's rows. da is read in place, or
-// (k > 0) gathered from the columns' gradient as k_col2im does, da the
-// gradient of a convolution's channels-last input of T positions, kernel k,
-// stride s. Block: 256 threads over `rows_b` rows × 256 / cols at a time.
-__global__ void __launch_bounds__(256) k_dy(const float* y, const float* da, uint16_t* dyb, float* shares, int rows,
-                                            int cols, int act, int T, int k, int s, int To, int rows_b) {
-    __shared__ float sh[256];
-    const int wide = min(cols, 256), groups = 256 / wide;
-    const int g = threadIdx.x / wide, c = blockIdx.y * 256 + threadIdx.x - g * wide;
-    const int r1 = min(rows, (int)(blockIdx.x + 1) * rows_b);
-    float sum = 0.0f;
-    if (g < groups && c < cols)
-        for (int r = blockIdx.x * rows_b + g; r < r1; r += groups) {
-            const size_t at = (size_t)r * cols + c;
-            float d = 0.0f;
-            if (k > 0) {
-                const int b = r / T, t = r - b * T;
-                for (int to = min(t / s, To - 1); to >= 0; --to) {
-                    const int tap = t - to * s;
-                    if (tap >= k) break;
-                    d += da[((size_t)b * To + to) * ((size_t)k * cols) + (size_t)tap * cols + c];
-                }
-            } else {
-                d = da[at];
+// The adjoint of an activation: dy = da·act'(y) (act 0: dy = da) and
+// bf16(dy). da is read in place, or (k > 0) gathered from the columns' gradient
+// as k_col2im does, da the gradient of a convolution's channels-last input of T
+// positions, kernel k, stride s. Bound by its loads; four elements per thread
+// keep them in flight.
+constexpr int kDyPer = 4;
+__global__ void __launch_bounds__(256) k_dy(const float* y, const float* da, uint16_t* dyb, float* dy, size_t n, int cols,
+                                            int act, int T, int k, int s, int To) {
+    const size_t q0 = (size_t)blockIdx.x * (256 * kDyPer) + threadIdx.x;
+#pragma unroll
+    for (int e = 0; e < kDyPer; ++e) {
+        const size_t q = q0 + (size_t)e * 256;
+        if (q >= n) break;
+        float d = 0.0f;
+        if (k > 0) {
+            const size_t r = q / cols;
+            const int c = (int)(q - r * cols), b = (int)(r / T), t = (int)(r - (size_t)b * T);
+            for (int to = min(t / s, To - 1); to >= 0; --to) {
+                const int tap = t - to * s;
+                if (tap >= k) break;
+                d += da[((size_t)b * To + to) * ((size_t)k * cols) + (size_t)tap * cols + c];
             }
-            if (act) {
-                const float v = y[at], q = sigmoid(v);
-                d = d * (q + v * q * (1.0f - q));
-            }
-            dyb[at] = bf16_of(d);
-            sum += d;
+        } else {
+            d = da[q];
         }
-    sh[threadIdx.x] = sum;
-    __syncthreads();
-    if (g == 0 && c < cols) {
-        for (int q = 1; q < groups; ++q) sum += sh[q * wide + threadIdx.x];
-        shares[(size_t)blockIdx.x * cols + c] = sum;
+        if (act) {
+            const float v = y[q], g = sigmoid(v);
+            d = d * (g + v * g * (1.0f - g));
+        }
+        dy[q] = d;
+        dyb[q] = bf16_of(d);
     }
 }
 
-// Column sums of the shares [blocks][cols], one warp per column.
-__global__ void __launch_bounds__(256) k_share_sum(const float* shares, float* out, int blocks, int cols, float scale) {
-    const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (c >= cols) return;
+// Column sums of dy in the order of k_bias_grad (256 strided partial sums,
+// then a tree), four columns per block, so that a warp reads 128 bytes in
+// place of 32 scattered values. A thread's serial sum bounds it (32 columns over
+// 32704 rows: 24 us, 64 over 8064: 12 us).
+__global__ void __launch_bounds__(1024) k_col_sum(const float* dy, float* db, int rows, int cols) {
+    __shared__ float sh[4][256];
+    const int c = blockIdx.x * 4 + (threadIdx.x & 3), t = threadIdx.x >> 2;
     float s = 0.0f;
-    for (int b = lane; b < blocks; b += 32) s += shares[(size_t)b * cols + c];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) out[c] = s * scale;
-}
-
-// The MSE gradient, and the loss's shares (k_share_sum ends it).
-__global__ void __launch_bounds__(256) k_mse(const float* out, const float* target, float* grad, float* shares, size_t n) {
-    __shared__ float sh[8];
-    float s = 0.0f;
-    for (size_t q = (size_t)blockIdx.x * 256 + threadIdx.x; q < n; q += (size_t)gridDim.x * 256) {
-        const float d = out[q] - target[q];
-        grad[q] = 2.0f * d / (float)n;
-        s += d * d;
+    if (c < cols) {
+#pragma unroll 16
+        for (int r = t; r < rows; r += 256) s += dy[(size_t)r * cols + c];
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    sh[threadIdx.x & 3][t] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) s += sh[w];
-        shares[blockIdx.x] = s;
+    const int q = threadIdx.x >> 8, at = threadIdx.x & 255;
+    for (int w = 128; w > 0; w >>= 1) {
+        if (at < w) sh[q][at] += sh[q][at + w];
+        __syncthreads();
     }
+    if (at == 0 && blockIdx.x * 4 + q < cols) db[blockIdx.x * 4 + q] = sh[q][0];
 }
 
 __global__ void k_mse_grad(const float* out, const float* target, float* grad, size_t n) {
@@ -524,7 +616,7 @@ __global__ void k_adam(float* p, uint16_t* pb, const float* g, float* m, float* 
     v[q] = vq;
     const float pq = p[q] - lr * (mq / c1) / (sqrtf(vq / c2) + eps);
     p[q] = pq;
-    pb[q] = bf16_bits(pq);
+    pb[q] = bf16_of(pq);
 }
 
 inline unsigned blocks(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
@@ -539,50 +631,42 @@ int operand_mode(const Operand& o) {
     return 0;
 }
 
-// Tile width, row and column tiles and shares of K. A share takes at least
-// two chunks (the second's loads overlap the first's product); more shares
-// only while the chip has SMs left (148) and a tile's shares stay below what
-// k_gemm_sum reads in a few microseconds.
-struct GemmPlan {
-    int tn, tm, tiles_n, shares, per;
-};
-GemmPlan gemm_plan(int M, int N, int K, size_t ws_floats) {
-    GemmPlan g;
-    g.tn = N >= 128 ? 128 : (N + 15) / 16 * 16;
-    g.tm = (M + TM - 1) / TM;
-    g.tiles_n = (N + g.tn - 1) / g.tn;
-    const int64_t tiles = (int64_t)g.tm * g.tiles_n, chunks = (K + TK - 1) / TK;
-    const int64_t tile = (int64_t)TM * g.tn;
-    const int64_t used = (int64_t)(M < TM ? M : TM) * (N < g.tn ? N : g.tn) * 4;
-    int64_t sh = 148 / tiles;
-    if (sh > (chunks + 1) / 2) sh = (chunks + 1) / 2;
-    if (sh > (int64_t)kSumBytes / used) sh = (int64_t)kSumBytes / used;
-    if (sh > (int64_t)(ws_floats / tile) / tiles) sh = (int64_t)(ws_floats / tile) / tiles;
-    if (sh > 64) sh = 64;
-    if (sh < 1) sh = 1;
-    g.per = (int)((chunks + sh - 1) / sh);
-    g.shares = (int)((chunks + g.per - 1) / g.per);
-    return g;
-}
-
-int gemm(Operand A, Operand B, const Epilogue& E, int M, int N, int K, float* ws, size_t ws_floats, cudaStream_t s) {
+// Makes a job of C = A·B; nonzero if it is none.
+int gemm_job(Operand A, Operand B, Epilogue E, int M, int N, int K, Job& J) {
     if (!A.p || !B.p || M <= 0 || N <= 0 || K <= 0) return 1;
     if (E.bias ? !(E.C || E.outf || E.outb) : !E.C) return 1;
-    // Element offsets are formed in 64 bits; one grid dimension per tile axis.
-    if ((M + TM - 1) / TM > 65535) return 1;
+    if ((M - 1) / TM >= 65535) return 1;
+    E.wide = E.ldc % 8 == 0 && !(((uintptr_t)E.C | (uintptr_t)E.outf | (uintptr_t)E.outb) & 15);
     A.mode = operand_mode(A);
     B.mode = operand_mode(B);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    const int ra = M >= TM ? TM : (M + 15) / 16 * 16, tn = N >= 128 ? 128 : (N + 15) / 16 * 16;
+    const int chunks = (K - 1) / TK + 1, fit = (int)(kStageBytes / (chunk_bytes(ra) + chunk_bytes(tn)));
+    // A stage holds up to four chunks, where three stages of it fit: handing one
+    // over costs as much as the copies and products of a small chunk.
+    const int deep = std::max(1, std::min(std::min(4, fit / 3), chunks));
+    const int stages = std::min(std::min((chunks - 1) / deep + 1, kMaxStages), fit / deep);
+    J = Job{A, B, E, M, N, K, ra, tn, stages, deep, (N - 1) / tn + 1};
+    return 0;
+}
+
+// Launches the products of `jobs` together.
+int gemm(const Job* jobs, int n, cudaStream_t s) {
+    static const cudaError_t attr = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)(kStageBytes + kBarBytes));
     if (attr != cudaSuccess) return 2;
-    const GemmPlan g = gemm_plan(M, N, K, ((uintptr_t)ws & 15) ? 0 : ws_floats);
-    k_gemm_tc<<<dim3(g.tiles_n, g.tm, g.shares), 256, kGemmSmem, s>>>(A, B, E, M, N, K, g.tn, g.per,
-                                                                     g.shares > 1 ? ws : nullptr);
-    if (g.shares > 1) {
-        const int rows = M < TM ? M : TM;
-        k_gemm_sum<<<dim3(blocks((size_t)rows * (g.tn / 4), 128), g.tm * g.tiles_n), 128, 0, s>>>(ws, E, M, N, g.tn, g.shares,
-                                                                                               g.tiles_n);
+    Jobs P{};
+    uint32_t bytes = 0;
+    int64_t blocks = 0;
+    for (int q = 0; q < kJobs; ++q) {
+        P.first[q] = q < n ? (int)blocks : INT_MAX;
+        if (q >= n) continue;
+        const Job& J = P.job[q] = jobs[q];
+        bytes = std::max(bytes, (uint32_t)(J.stages * J.deep) * (chunk_bytes(J.ra) + chunk_bytes(J.tn)) + kBarBytes);
+        if (J.tn > 64) bytes = std::max(bytes, kWideBytes);
+        blocks += (int64_t)((J.M - 1) / TM + 1) * J.tiles_n;
+        if (blocks >= INT_MAX) return 1;
     }
+    k_gemm_tc<<<(unsigned)blocks, kGemmThreads, bytes, s>>>(P);
     return launched();
 }
 
@@ -592,8 +676,10 @@ extern "C" {
 
 int ems_learn_gemm_bf16(const uint16_t* A, int64_t sa0, int64_t sa1, const uint16_t* B, int64_t sb0, int64_t sb1,
                         float* C, int64_t ldc, int M, int N, int K, float alpha, float beta, void* stream) {
-    return gemm(Operand{A, sa0, sa1, 0, 0, 0, 0}, Operand{B, sb1, sb0, 0, 0, 0, 0},
-                Epilogue{C, ldc, alpha, beta, nullptr, 0, nullptr, nullptr}, M, N, K, nullptr, 0, (cudaStream_t)stream);
+    Job J;
+    const int st = gemm_job(Operand{A, sa0, sa1, 0, 0, 0, 0}, Operand{B, sb1, sb0, 0, 0, 0, 0},
+                            Epilogue{C, ldc, alpha, beta, nullptr, 0, nullptr, nullptr, false}, M, N, K, J);
+    return st ? st : gemm(&J, 1, (cudaStream_t)stream);
 }
 
 int ems_learn_run(const ems_learn_cmd* cmds, size_t n, void* stream) {
@@ -604,35 +690,41 @@ int ems_learn_run(const ems_learn_cmd* cmds, size_t n, void* stream) {
         int st = 1;
         switch (c.kind) {
         case EMS_LEARN_TO_BF16: st = ems_learn_to_bf16((const float*)c.p[0], (uint16_t*)c.p[1], (size_t)c.s[0], stream); break;
-        case EMS_LEARN_GEMM:
-            st = gemm(Operand{(const uint16_t*)c.p[0], c.s[0], c.s[1], c.s[5], c.i[4], 0, 0},
-                      Operand{(const uint16_t*)c.p[1], c.s[3], c.s[2], c.s[6], 0, c.i[5], 0},
-                      Epilogue{(float*)c.p[2], c.s[4], 1.0f, 0.0f, (const float*)c.p[3], c.i[3], (float*)c.p[5],
-                               (uint16_t*)c.p[4]},
-                      c.i[0], c.i[1], c.i[2], (float*)c.p[6], (size_t)c.s[7], s);
+        case EMS_LEARN_GEMM: {
+            // The GEMMs that follow without depending on it join its launch.
+            Job jobs[kJobs];
+            int m = 0;
+            for (; m < kJobs && q + m < n && cmds[q + m].kind == EMS_LEARN_GEMM && (!m || cmds[q + m].i[6]); ++m) {
+                const ems_learn_cmd& g = cmds[q + m];
+                st = gemm_job(Operand{(const uint16_t*)g.p[0], g.s[0], g.s[1], g.s[5], g.i[4], 0, 0},
+                              Operand{(const uint16_t*)g.p[1], g.s[3], g.s[2], g.s[6], 0, g.i[5], 0},
+                              Epilogue{(float*)g.p[2], g.s[4], 1.0f, 0.0f, (const float*)g.p[3], g.i[3], (float*)g.p[5],
+                                       (uint16_t*)g.p[4], false},
+                              g.i[0], g.i[1], g.i[2], jobs[m]);
+                if (st) break;
+            }
+            if (m) {
+                const int launch = gemm(jobs, m, s);
+                if (launch) st = launch;
+                q += (size_t)(m - 1);
+            }
             break;
+        }
         case EMS_LEARN_DY: {
-            const int rows = c.i[0], cols = c.i[1], T = c.i[3], k = c.i[4], sd = c.i[5], rows_b = c.i[6];
-            if (!c.p[1] || !c.p[2] || !c.p[3] || !c.p[4] || (c.i[2] && !c.p[0]) || rows <= 0 || cols <= 0 || rows_b <= 0) break;
+            const int rows = c.i[0], cols = c.i[1], T = c.i[3], k = c.i[4], sd = c.i[5];
+            if (!c.p[1] || !c.p[2] || !c.p[3] || !c.p[4] || (c.i[2] && !c.p[0]) || rows <= 0 || cols <= 0) break;
             if (k > 0 && (sd <= 0 || T < k || rows % T)) break;
-            const unsigned nb = blocks((size_t)rows, (unsigned)rows_b);
-            if ((cols + 255) / 256 > 65535) break;
-            k_dy<<<dim3(nb, (cols + 255) / 256), 256, 0, s>>>((const float*)c.p[0], (const float*)c.p[1], (uint16_t*)c.p[2],
-                                                             (float*)c.p[3], rows, cols, c.i[2], T, k, sd,
-                                                             k > 0 ? (T - k) / sd + 1 : 0, rows_b);
-            k_share_sum<<<(cols + 7) / 8, 256, 0, s>>>((const float*)c.p[3], (float*)c.p[4], (int)nb, cols, 1.0f);
+            const size_t m = (size_t)rows * cols;
+            k_dy<<<blocks(m, 256 * kDyPer), 256, 0, s>>>((const float*)c.p[0], (const float*)c.p[1], (uint16_t*)c.p[2],
+                                                         (float*)c.p[3], m, cols, c.i[2], T, k, sd,
+                                                         k > 0 ? (T - k) / sd + 1 : 0);
+            k_col_sum<<<(cols + 3) / 4, 1024, 0, s>>>((const float*)c.p[3], (float*)c.p[4], rows, cols);
             st = launched();
             break;
         }
-        case EMS_LEARN_MSE: {
-            const size_t m = (size_t)c.s[0];
-            if (!c.p[0] || !c.p[1] || !c.p[2] || !c.p[3] || !c.p[4] || !m) break;
-            const unsigned nb = (unsigned)(m < 64 * 256 ? blocks(m, 256) : 64);
-            k_mse<<<nb, 256, 0, s>>>((const float*)c.p[0], (const float*)c.p[1], (float*)c.p[2], (float*)c.p[4], m);
-            k_share_sum<<<1, 256, 0, s>>>((const float*)c.p[4], (float*)c.p[3], (int)nb, 1, 1.0f / (float)m);
-            st = launched();
+        case EMS_LEARN_MSE:
+            st = ems_learn_mse((const float*)c.p[0], (const float*)c.p[1], (float*)c.p[2], (float*)c.p[3], (size_t)c.s[0], stream);
             break;
-        }
         default: break;
         }
         if (st) return st;

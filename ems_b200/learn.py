@@ -48,7 +48,6 @@ CONVS = [(2, 32, 8, 4), (32, 64, 8, 4), (64, 128, 8, 4)]  # (c_in, c_out, kernel
 HIDDEN = 64
 
 TO_BF16, GEMM, DY, MSE = 0, 1, 2, 3  # kinds of Cmd
-WS_FLOATS = 4 << 20  # workspace of the split GEMMs (shares of the largest gradient: 0.5 M floats)
 
 
 class Cmd(C.Structure):
@@ -151,8 +150,7 @@ class Net:
         self.W = param_views(self.p, k_in, t_out)
         self.Wb = param_views(self.pb, k_in, t_out)
         self.G = param_views(self.g, k_in, t_out)
-        self.shares = []  # shares of the bias gradients
-        self.ws = torch.empty(WS_FLOATS, dtype=torch.float32, device=self.dev)
+        self.dy = []  # the layers' gradients in f32
         self._buf_b = -1
 
     # -- plumbing
@@ -179,21 +177,19 @@ class Net:
         return c
 
     def _gemm(self, A, sa, B, sb, M, N, K, C=None, ldc=None, bias=None, act=0, outb=None, outf=None, rows_a=None,
-              rows_b=None):
+              rows_b=None, join=False):
         """C (or act(C + bias)) = A·B; sa, sb: strides of (i, k) and (k, j); rows_a, rows_b: (inner count, outer
-        stride) of a two-level row index."""
+        stride) of a two-level row index; join: with the GEMM before it in the list in one launch."""
         pa, ba = rows_a or (0, 0)
         pb, bb = rows_b or (0, 0)
-        return self._cmd(GEMM, (M, N, K, act, pa, pb), (*sa, *sb, N if ldc is None else ldc, ba, bb, WS_FLOATS),
-                         (A, B, C, bias, outb, outf, self.ws))
+        return self._cmd(GEMM, (M, N, K, act, pa, pb, int(join)), (*sa, *sb, N if ldc is None else ldc, ba, bb),
+                         (A, B, C, bias, outb, outf))
 
     def _dy(self, y, da, dyb, db, rows, cols, act, conv=None):
         """bf16(da·act'(y)) and the bias gradient; conv (T, k, s): da through the adjoint of im2col."""
-        per = 16 * max(1, 256 // cols)  # 16 rows per thread of a block
         T, k, st = conv or (0, 0, 0)
-        n = (rows + per - 1) // per * cols
-        self.shares.append(self.torch.empty(n, dtype=self.torch.float32, device=self.dev))
-        return self._cmd(DY, (rows, cols, act, T, k, st, per), (), (y, da, dyb, self.shares[-1], db))
+        self.dy.append(self.torch.empty(rows * cols, dtype=self.torch.float32, device=self.dev))
+        return self._cmd(DY, (rows, cols, act, T, k, st), (), (y, da, dyb, self.dy[-1], db))
 
     def _bufs(self, B: int):
         """Activation buffers and the launch lists for batch size B."""
@@ -203,7 +199,7 @@ class Net:
         f32, bf = dict(dtype=t.float32, device=self.dev), dict(dtype=t.int16, device=self.dev)
         T, flat, no = self.T, self.shapes[3][2], 2 * self.t_out
         rows = [B * T[q + 1] for q in range(3)]
-        self.shares = []
+        self.dy = []
         # The layers' bf16 inputs, pre-activations and the bf16 gradients of these.
         self.xb = [t.empty(B * T[0] * 2, **bf)] + [t.empty(rows[q] * CONVS[q][1], **bf) for q in range(3)]
         self.ys = [t.empty(rows[q] * CONVS[q][1], **f32) for q in range(3)]
@@ -213,7 +209,7 @@ class Net:
         self.dy5_b, self.da4 = t.empty(B * no, **bf), t.empty(B * HIDDEN, **f32)
         self.dy4_b, self.da3 = t.empty(B * HIDDEN, **bf), t.empty(B * flat, **f32)
         self.grad = t.empty(B * no, **f32)
-        self.loss, self.loss_shares = t.zeros(1, **f32), t.empty(64, **f32)
+        self.loss = t.zeros(1, **f32)
 
         fwd = [self._cmd(TO_BF16, s=(B * T[0] * 2,), p=(None, self.xb[0]))]
         for q, (ci, co, k, st) in enumerate(CONVS):
@@ -224,24 +220,26 @@ class Net:
         fwd.append(self._gemm(self.a4_b, (HIDDEN, 1), self.Wb[4][0], (1, HIDDEN), B, no, HIDDEN, bias=self.W[4][1],
                               outf=self.out))
 
-        # fc2 (identity activation): dW5 = dy5ᵀ a4, db5, da4 = dy5 W5; fc1; the convolutions, last to first.
+        # The gradients of the layers' outputs, last to first: fc2 (identity activation), fc1, the convolutions.
         bwd = [self._dy(None, None, self.dy5_b, self.G[4][1], B, no, 0),
-               self._gemm(self.dy5_b, (1, no), self.a4_b, (HIDDEN, 1), no, HIDDEN, B, self.G[4][0]),
                self._gemm(self.dy5_b, (no, 1), self.Wb[4][0], (HIDDEN, 1), B, HIDDEN, no, self.da4),
                self._dy(self.y4, self.da4, self.dy4_b, self.G[3][1], B, HIDDEN, 1),
-               self._gemm(self.dy4_b, (1, HIDDEN), self.xb[3], (flat, 1), HIDDEN, flat, B, self.G[3][0]),
                self._gemm(self.dy4_b, (HIDDEN, 1), self.Wb[3][0], (flat, 1), B, flat, HIDDEN, self.da3)]
         da, conv = self.da3, None
         for q in range(len(CONVS) - 1, -1, -1):
             ci, co, k, st = CONVS[q]
             bwd.append(self._dy(self.ys[q], da, self.dyb[q], self.G[q][1], rows[q], co, 1, conv))
-            bwd.append(self._gemm(self.dyb[q], (1, co), self.xb[q], (st * ci, 1), co, k * ci, rows[q], self.G[q][0],
-                                  rows_b=(T[q + 1], T[q] * ci)))
             if q:
                 bwd.append(self._gemm(self.dyb[q], (co, 1), self.Wb[q][0], (k * ci, 1), rows[q], k * ci, co,
                                       self.dcols[q]))
                 da, conv = self.dcols[q], (T[q], k, st)
-        mse = self._cmd(MSE, s=(B * no,), p=(self.out, None, self.grad, self.loss, self.loss_shares))
+        # The weights' gradients, dW = dyᵀ·x, in one launch, the longest sums first.
+        for q, (ci, co, k, st) in enumerate(CONVS):
+            bwd.append(self._gemm(self.dyb[q], (1, co), self.xb[q], (st * ci, 1), co, k * ci, rows[q], self.G[q][0],
+                                  rows_b=(T[q + 1], T[q] * ci), join=q > 0))
+        bwd += [self._gemm(self.dy4_b, (1, HIDDEN), self.xb[3], (flat, 1), HIDDEN, flat, B, self.G[3][0], join=True),
+                self._gemm(self.dy5_b, (1, no), self.a4_b, (HIDDEN, 1), no, HIDDEN, B, self.G[4][0], join=True)]
+        mse = self._cmd(MSE, s=(B * no,), p=(self.out, None, self.grad, self.loss))
         self._fwd = (Cmd * len(fwd))(*fwd)
         self._mse = (Cmd * 1)(mse)
         self._bwd = (Cmd * len(bwd))(*bwd)

@@ -45,13 +45,15 @@ int ems_learn_gemm_bf16(const uint16_t* A, int64_t sa0, int64_t sa1, const uint1
  *           two-level, r -> (r / i[4])*s[5] + (r mod i[4])*s[0]; i[5] > 0: the
  *           same for B's k index with s[6] (the rows of a valid convolution of
  *           x[b][T][c] with stride d: i = T_out, outer stride T*c, inner d*c).
- *           p[6], s[7]: workspace of that many floats (16-byte aligned) for a
- *           reduction split over the chip; NULL: not split.
- *  DY       dy = da (p[1]) * act'(y (p[0])) (i[2] as above), bf16(dy) to p[2] and
- *           its column sums to p[4]; rows i[0], cols i[1]. i[4] > 0: da is the
- *           adjoint of im2col of p[1] (kernel i[4], stride i[5], T = i[3]; rows =
- *           B*T). p[3]: ceil(rows / i[6]) * cols floats, i[6] rows per share.
- *  MSE      as ems_learn_mse: p out, target, grad, loss, shares (64 floats); s n. */
+ *           i[6] != 0: does not depend on the GEMM before it in the list (up to six
+ *           such run in one launch).
+ *  DY       dy = da (p[1]) * act'(y (p[0])) (i[2] as above) to p[3], bf16(dy) to
+ *           p[2] and its column sums (as ems_learn_bias_grad) to p[4]; rows i[0],
+ *           cols i[1]. i[4] > 0: da is the adjoint of im2col of p[1] (kernel i[4],
+ *           stride i[5], T = i[3]; rows = B*T).
+ *  MSE      as ems_learn_mse: p out, target, grad, loss; s n.
+ * Every element of a GEMM is one sum over k in order, so the rows of a batch
+ * come out as each would alone. */
 enum { EMS_LEARN_TO_BF16 = 0, EMS_LEARN_GEMM = 1, EMS_LEARN_DY = 2, EMS_LEARN_MSE = 3 };
 typedef struct {
     int32_t kind;

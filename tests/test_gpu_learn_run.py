@@ -1,6 +1,6 @@
-"""Launch lists of the learned stop (ems_learn_run): the GEMM with its
-reduction split over the chip, operands read along either index, rows of a
-convolution read in place, bias and activation in the epilogue; the
+"""Launch lists of the learned stop (ems_learn_run): the GEMM with its sum over
+k in one chain, operands read along either index, rows of a convolution read in
+place, bias and activation in the epilogue; the
 activation adjoint with its bias gradient; the loss. Against numpy in f64 on
 the bf16-rounded operands.
 
@@ -146,3 +146,77 @@ def test_network_at_other_batch_sizes(B):
         assert np.linalg.norm(out - want) <= 5e-3 * np.linalg.norm(want)
         g = cnn.backward(cache, dout, L.T_OUT)
         assert np.linalg.norm(net.g.cpu().numpy() - g) <= 2e-2 * np.linalg.norm(g)
+
+
+def _bits(t):
+    return t.cpu().numpy().view(np.uint32)
+
+
+@pytest.mark.parametrize("B", [2, 33, 130])
+def test_rows_of_a_batch_come_out_as_alone(B):
+    """Every output is one sum over k in order, whatever the batch: bit for bit."""
+    from ems_b200 import learn as L
+
+    net = L.Net(seed=4)
+    x = net.torch.from_numpy(np.random.default_rng(B).standard_normal((B, L.K_IN, 2)).astype(np.float32)).cuda()
+    out = _bits(net.forward(x))
+    for q in (0, B // 2, B - 1):
+        assert np.array_equal(_bits(net.forward(x[q:q + 1]))[0], out[q]), q
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (255, 3), (256, 4), (257, 32), (5000, 5), (32704, 32), (64, 768)])
+def test_bias_gradient_is_summed_as_bias_grad(net, rows, cols):
+    t = net.torch
+    d = t.from_numpy(np.random.default_rng(rows).standard_normal((rows, cols)).astype(np.float32)).cuda()
+    H, S, want = t.empty(rows, cols, dtype=t.int16, device="cuda"), t.empty(cols, device="cuda"), t.empty(cols, device="cuda")
+    _run(net, net._dy(None, d, H, S, rows, cols, 0))
+    assert net.lib.ems_learn_bias_grad(net._ptr(d), net._ptr(want), rows, cols, net._s()) == 0
+    assert np.array_equal(_bits(S), _bits(want))
+
+
+@pytest.mark.parametrize("n", [1, 1025, 49152, 100001])
+def test_loss_is_summed_as_mse(net, n):
+    from ems_b200 import learn as L
+
+    t = net.torch
+    a, b = (t.from_numpy(v).cuda() for v in np.random.default_rng(n).standard_normal((2, n)).astype(np.float32))
+    G, loss, sh, G1, want = (t.empty(q, device="cuda") for q in (n, 1, 64, n, 1))
+    _run(net, net._cmd(L.MSE, s=(n,), p=(a, b, G, loss, sh)))
+    assert net.lib.ems_learn_mse(net._ptr(a), net._ptr(b), net._ptr(G1), net._ptr(want), n, net._s()) == 0
+    assert np.array_equal(_bits(G), _bits(G1)) and np.array_equal(_bits(loss), _bits(want))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 17, 15), (16, 16, 16), (17, 15, 17), (127, 129, 63), (128, 128, 64),
+                                   (129, 127, 65), (24, 40, 255), (40, 24, 256), (8, 8, 257), (32, 16, 2047),
+                                   (128, 64, 769), (256, 256, 320)])
+def test_layouts_and_joined_launches_agree(net, M, N, K):
+    """Operands read along k, along the rows and element by element (tiles',
+    stages' and vectors' edges), alone and several in a launch: the same bits,
+    and the value within the bound above."""
+    t = net.torch
+    rng = np.random.default_rng(M + N + K)
+    (ab, a), (bb, b) = (_bf16(rng.standard_normal(s)) for s in ((M, K), (K, N)))
+    up = lambda n: (n + 7) // 8 * 8  # noqa: E731
+
+    def lay(v, ld, off=0):  # rows of v `ld` elements apart, from element `off` of an allocation on
+        buf = t.zeros(off + v.shape[0] * ld, dtype=t.int16, device="cuda")
+        buf[off:].view(v.shape[0], ld)[:, :v.shape[1]] = t.from_numpy(np.ascontiguousarray(v)).cuda()
+        return buf[off:]
+
+    A = [(lay(ab, up(K)), (up(K), 1)), (lay(ab.T, up(M)), (1, up(M))), (lay(ab, K + 1, 1), (K + 1, 1))]
+    Bs = [(lay(bb.T, up(K)), (1, up(K))), (lay(bb, up(N)), (up(N), 1)), (lay(bb, N + 1, 1), (N + 1, 1))]
+    C = [t.empty(M, N, device="cuda") for _ in range(9)]
+    cmds = [net._gemm(*A[q % 3], *Bs[q // 3], M, N, K, C[q]) for q in range(9)]
+    for c in cmds:
+        _run(net, c)
+    one = [_bits(c) for c in C]
+    tol = 4 * np.sqrt(K) * 2.0 ** -24 * np.max(np.linalg.norm(a, axis=1)) * np.max(np.linalg.norm(b, axis=0))
+    assert np.max(np.abs(C[0].cpu().numpy() - a @ b)) <= tol + 2.0 ** -23 * np.max(np.abs(a @ b))
+    for q in range(1, 9):
+        assert np.array_equal(one[q], one[0]), q
+    for q, c in enumerate(cmds):
+        C[q].zero_()
+        c.i[6] = int(q > 0)
+    _run(net, *cmds)  # six products in the first launch, three in the second
+    for q in range(9):
+        assert np.array_equal(_bits(C[q]), one[0]), q
