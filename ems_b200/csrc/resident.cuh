@@ -94,6 +94,25 @@ struct ResArgs {
     uint64_t wait_ns;
 };
 
+// The barrier counter of a gang: the release covers the block's writes (ordered
+// before it by the block barrier), the acquire its reads after the next one.
+#ifndef EMS_HOST_EMULATION
+#define EMS_GANG_SHARED __shared__
+__device__ __forceinline__ void gang_arrive(uint32_t* bar) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t gang_count(const uint32_t* bar) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+    return v;
+}
+#else
+#define EMS_GANG_SHARED static thread_local
+inline void gang_arrive(uint32_t* bar) { emu::gang_arrive(bar); }
+inline uint32_t gang_count(const uint32_t* bar) { return emu::gang_count(bar); }
+inline uint64_t global_ns() { return 0; }
+#endif
+
 // The barrier of a gang: every write of its blocks before it is visible to
 // all of them after it. False once a wait has run out.
 struct Gang {
@@ -108,14 +127,10 @@ __device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
     ++G.epoch;
     if (threadIdx.x == 0) {
         const uint32_t want = G.epoch * G.size;
-        uint32_t v;
-        // The release covers the block's writes (ordered before it by the
-        // block barrier), the acquire its reads after the next one.
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(G.bar) : "memory");
+        gang_arrive(G.bar);
         uint64_t t0 = 0;
         for (uint32_t it = 0;; ++it) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(G.bar) : "memory");
-            if ((int32_t)(v - want) >= 0) break;
+            if ((int32_t)(gang_count(G.bar) - want) >= 0) break;
             if ((it & 255u) != 255u) continue;
             const uint64_t now = global_ns();
             if (!t0) t0 = now;
@@ -267,11 +282,8 @@ __device__ __forceinline__ void res_update(const ResModel& R, uint32_t t, uint32
 // The slab hooks of one side after its update, each followed by a barrier of
 // the gang; false once a wait has run out.
 template <int SIDE>
-__device__ __forceinline__ bool res_slabs(const ResModel& R, Gang& G, uint32_t rank, int* ok, bool capture) {
+__device__ __forceinline__ bool res_slabs(const ResModel& R, Gang& G, uint32_t rank, int* ok) {
     const uint32_t t = rank * blockDim.x + threadIdx.x, stride = G.size * blockDim.x;
-    // The saved values of the other field's poles: it does not change here.
-    if (SIDE == 0 && capture) res_capture(R, true, t, stride);
-    if (SIDE == 1 && R.m.ph.n_edges && !R.fold_h) res_capture(R, false, t, stride);
     for (int q = 0; q < 2 && R.order[q] >= 0; ++q) {
         if (R.order[q] == 0) {
             if (!R.units[SIDE] || R.quad_cpml) continue;
@@ -296,8 +308,8 @@ constexpr uint32_t kHookGang = 8;
 
 template <bool OE>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_constant__ ResArgs A) {
-    __shared__ __align__(16) unsigned char raw[sizeof(ResModel)];
-    __shared__ int ok;
+    __align__(16) EMS_GANG_SHARED unsigned char raw[sizeof(ResModel)];
+    EMS_GANG_SHARED int ok;
     const ResModel& R = *reinterpret_cast<const ResModel*>(raw);
     const uint4 b = A.blocks[blockIdx.x];
     Gang G{A.bars + b.x * 32u, b.z, 0u, A.status, A.wait_ns};
@@ -327,16 +339,25 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 serial_pre(R.m.f, R.ops, R.n_ops);
                 if (R.late_probes && s) hook(true, step - 1u, true, false);
             }
-            if (!(apart && hooks)) res_update<0, OE>(R, t, stride);
+            // The saved values of the other field's poles go beside an update: the
+            // field does not change before the barrier behind it. (After that
+            // barrier there may be none up to the update that writes the field.)
+            if (!(apart && hooks)) {
+                if (R.m.pe.n_edges && (!R.fold_e || (R.capture_first && s == 0))) res_capture(R, true, t, stride);
+                res_update<0, OE>(R, t, stride);
+            }
             if (!gang_sync(G, &ok)) return;
-            if (!res_slabs<0>(R, G, rank, &ok, R.m.pe.n_edges && (!R.fold_e || (R.capture_first && s == 0)))) return;
+            if (!res_slabs<0>(R, G, rank, &ok)) return;
             // Hooks that write i before the E update, in order with the current
             // probes; else the probes beside it.
             if (hooks) hook(false, step, true, true);
             if (R.serial_h && !gang_sync(G, &ok)) return;
-            if (!(apart && hooks)) res_update<1, OE>(R, t, stride);
+            if (!(apart && hooks)) {
+                if (R.m.ph.n_edges && !R.fold_h) res_capture(R, false, t, stride);
+                res_update<1, OE>(R, t, stride);
+            }
             if (!gang_sync(G, &ok)) return;
-            if (!res_slabs<1>(R, G, rank, &ok, false)) return;
+            if (!res_slabs<1>(R, G, rank, &ok)) return;
             if (R.writes_e || (R.serial_e && !R.late_probes)) {
                 if (hooks) hook(true, step, !R.late_probes, true);
                 if (!gang_sync(G, &ok)) return;

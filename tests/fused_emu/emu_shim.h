@@ -67,6 +67,11 @@ inline void sincospi(double x, double* s, double* c) {
     *c = std::cos(3.14159265358979323846 * x);
 }
 
+inline uint32_t __umulhi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+// Lane 0's own value: the emulated kernels read it for sums of one entry only.
+template <class T>
+inline T __shfl_sync(unsigned, T v, unsigned) { return v; }
+
 inline unsigned atomicAdd(uint32_t* p, uint32_t v) { return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST); }
 inline int atomicExch(int* p, int v) { return __atomic_exchange_n(p, v, __ATOMIC_SEQ_CST); }
 
@@ -94,6 +99,11 @@ struct Block {
 extern Block* cur;
 
 void fail(const char* what);
+
+// The barrier counter of a gang of one-thread blocks (k_resident): a waiting
+// block hands the run over to the next one (harness.cpp).
+void gang_arrive(uint32_t* bar);
+uint32_t gang_count(const uint32_t* bar);
 
 inline unsigned char* dynamic_smem() { return cur->smem; }
 

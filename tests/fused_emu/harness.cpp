@@ -5,7 +5,9 @@
 // the surrounding tables' sizes (the tests run it under the same sizes).
 #include "emu_shim.h"
 
+#include <condition_variable>
 #include <memory>
+#include <mutex>
 
 thread_local EmuDim threadIdx;
 EmuDim blockIdx, blockDim, gridDim;
@@ -13,6 +15,41 @@ namespace emu {
 Block* cur = nullptr;
 void fail(const char* what) {
     if (cur && cur->errors.fetch_add(1) == 0) std::snprintf(cur->msg, sizeof cur->msg, "%s", what);
+}
+
+// The blocks of a gang run one at a time: a block keeps the run until it waits
+// at a barrier that is not complete (or ends), then the next in turn has it.
+// The last to arrive goes on alone to its next barrier, far ahead of the others,
+// so work that misses a barrier sees the most reordering one barrier allows.
+struct Turns {
+    std::mutex m;
+    std::condition_variable cv;
+    unsigned n = 0, at = 0;
+    bool down = false;  // from the last block to the first
+    std::vector<bool> done;
+    void wait(std::unique_lock<std::mutex>& l, unsigned me) { cv.wait(l, [&] { return at == me; }); }
+    void pass() {
+        for (unsigned q = 0; q < n; ++q) {
+            at = down ? (at + n - 1) % n : (at + 1) % n;
+            if (!done[at]) break;
+        }
+        cv.notify_all();
+    }
+};
+static Turns* turns = nullptr;
+static thread_local unsigned turn_me;
+void gang_arrive(uint32_t* bar) { ++*bar; }
+// Read again only after the other blocks have had their turns.
+uint32_t gang_count(const uint32_t* bar) {
+    static thread_local bool again = false;
+    static thread_local uint32_t last = 0;
+    if (again && *bar == last) {
+        std::unique_lock<std::mutex> l(turns->m);
+        turns->pass();
+        turns->wait(l, turn_me);
+    }
+    again = true;
+    return last = *bar;
 }
 }  // namespace emu
 
@@ -22,6 +59,12 @@ void fail(const char* what) {
 #include "../../ems_b200/csrc/split.cuh"
 #include "../../ems_b200/csrc/interior.cuh"
 #include "../../ems_b200/csrc/march.cuh"
+#include "../../ems_b200/csrc/batch.cuh"
+// The blocks of a gang are host threads, each with a block index of its own.
+static thread_local EmuDim gang_block;
+#define blockIdx gang_block
+#include "../../ems_b200/csrc/resident.cuh"
+#undef blockIdx
 
 using namespace emsk;
 
@@ -851,4 +894,174 @@ extern "C" int emu_march_run(const ems_engine_desc* d, uint64_t steps, float** f
     if (rows == 3) return march_run<3, 4>(d, steps, fields, planes);
     std::snprintf(g_err, sizeof g_err, "rows must be 3, 7 or 8");
     return 1;
+}
+
+// Runs `steps` resident steps (k_resident) of a gang of `blocks` one-thread
+// blocks, in the order of Turns (down: from the last block), from the fields
+// given in reference layout (overwritten). fold: the pole kernels store the
+// saved values where the model allows it, as a single engine's; 0: they are
+// captured every step, as in a batch. Models with a CPML first (or none), poles
+// and no serial hooks.
+extern "C" int emu_resident_run(const ems_engine_desc* d, unsigned blocks, int down, int fold, uint64_t steps,
+                                float** fields) {
+    g_err[0] = 0;
+    Grid g{};
+    g.nx = (uint32_t)d->nodes[0];
+    g.ny = (uint32_t)d->nodes[1];
+    g.nz = (uint32_t)d->nodes[2];
+    g.pitch = (g.nz + 31u) & ~31u;
+    g.n = (uint64_t)g.nx * g.ny * g.nz;
+    g.np = (uint64_t)g.nx * g.ny * g.pitch;
+    FusedTables T = build_fused_tables(d, g.pitch);
+    if (!T.why.empty()) {
+        std::snprintf(g_err, sizeof g_err, "not eligible: %s", T.why.c_str());
+        return 1;
+    }
+    auto pad = [&](const float* src, std::vector<float>& dst) {
+        dst.assign(g.np, 0.0f);
+        for (size_t r = 0; r < (size_t)g.nx * g.ny; ++r) std::memcpy(&dst[r * g.pitch], src + r * g.nz, g.nz * 4);
+    };
+    std::vector<float> buf[6], dense[12];
+    ResModel R{};
+    FusedParams& P = R.m.P;
+    P.g = g;
+    P.dt = d->dt;
+    for (int c = 0; c < 6; ++c) pad(fields[c], buf[c]);
+    for (int l = 0; l < 12; ++l) {
+        pad(d->coeff[l], dense[l]);
+        R.m.c.c[l] = dense[l].data();
+        if (T.lane[l].pooled) {
+            P.lane[l].rid = T.lane[l].rid.data();
+            P.lane[l].rows = T.lane[l].rows.data();
+        } else {
+            P.lane[l].dense = dense[l].data();
+        }
+    }
+    std::vector<std::vector<float>> psi;
+    for (int side = 0; side < 2; ++side)
+        for (int c = 0; c < 3; ++c) P.nslab[side][c] = T.nslab[side][c];
+    for (const FusedSlabSpec& sp : T.slabs) {
+        FSlab& f = P.slab[sp.side][sp.comp][sp.q];
+        for (int a = 0; a < 3; ++a) {
+            f.lo[a] = (uint32_t)sp.src->lo[a];
+            f.hi[a] = (uint32_t)sp.src->hi[a];
+        }
+        f.normal = (uint32_t)sp.src->normal;
+        f.b = sp.src->b;
+        f.a = sp.src->a;
+        f.k = sp.src->k;
+        psi.emplace_back(sp.len, 0.0f);
+        f.psi_old = f.psi_new = psi.back().data();
+    }
+    for (int a = 0; a < 3; ++a) {
+        P.cmask[a] = T.cmask[a].data();
+        P.uo[a] = P.un[a] = R.m.f.u[a] = buf[a].data();
+        P.io[a] = P.in[a] = R.m.f.i[a] = buf[3 + a].data();
+    }
+    R.order[0] = R.order[1] = -1;
+    int n_ops = 0;
+    std::vector<uint32_t> node[2];
+    std::vector<float> prev[2];
+    std::vector<double> j[2], q[2];
+    for (size_t k = 0; k < d->n_ops; ++k) {
+        const int kind = d->ops[k].kind;
+        if (kind == EMS_OP_CPML && n_ops == 0) {
+            R.order[n_ops++] = 0;
+            R.quad_cpml = 1;
+        } else if (kind == EMS_OP_POLES) {
+            R.order[n_ops++] = 1;
+            const auto* p = (const ems_poles*)d->ops[k].table;
+            for (int s = 0; s < 2; ++s) {
+                const ems_pole_side& t = s ? p->magnetic : p->electric;
+                PoleSideDev& o = s ? R.m.ph : R.m.pe;
+                for (size_t e = 0; e < t.n_edges; ++e)
+                    node[s].push_back((uint32_t)(t.node[e] / g.nz * g.pitch + t.node[e] % g.nz));
+                prev[s].assign(t.n_edges, 0.0f);
+                j[s].assign(t.n_poles, 0.0);
+                q[s].assign(t.n_poles, 0.0);
+                o.n_edges = t.n_edges;
+                o.n_poles = t.n_poles;
+                o.axis = t.axis;
+                o.node = node[s].data();
+                o.sum_inv_z = t.sum_inv_z;
+                o.pole_end = t.pole_end;
+                o.kind = t.kind;
+                o.a = t.a;
+                o.inv_c = t.inv_c;
+                o.inv_z = t.inv_z;
+                o.half_l = t.half_l;
+                o.prev = prev[s].data();
+                o.j = j[s].data();
+                o.q = q[s].data();
+            }
+        } else {
+            std::snprintf(g_err, sizeof g_err, "only a CPML, then poles are emulated");
+            return 1;
+        }
+    }
+    P.runs = T.runs.data();
+    P.sets = T.sets.data();
+    P.runs_h = T.h.runs.data();
+    P.sets_h = T.h.sets.data();
+    R.m.run_of[0] = T.run_of.data();
+    R.m.run_of[1] = T.h.run_of.data();
+    R.m.dt = d->dt;
+    R.fold_e = fold && T.has_poles && pole_prev_fold(d, true, false);
+    R.fold_h = fold && T.has_poles_h && pole_prev_fold(d, false, false);
+    R.capture_first = 1;
+    R.div_q = fast_div((g.nz + 3u) / 4u);
+    R.div_j = fast_div(g.ny);
+    R.quads = g.nx * g.ny * ((g.nz + 3u) / 4u);
+    std::vector<uint2> layer[2];
+    std::vector<uint32_t> inner[2];
+    for (int side = 0; side < 2 && R.quad_cpml; ++side) {
+        cpml_quads(slab_geometry(T), d->nodes, side, layer[side], inner[side]);
+        R.layer[side] = layer[side].data();
+        R.inner[side] = inner[side].data();
+        R.n_layer[side] = (uint32_t)layer[side].size();
+    }
+    std::vector<uint4> bl(blocks);
+    for (unsigned b = 0; b < blocks; ++b) bl[b] = uint4{0, b, blocks, 0};
+    const uint2 gang{0, 1};
+    const uint32_t list = 0;
+    uint32_t bars[64] = {};
+    int status = 0;
+    ResArgs A{&R, bl.data(), &gang, &list, bars, bars + 32, 1u, (uint32_t)steps, 0u, nullptr, &status, 1u};
+    blockDim = EmuDim{1, 1, 1};
+    gridDim = EmuDim{blocks, 1, 1};
+    emu::Block blk;
+    std::barrier<> bar(1);
+    blk.bar = &bar;
+    emu::cur = &blk;
+    emu::Turns turns;
+    turns.n = blocks;
+    turns.down = down != 0;
+    turns.at = down ? blocks - 1 : 0;
+    turns.done.assign(blocks, false);
+    emu::turns = &turns;
+    std::vector<std::thread> th;
+    for (unsigned b = 0; b < blocks; ++b)
+        th.emplace_back([&, b] {
+            threadIdx = EmuDim{};
+            gang_block.x = b;
+            emu::turn_me = b;
+            {
+                std::unique_lock<std::mutex> l(turns.m);
+                turns.wait(l, b);
+            }
+            k_resident<false>(A);
+            std::unique_lock<std::mutex> l(turns.m);
+            turns.done[b] = true;
+            turns.pass();
+        });
+    for (auto& t : th) t.join();
+    emu::cur = nullptr;
+    if (status) {
+        std::snprintf(g_err, sizeof g_err, "status flag set");
+        return 3;
+    }
+    for (int c = 0; c < 6; ++c)
+        for (size_t r = 0; r < (size_t)g.nx * g.ny; ++r)
+            std::memcpy(fields[c] + r * g.nz, &buf[c][r * g.pitch], g.nz * 4);
+    return 0;
 }

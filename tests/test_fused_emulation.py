@@ -43,6 +43,8 @@ def emu_lib(asan=False):
     lib.emu_march_run.argtypes = [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint32, C.c_uint32]
     lib.emu_march_timeout.restype = C.c_int
     lib.emu_march_timeout.argtypes = [C.c_void_p, C.c_void_p, C.c_uint64]
+    lib.emu_resident_run.restype = C.c_int
+    lib.emu_resident_run.argtypes = [C.c_void_p, C.c_uint, C.c_int, C.c_int, C.c_uint64, C.c_void_p]
     lib.emu_pole_prev_fold.restype = C.c_int
     lib.emu_pole_prev_fold.argtypes = [C.c_void_p, C.c_int]
     lib.emu_error.restype = C.c_char_p
@@ -266,6 +268,38 @@ def test_march_bounded_wait_runs_out_and_reports():
     arrs[2][6, 5, 14] = np.nan
     ptrs = (C.c_void_p * 6)(*[a.ctypes.data for a in arrs])
     assert lib.emu_march_run(m.desc, 1, ptrs, 7, 4) == 4, lib.emu_error().decode()
+
+
+@pytest.mark.parametrize("cpml", [0, 3])
+@pytest.mark.parametrize("sides", ["electric", "magnetic", "both"])
+@pytest.mark.parametrize("fold", [0, 1])
+def test_resident_gang_equals_oracle(cpml, sides, fold):
+    """The resident kernel over a gang of blocks that run as far ahead of one
+    another as its barriers allow (one at a time, in both orders), from nonzero
+    fields, the saved values of the poles captured every step (as in a batch) or
+    at the first one: fields bit-exact with the oracle. The pole edges keep only
+    part of the gang busy."""
+    n = (9, 8, 11)
+    m = E.Model.uniform(n, [1e-3] * 3)
+    m.fill(m.cells().box([2, 2, 2], [6, 6, 7]), m.material(eps_r=2.0, kappa=0.01))
+    m.build()
+    if cpml:
+        m.add_cpml([2] * 6, kappa_max=1.5, alpha_max=0.02)
+    d = E.Dispersive()
+    if sides != "magnetic":
+        d.fill_cells(m, m.cells().box([5, 4, 4], [8, 7, 9]), W.lorentz_poles(5))
+    if sides != "electric":
+        d.fill_cells(m, m.cells().box([3, 3, 5], [6, 6, 8]), [E.Pole.drude(2e10, 3e9)], field=1)
+    m.add_dispersive(d, E.TRAPEZOIDAL)
+    state, lib, steps = random_state(m, seed=8), emu_lib(), 3
+    want, _, _ = run_oracle(m, state, steps)
+    for blocks, down in ((5, 0), (5, 1), (9, 0), (9, 1), (1, 0)):
+        arrs = [np.ascontiguousarray(x.copy()) for x in state]
+        ptrs = (C.c_void_p * 6)(*[a.ctypes.data for a in arrs])
+        assert lib.emu_resident_run(m.desc, blocks, down, fold, steps, ptrs) == 0, lib.emu_error().decode()
+        for name, a, b in zip(["u_x", "u_y", "u_z", "i_x", "i_y", "i_z"], arrs, want):
+            bad = np.argwhere(a.view(np.uint32) != b.view(np.uint32))
+            assert bad.size == 0, f"{blocks} blocks, down {down}, {name}: {len(bad)} differ, first {tuple(bad[0])}"
 
 
 def test_pole_capture_fold_decision():

@@ -89,6 +89,66 @@ def test_resident_equals_split(name, curl):
         assert np.array_equal(x.view(np.uint64), y.view(np.uint64)), (name, op, which)
 
 
+def _poles(n, sides, cpml, source, first=False):
+    """Poles that keep only part of a gang busy; a source on a pole edge makes
+    the saved values be captured every step; first: before the CPML."""
+    m = E.Model.uniform(n, [1e-3] * 3)
+    m.build(courant=0.95)
+    h = [q // 2 for q in n]
+
+    def poles():
+        d = E.Dispersive()
+        if sides != "magnetic":
+            d.fill_cells(m, m.cells().box([h[0], h[1], 2], [n[0] - 2, n[1] - 2, n[2] - 2]), W.lorentz_poles(5))
+        if sides != "electric":
+            d.fill_cells(m, m.cells().box([2, 2, h[2]], [h[0], h[1], n[2] - 1]), [E.Pole.drude(2e10, 3e9)], field=1)
+        m.add_dispersive(d, E.LEAPFROG)
+
+    if first:
+        poles()
+    if cpml:
+        m.add_cpml([4] * 6)
+    if not first:
+        poles()
+    if source:
+        m.add_source_table(E.SOFT_E, [(E.Z, (h[0] + 2, h[1] + 2, h[2]), 1.0)], np.cos(0.2 * np.arange(100)))
+    return m
+
+
+@pytest.mark.parametrize("sides", ["electric", "magnetic", "both"])
+@pytest.mark.parametrize("cpml,source,first", [(0, 0, 0), (1, 0, 0), (1, 1, 0), (0, 1, 0), (1, 0, 1), (1, 1, 1)])
+def test_resident_poles_equal_split(sides, cpml, source, first):
+    """Electric and magnetic poles over a gang of many blocks, resident against
+    split and in a batch, from nonzero fields and after an upload."""
+    n = (61, 45, 53)
+    m = _poles(n, sides, cpml, source, first)
+    g, s = E.Engine(m), E.Engine(m)
+    s.set_schedule(4)
+    rng = np.random.default_rng(11)
+    for e in (g, s):
+        before = e.launches
+        e.run(1)
+        assert (e.launches - before == 1) == (e is g)
+    for steps in (7, 1, 12):
+        u = [rng.standard_normal(g.nodes).astype(np.float32) for _ in range(2)]
+        for e in (g, s):
+            for f in range(2):
+                e.set_field(f, 2, u[f])
+            e.run(steps)
+        assert_fields_equal(g, s, f"{steps} steps")
+    if source:
+        b = E.Batch([m, _cavity((9, 8, 7))[0], m], max_steps=100)
+        s = E.Engine(m)
+        s.set_schedule(4)
+        for steps in (30, 11):
+            b.run(steps)
+            s.run(steps)
+        for q in (0, 2):
+            for f in range(2):
+                for a in range(3):
+                    assert np.array_equal(b.field(q, f, a).view(np.uint32), s.field(f, a).view(np.uint32)), (q, f, a)
+
+
 def test_batch_of_more_models_than_blocks():
     """More models than resident blocks (two per SM): a block takes several,
     each for the whole run."""
