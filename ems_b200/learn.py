@@ -260,8 +260,16 @@ class Net:
 
     def backward(self, dout):
         """Gradients of the last forward's output dout (B, 2·t_out) → self.g."""
-        dout = dout.to(self.torch.float32).contiguous()
-        self._bwd[0].p[1] = dout.data_ptr()
+        n = self._buf_b * 2 * self.t_out
+        if tuple(dout.shape[:1]) != (self._buf_b,):
+            raise RuntimeError(f"backward: a gradient of shape {tuple(dout.shape)} for outputs of shape ({self._buf_b}, "
+                               f"{2 * self.t_out})")
+        d = dout.reshape(-1)
+        if d.shape[0] != n or d.dtype != self.torch.float32 or d.device != self.grad.device or not d.is_contiguous():
+            # Another type, device or layout; refuses another number of values.
+            self.grad.copy_(d)
+            d = self.grad
+        self._bwd[0].p[1] = d.data_ptr()
         self._run(self._bwd)
 
     def adam(self, lr: float = 1e-3, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8) -> None:

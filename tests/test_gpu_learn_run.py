@@ -220,3 +220,22 @@ def test_layouts_and_joined_launches_agree(net, M, N, K):
     _run(net, *cmds)  # six products in the first launch, three in the second
     for q in range(9):
         assert np.array_equal(_bits(C[q]), one[0]), q
+
+
+def test_backward_takes_gradients_of_other_types_and_places():
+    from ems_b200 import learn as L
+
+    net = L.Net(seed=5)
+    t = net.torch
+    rng = np.random.default_rng(1)
+    net.forward(t.from_numpy(rng.standard_normal((5, L.K_IN, 2)).astype(np.float32)).cuda())
+    d = t.from_numpy(rng.standard_normal((5, 2 * L.T_OUT)).astype(np.float32)).cuda()
+    net.backward(d)
+    want = _bits(net.g)
+    for other in (d.cpu(), d.double(), d.t().contiguous().t()):
+        net.g.zero_()
+        net.backward(other)
+        assert np.array_equal(_bits(net.g), want)
+    for bad in (d[:4], d[:, :-1], t.cat([d, d])):
+        with pytest.raises(RuntimeError):
+            net.backward(bad)

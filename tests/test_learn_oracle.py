@@ -64,3 +64,31 @@ def test_example_verify_and_splice_on_an_exact_prediction():
     cut = Lr.s11_db(np.arange(stop), v[:stop], i[:stop], dt, freqs)
     err_sp, err_cut = np.max(np.abs(sp - full)), np.max(np.abs(cut - full))
     assert err_sp < 0.1 and err_cut > 5 * err_sp  # the predicted tail is what makes the early stop exact
+
+
+def test_backward_checks_its_gradient():
+    """What Net.backward hands to the kernels: the gradient itself where it is
+    what they read, else a copy of it in the network's buffer; a gradient of
+    another shape is refused (on the CPU, the launches recorded)."""
+    import ctypes as C
+
+    import pytest
+    import torch
+
+    from ems_b200 import learn as L
+
+    net = L.Net.__new__(L.Net)
+    net.torch, net.t_out, net._buf_b = torch, 3, 4
+    net.grad = torch.zeros(24)
+    net._bwd, seen = (L.Cmd * 1)(), []
+    net._run = lambda cmds: seen.append((cmds[0].p[1], np.ctypeslib.as_array((C.c_float * 24).from_address(cmds[0].p[1])).copy()))
+    ok = torch.randn(4, 6)
+    for d in (ok, ok.view(4, 3, 2), ok.double(), ok.half(), ok.t().contiguous().t(), ok[:, :1].expand(4, 6)):
+        net.backward(d)
+        at, values = seen.pop()
+        assert np.array_equal(values, d.float().reshape(-1).numpy())
+        assert (at == ok.data_ptr()) == (d.data_ptr() == ok.data_ptr() and d.is_contiguous())
+    for shape in ((3, 6), (4, 5), (8, 3), (2, 12), (4, 7), (5, 6), (1, 6), ()):
+        with pytest.raises(RuntimeError):
+            net.backward(torch.zeros(shape))
+    assert not seen
