@@ -307,6 +307,7 @@ GPU_SYMBOLS = {
     "ems_batch_samples": (C.c_int, [C.c_void_p, C.c_size_t, C.c_size_t, C.c_int, C.c_void_p, C.c_size_t,
                                     C.c_void_p]),
     "ems_batch_download_field": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_void_p]),
+    "ems_batch_test_wait_timeout": (C.c_int, [C.c_void_p, C.c_uint64]),
     "ems_batch_stream": (C.c_int, [C.c_void_p, C.c_void_p]),
     "ems_batch_last_error": (C.c_char_p, [C.c_void_p]),
 }
@@ -927,7 +928,7 @@ class Engine:
         self._ck(self._lib.ems_gpu_check(self._h))
 
     def test_wait_timeout(self, limit_ns: int) -> None:
-        """Arms the bounded-wait test hook for the next marching step."""
+        """Arms the bounded-wait test hook for the next marching step or resident launch."""
         self._ck(self._lib.ems_gpu_test_wait_timeout(self._h, limit_ns))
 
     def set_march(self, shape: int = 0, planes: int = 32) -> None:
@@ -1133,6 +1134,10 @@ class Batch:
         out = np.empty(self._models[model].nodes, dtype=np.float32)
         self._ck(self._lib.ems_batch_download_field(self._h, model, field, axis, out.ctypes.data))
         return out
+
+    def test_wait_timeout(self, limit_ns: int) -> None:
+        """Arms the bounded-wait test hook for the next resident launch."""
+        self._ck(self._lib.ems_batch_test_wait_timeout(self._h, limit_ns))
 
     @property
     def stream(self) -> int:

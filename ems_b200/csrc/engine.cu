@@ -90,7 +90,7 @@ struct ems_gpu {
     double* shares = nullptr;     // first pass of a long sum (kSumBlocks)
     int* flags = nullptr;         // pinned copy of the status and divergence flags
     int* diverged = nullptr;      // set on the device where a marching step writes a non-finite value
-    uint64_t test_wait_ns = 0;    // ems_gpu_test_wait_timeout: the next marching step's waits run out
+    uint64_t test_wait_ns = 0;    // ems_gpu_test_wait_timeout: the next marching or resident launch's waits run out
     struct CpmlDev {
         SlabDev s;
     };
@@ -219,7 +219,8 @@ struct ems_gpu {
         std::vector<int> place;           // per operator its place, -1: not in the table
         uint64_t ready = ~0ull;           // buffers and amplitudes hold the steps before this one
         bool late_h = false;              // no hook writes i: current probes wait for the electric hooks
-        double* mail = nullptr;           // pinned, 3 per operator
+        double* mail = nullptr;           // pinned, 3 per operator, then `told`
+        int* told = nullptr;              // set by a resident launch whose wait ran out
     } hooks;
     // Pinned staging of field downloads, two buffers of `cap` floats, made on
     // the first download.
@@ -1402,6 +1403,12 @@ unsigned resident_blocks(int device, int threads) {
     return (unsigned)(sms * std::min(per, oe));
 }
 
+// Arms the test hook of the bounded waits: a counter one short, so that the
+// first barrier's waits run out.
+ems_status resident_short(uint32_t* bar, cudaStream_t s) {
+    return cudaMemsetAsync(bar, 0xff, sizeof(uint32_t), s) == cudaSuccess ? EMS_OK : EMS_ERR_CUDA;
+}
+
 // The model's tables for the resident kernel (all but its ops).
 void resident_model(ems_gpu* h, ResModel& R) {
     const Grid& g = h->g;
@@ -1528,9 +1535,12 @@ ems_status put_table(ems_gpu* h, std::vector<unsigned char>& held, void* dev, co
 ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
     auto& k = h->hooks;
     if (k.ready == h->step + n) return EMS_OK;
-    if (!k.mail && check(h, cudaHostAlloc((void**)&k.mail, (h->ops.size() + 1) * 3 * sizeof(double), cudaHostAllocMapped),
-                         "serial hooks"))
-        return EMS_ERR_CUDA;
+    if (!k.mail) {
+        const size_t n = (h->ops.size() + 1) * 3;
+        if (check(h, cudaHostAlloc((void**)&k.mail, n * sizeof(double), cudaHostAllocMapped), "serial hooks")) return EMS_ERR_CUDA;
+        std::memset(k.mail, 0, n * sizeof(double));
+        k.told = (int*)(k.mail + n - 3);
+    }
     bool moved = k.held.empty();
     for (auto& op : h->ops) {
         ems_status st = EMS_OK;
@@ -1708,7 +1718,12 @@ ems_status run_resident(ems_gpu* h, uint64_t n) {
     st = put_table(h, r.model, r.d_model, raw, sizeof raw);
     if (st) return st;
     ResArgs A{r.d_model, r.blocks, r.gangs, r.list, r.bars + 32 * r.flip, r.bars + 32 * (r.flip ^ 1), 1u, (uint32_t)n,
-              (uint32_t)h->step, nullptr, h->status, kWaitNs};
+              (uint32_t)h->step, nullptr, h->status, h->hooks.told, kWaitNs};
+    if (h->test_wait_ns) {
+        A.wait_ns = h->test_wait_ns;
+        h->test_wait_ns = 0;
+        if (resident_short(A.bars, h->stream)) return fail(h, EMS_ERR_CUDA, "test hook");
+    }
     r.flip ^= 1;
     cudaError_t e;
     launch_resident(A, h->oe_curl, r.grid, kResThreads, h->stream, &e);
@@ -2784,6 +2799,7 @@ static ems_status device_status(ems_gpu* h) {
     if (check(h, cudaStreamSynchronize(h->stream), "status")) return EMS_ERR_CUDA;
     const int st[2] = {h->flags[0], h->flags[1]};
     if (st[0] || st[1]) {
+        if (h->hooks.told) *(volatile int*)h->hooks.told = 0;
         if (h->status) cudaMemsetAsync(h->status, 0, sizeof(int), h->stream);
         cudaMemsetAsync(h->diverged, 0, sizeof(int), h->stream);
         if (check(h, cudaStreamSynchronize(h->stream), "status")) return EMS_ERR_CUDA;
@@ -2975,8 +2991,10 @@ ems_status ems_gpu_last_sample(ems_gpu* h, size_t op, int which, double* out) {
         cnt = o.lumped.count;
     }
     if (!src || !cnt) return fail(h, EMS_ERR_INVALID, "no sample");
-    // The hooks have left the newest samples in host memory.
+    // The hooks have left the newest samples in host memory, and a launch that
+    // gave up its flag.
     if (check(h, cudaStreamSynchronize(h->stream), "sample")) return EMS_ERR_CUDA;
+    if (*(volatile int*)h->hooks.told) return device_status(h);
     *out = ((volatile double*)h->hooks.mail)[3 * op + which];
     return EMS_OK;
 }
@@ -3187,6 +3205,7 @@ struct ems_batch {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
     } tune;
     int grid_code = 1;
+    uint64_t test_wait_ns = 0;  // ems_batch_test_wait_timeout
     // Resident steps (resident.cuh): a gang of blocks per active model.
     struct Resident {
         bool ok = false, stale = true;  // stale: the gangs are not those of the active models
@@ -3377,7 +3396,12 @@ ems_status batch_resident(ems_batch* b, uint64_t n) {
         if (ems_status st = resident_plan(b)) return st;
     if (!r.grid) return EMS_OK;
     ResArgs A{r.models, r.blocks, r.gangs, r.list, r.bars + (size_t)32 * r.fit * r.flip,
-              r.bars + (size_t)32 * r.fit * (r.flip ^ 1), r.fit, (uint32_t)n, 0u, b->d_steps, r.status, kWaitNs};
+              r.bars + (size_t)32 * r.fit * (r.flip ^ 1), r.fit, (uint32_t)n, 0u, b->d_steps, r.status, nullptr, kWaitNs};
+    if (b->test_wait_ns) {
+        A.wait_ns = b->test_wait_ns;
+        b->test_wait_ns = 0;
+        if (resident_short(A.bars, b->stream)) return bfail(b, EMS_ERR_CUDA, "test hook");
+    }
     r.flip ^= 1;
     cudaError_t e;
     launch_resident(A, false, r.grid, kGangThreads, b->stream, &e);
@@ -3840,7 +3864,15 @@ ems_status ems_batch_download_field(ems_batch* b, size_t model, int field, int a
     if (!b || model >= b->models.size()) return EMS_ERR_INVALID;
     cudaSetDevice(b->device);
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return bfail(b, EMS_ERR_CUDA, "download");
-    return ems_gpu_download_field(b->models[model], field, axis, host);
+    const ems_status waited = batch_status(b);
+    const ems_status st = ems_gpu_download_field(b->models[model], field, axis, host);
+    return waited ? waited : st;
+}
+
+ems_status ems_batch_test_wait_timeout(ems_batch* b, uint64_t limit_ns) {
+    if (!b || !limit_ns || limit_ns > 10000000000ull) return EMS_ERR_INVALID;
+    b->test_wait_ns = limit_ns;
+    return EMS_OK;
 }
 
 ems_status ems_batch_stream(const ems_batch* b, void** stream) {

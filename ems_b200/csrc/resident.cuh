@@ -16,7 +16,7 @@
 // amplitude tables and sample buffers on the device. Fields change within
 // the launch, so they are read through the coherent path, never __ldg.
 //
-// A barrier wait is bounded: after kWaitNs the block sets the status flag and
+// A barrier wait is bounded: after wait_ns the block sets the status flags and
 // leaves the kernel, and so do the others of its gang when their waits end.
 #pragma once
 
@@ -91,6 +91,7 @@ struct ResArgs {
     uint32_t step0;          // first step (steps null)
     uint32_t* steps;         // per model: completed steps (advanced), or null
     int* status;
+    int* told;               // the same flag in host memory, or null
     uint64_t wait_ns;
 };
 
@@ -118,10 +119,8 @@ inline uint64_t global_ns() { return 0; }
 struct Gang {
     uint32_t* bar;
     uint32_t size, epoch;
-    int* status;
-    uint64_t wait_ns;
 };
-__device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
+__device__ __forceinline__ bool gang_sync(Gang& G, const ResArgs& A, int* ok) {
     __syncthreads();
     if (G.size == 1) return true;
     ++G.epoch;
@@ -134,8 +133,9 @@ __device__ __forceinline__ bool gang_sync(Gang& G, int* ok) {
             if ((it & 255u) != 255u) continue;
             const uint64_t now = global_ns();
             if (!t0) t0 = now;
-            if (now - t0 > G.wait_ns) {
-                atomicExch(G.status, 1);
+            if (now - t0 > A.wait_ns) {
+                atomicExch(A.status, 1);
+                if (A.told) *(volatile int*)A.told = 1;
                 *ok = 0;
                 break;
             }
@@ -282,7 +282,7 @@ __device__ __forceinline__ void res_update(const ResModel& R, uint32_t t, uint32
 // The slab hooks of one side after its update, each followed by a barrier of
 // the gang; false once a wait has run out.
 template <int SIDE>
-__device__ __forceinline__ bool res_slabs(const ResModel& R, Gang& G, uint32_t rank, int* ok) {
+__device__ __forceinline__ bool res_slabs(const ResModel& R, const ResArgs& A, Gang& G, uint32_t rank, int* ok) {
     const uint32_t t = rank * blockDim.x + threadIdx.x, stride = G.size * blockDim.x;
     for (int q = 0; q < 2 && R.order[q] >= 0; ++q) {
         if (R.order[q] == 0) {
@@ -294,7 +294,7 @@ __device__ __forceinline__ bool res_slabs(const ResModel& R, Gang& G, uint32_t r
             if (!p.n_edges) continue;
             res_poles(R, SIDE == 1, t, stride);
         }
-        if (!gang_sync(G, ok)) return false;
+        if (!gang_sync(G, A, ok)) return false;
     }
     return true;
 }
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
     EMS_GANG_SHARED int ok;
     const ResModel& R = *reinterpret_cast<const ResModel*>(raw);
     const uint4 b = A.blocks[blockIdx.x];
-    Gang G{A.bars + b.x * 32u, b.z, 0u, A.status, A.wait_ns};
+    Gang G{A.bars + b.x * 32u, b.z, 0u};
     const uint32_t rank = b.y;
     if (blockIdx.x == 0)
         for (uint32_t w = threadIdx.x; w < A.n_bars; w += blockDim.x) A.bars_next[w * 32u] = 0u;
@@ -346,21 +346,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
                 if (R.m.pe.n_edges && (!R.fold_e || (R.capture_first && s == 0))) res_capture(R, true, t, stride);
                 res_update<0, OE>(R, t, stride);
             }
-            if (!gang_sync(G, &ok)) return;
-            if (!res_slabs<0>(R, G, rank, &ok)) return;
+            if (!gang_sync(G, A, &ok)) return;
+            if (!res_slabs<0>(R, A, G, rank, &ok)) return;
             // Hooks that write i before the E update, in order with the current
             // probes; else the probes beside it.
             if (hooks) hook(false, step, true, true);
-            if (R.serial_h && !gang_sync(G, &ok)) return;
+            if (R.serial_h && !gang_sync(G, A, &ok)) return;
             if (!(apart && hooks)) {
                 if (R.m.ph.n_edges && !R.fold_h) res_capture(R, false, t, stride);
                 res_update<1, OE>(R, t, stride);
             }
-            if (!gang_sync(G, &ok)) return;
-            if (!res_slabs<1>(R, G, rank, &ok)) return;
+            if (!gang_sync(G, A, &ok)) return;
+            if (!res_slabs<1>(R, A, G, rank, &ok)) return;
             if (R.writes_e || (R.serial_e && !R.late_probes)) {
                 if (hooks) hook(true, step, !R.late_probes, true);
-                if (!gang_sync(G, &ok)) return;
+                if (!gang_sync(G, A, &ok)) return;
             }
         }
         if (R.late_probes && hooks && A.n) hook(true, step0 + A.n - 1u, true, false);

@@ -450,16 +450,22 @@ ems_status ems_gpu_set_interior_planes(ems_gpu* h, uint32_t planes);
  * since the last check (and clears them): EMS_ERR_TIMEOUT if a bounded wait
  * of the fused, marching or resident kernel ran out, EMS_ERR_DIVERGED if a marching
  * step wrote a non-finite field value (NaN or Inf). Field downloads, sample
- * reads and step_with_energy report the same at their end. This is the
+ * reads and step_with_energy report the same at their end (the newest sample's
+ * read the resident kernel's timeout alone, a series' count nothing). After a
+ * timeout the fields and the samples of the launch that gave up are not
+ * defined: for a resident launch up to 4096 steps, which the step and sample
+ * counts hold all the same. This is the
  * check at which device errors surface: stepping itself never fails, as in
  * the reference (src/engine/mod.rs:456-458; the run loop's Diverged outcome,
  * src/engine/run.rs:156-161). */
 ems_status ems_gpu_check(ems_gpu* h);
 
-/* Test hook of the bounded waits: the next marching step's first block
+/* Test hook of the bounded waits: in the next resident launch the gang's first
+ * barrier waits for one block more than there is (a gang of one block has no
+ * barrier); in the next marching step, if that comes first, the first block
  * expects 16 more bytes on its first ring barrier than its copies deliver
  * (every copy lands; the phase never completes) and its waits give up after
- * `limit_ns` nanoseconds (1 .. 10^10). That block then sets the timeout flag
+ * `limit_ns` nanoseconds (1 .. 10^10). The waiting block then sets the timeout flag
  * and returns; the step's result is not defined, and the next check returns
  * EMS_ERR_TIMEOUT. The handle and the device context stay usable. */
 ems_status ems_gpu_test_wait_timeout(ems_gpu* h, uint64_t limit_ns);
@@ -604,7 +610,8 @@ ems_status ems_batch_timestep(ems_batch* b, size_t model, uint64_t* n);
 /* A model's series as ems_gpu_samples (op: index into its descriptor's ops). */
 ems_status ems_batch_samples(ems_batch* b, size_t model, size_t op, int which, double* out, size_t cap, size_t* n);
 
-/* A model's field component in reference layout. */
+/* A model's field component in reference layout (EMS_ERR_TIMEOUT, after the
+ * copy, if a wait of the resident kernel ran out since the last check). */
 ems_status ems_batch_download_field(ems_batch* b, size_t model, int field, int axis, float* host);
 
 /* Picks the persistent grid of the batched kernels (one block per work
@@ -613,6 +620,10 @@ ems_status ems_batch_download_field(ems_batch* b, size_t model, int field, int a
  * next steps ems_batch_run takes (results do not depend on the grid) and
  * appending the pick to the file. No counterpart in the reference. */
 ems_status ems_batch_autotune(ems_batch* b, const char* cache_path);
+
+/* The test hook of ems_gpu_test_wait_timeout for the batch's next resident
+ * launch: the waits of its first gang run out. */
+ems_status ems_batch_test_wait_timeout(ems_batch* b, uint64_t limit_ns);
 
 /* The batch's CUDA stream (cudaStream_t). */
 ems_status ems_batch_stream(const ems_batch* b, void** stream);

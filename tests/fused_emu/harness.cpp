@@ -1026,7 +1026,7 @@ extern "C" int emu_resident_run(const ems_engine_desc* d, unsigned blocks, int d
     const uint32_t list = 0;
     uint32_t bars[64] = {};
     int status = 0;
-    ResArgs A{&R, bl.data(), &gang, &list, bars, bars + 32, 1u, (uint32_t)steps, 0u, nullptr, &status, 1u};
+    ResArgs A{&R, bl.data(), &gang, &list, bars, bars + 32, 1u, (uint32_t)steps, 0u, nullptr, &status, nullptr, 1u};
     blockDim = EmuDim{1, 1, 1};
     gridDim = EmuDim{blocks, 1, 1};
     emu::Block blk;

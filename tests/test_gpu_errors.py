@@ -5,6 +5,8 @@
   lands; the phase never completes), its waits give up after 20 ms, the
   block sets the timeout flag and returns. The next check reports
   EMS_ERR_TIMEOUT; the handle and the context stay usable.
+* The same of the resident kernel: its first barrier waits for a block more
+  than there is; every read reports it, once.
 * Divergence: a NaN uploaded into a field makes the next marching step write
   non-finite values; the next check reports EMS_ERR_DIVERGED, and the run
   loop ends with the Diverged outcome (src/engine/run.rs:156-161).
@@ -74,3 +76,52 @@ def test_run_loop_ends_diverged_on_nan():
     out = E.run_until(g, E.energy_decay_limits(2000, -40.0, w.model.dt))
     assert out.reason == 2  # Diverged
     assert out.checks == 1
+
+
+def _resident():
+    m = E.Model.uniform([40, 30, 33], [1e-3] * 3)
+    m.build(courant=0.95)
+    m.add_cpml([4] * 6)
+    src = m.add_source_table(E.SOFT_E, [(E.Z, (20, 15, 16), 1.0)], np.sin(0.3 * np.arange(100)))
+    return m, src, m.add_probe(E.VOLTAGE, [(E.Z, (21, 15, 16), 1.0)])
+
+
+@pytest.mark.parametrize("read", ["check", "last_sample", "samples", "field", "energy"])
+def test_resident_wait_runs_out_and_every_read_reports_it(read):
+    m, _, probe = _resident()
+    g = E.Engine(m)
+    g.run(3)
+    g.last_sample(probe)
+    g.test_wait_timeout(5_000_000)
+    g.run(2)
+    call = {"check": g.check, "last_sample": lambda: g.last_sample(probe), "samples": lambda: g.samples(probe),
+            "field": lambda: g.field(0, 2), "energy": g.step_with_energy}[read]
+    with pytest.raises(E.EngineError) as ei:
+        call()
+    assert ei.value.status == E.ERR_TIMEOUT
+    # Reported once; the handle and the device step on.
+    for _ in range(2):
+        g.run(2)
+        g.last_sample(probe)
+        call()
+    h, o = E.Engine(m), OracleEngine(m, threads=4)
+    h.run(30)
+    o.run(30)
+    h.check()
+    assert_fields_equal(h, o, "after a bounded wait ran out")
+
+
+@pytest.mark.parametrize("read", ["samples", "field", "energy"])
+def test_batch_wait_runs_out_and_every_read_reports_it(read):
+    m, _, probe = _resident()
+    b = E.Batch([m, m], max_steps=100)
+    b.run(3)
+    b.test_wait_timeout(5_000_000)
+    b.run(2)
+    call = {"samples": lambda: b.samples(0, probe), "field": lambda: b.field(0, 0, 2), "energy": b.step_with_energy}[read]
+    with pytest.raises(E.EngineError) as ei:
+        call()
+    assert ei.value.status == E.ERR_TIMEOUT
+    b.run(2)
+    call()
+    assert b.samples(1, probe).size == b.timestep(1)
