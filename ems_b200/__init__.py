@@ -295,6 +295,7 @@ GPU_SYMBOLS = {
     "ems_gpu_set_interior_planes": (C.c_int, [C.c_void_p, C.c_uint32]),
     "ems_gpu_set_march": (C.c_int, [C.c_void_p, C.c_int, C.c_uint32]),
     "ems_gpu_check": (C.c_int, [C.c_void_p]),
+    "ems_gpu_test_fail_alloc": (C.c_int, [C.c_void_p, C.c_uint64]),
     "ems_gpu_test_wait_timeout": (C.c_int, [C.c_void_p, C.c_uint64]),
     "ems_gpu_freq_dump_read": (C.c_int, [C.c_void_p, C.c_size_t, C.c_size_t, C.c_void_p, C.c_size_t]),
     "ems_batch_autotune": (C.c_int, [C.c_void_p, C.c_char_p]),
@@ -930,6 +931,10 @@ class Engine:
     def test_wait_timeout(self, limit_ns: int) -> None:
         """Arms the bounded-wait test hook for the next marching step or resident launch."""
         self._ck(self._lib.ems_gpu_test_wait_timeout(self._h, limit_ns))
+
+    def test_fail_alloc(self, n: int) -> None:
+        """Makes the engine's n-th device allocation from now on fail."""
+        self._ck(self._lib.ems_gpu_test_fail_alloc(self._h, n))
 
     def set_march(self, shape: int = 0, planes: int = 32) -> None:
         """The marching schedule's tile shape (0..3) and planes per block."""

@@ -217,6 +217,7 @@ struct ems_gpu {
         ResOp* dev = nullptr;
         std::vector<unsigned char> held;  // what the device table holds
         std::vector<int> place;           // per operator its place, -1: not in the table
+        bool stale = true;                // a buffer in the table has moved since its upload
         uint64_t ready = ~0ull;           // buffers and amplitudes hold the steps before this one
         bool late_h = false;              // no hook writes i: current probes wait for the electric hooks
         double* mail = nullptr;           // pinned, 3 per operator, then `told`
@@ -344,8 +345,11 @@ struct ems_gpu {
     char* arena = nullptr;
     size_t arena_used = 0;
 
+    uint64_t test_fail_alloc = 0;  // ems_gpu_test_fail_alloc: the n-th allocation from now fails
+
     template <class T>
     T* alloc(size_t n) {
+        if (test_fail_alloc && --test_fail_alloc == 0) return nullptr;
         const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
         if (bytes < kArenaMax) {
             const size_t need = (bytes + 255) & ~(size_t)255;
@@ -1526,12 +1530,15 @@ ems_status sync_amp(ems_gpu* h, const std::vector<T>& amp, ems_gpu::AmpDev<T>& d
 ems_status put_table(ems_gpu* h, std::vector<unsigned char>& held, void* dev, const void* host, size_t bytes) {
     if (held.size() == bytes && !std::memcmp(held.data(), host, bytes)) return EMS_OK;
     held.assign((const unsigned char*)host, (const unsigned char*)host + bytes);
-    return check(h, cudaMemcpyAsync(dev, held.data(), bytes, cudaMemcpyHostToDevice, h->stream), "resident tables");
+    const ems_status st = check(h, cudaMemcpyAsync(dev, held.data(), bytes, cudaMemcpyHostToDevice, h->stream), "resident tables");
+    if (st) held.clear();
+    return st;
 }
 
 // Makes the serial hooks ready for steps [step, step + n): room for their
-// samples (counted here), amplitudes on the device, and the table of hooks
-// uploaded again if a buffer has moved.
+// samples (counted here once there is room for all), amplitudes on the device,
+// and the table of hooks uploaded again if a buffer has moved, also in a call
+// that found no room for the next one.
 ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
     auto& k = h->hooks;
     if (k.ready == h->step + n) return EMS_OK;
@@ -1541,39 +1548,42 @@ ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
         std::memset(k.mail, 0, n * sizeof(double));
         k.told = (int*)(k.mail + n - 3);
     }
-    bool moved = k.held.empty();
     for (auto& op : h->ops) {
         ems_status st = EMS_OK;
         if (op.kind == EMS_OP_SOURCE && op.source.n <= kResidentEdges) {
             const float* was = op.source.amp_dev.p;
             st = sync_amp(h, op.source.amp, op.source.amp_dev, h->step, n);
-            moved |= was != op.source.amp_dev.p;
+            k.stale |= was != op.source.amp_dev.p;
         } else if (op.kind == EMS_OP_PROBE) {
             auto& p = op.probe;
             const uint64_t end = (h->step + n + p.interval - 1) / p.interval;
-            moved |= end > p.cap;
+            k.stale |= end > p.cap;
             st = grow(h, &p.values, p.count, &p.cap, end);
-            p.count = end;
         } else if (op.kind == EMS_OP_LUMPED) {
             auto& l = op.lumped;
             if (l.has_src) {
                 const double* was = l.amp_dev.p;
                 st = sync_amp(h, l.amp, l.amp_dev, h->step, n);
-                moved |= was != l.amp_dev.p;
+                k.stale |= was != l.amp_dev.p;
             }
             if (!st && l.record) {
                 const uint64_t end = h->step + n;
-                moved |= end > l.cap;
+                k.stale |= end > l.cap || (l.columns && end > std::min(l.vcap, l.icap));
                 st = grow(h, &l.rec, l.count, &l.cap, end);
                 if (!st && l.columns) st = grow(h, &l.pv, l.count, &l.vcap, end);
                 if (!st && l.columns) st = grow(h, &l.pi, l.count, &l.icap, end);
-                l.count = end;
             }
         }
         if (st) return st;
     }
-    k.ready = h->step + n;
-    if (!moved) return EMS_OK;
+    for (auto& op : h->ops) {
+        if (op.kind == EMS_OP_PROBE) op.probe.count = (h->step + n + op.probe.interval - 1) / op.probe.interval;
+        if (op.kind == EMS_OP_LUMPED && op.lumped.record) op.lumped.count = h->step + n;
+    }
+    if (!k.stale) {
+        k.ready = h->step + n;
+        return EMS_OK;
+    }
     std::vector<unsigned char> ops;
     for (size_t q = 0; q < h->ops.size(); ++q) {
         if (k.place[q] < 0) continue;
@@ -1600,7 +1610,11 @@ ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
         }
         ops.insert(ops.end(), raw, raw + sizeof(ResOp));
     }
-    return ops.empty() ? EMS_OK : put_table(h, k.held, k.dev, ops.data(), ops.size());
+    if (!ops.empty())
+        if (ems_status st = put_table(h, k.held, k.dev, ops.data(), ops.size())) return st;
+    k.stale = false;
+    k.ready = h->step + n;
+    return EMS_OK;
 }
 
 void launch_resident(const ResArgs& A, bool oe, unsigned grid, unsigned threads, cudaStream_t s, cudaError_t* e) {
@@ -1738,6 +1752,8 @@ ems_status run_resident(ems_gpu* h, uint64_t n) {
 // One step through the per-operator or split kernels; energy: record the
 // invariant's field part into d_energy[0].
 ems_status run_step(ems_gpu* h, bool energy) {
+    // Room for the samples first: a step is refused whole or not at all.
+    if (ems_status st = prepare_hooks(h, 1)) return st;
     const int sch = active_schedule(h);
     // Only the per-operator, split and sweep steps keep the electric saved values.
     if (sch != 4 && sch != 5 && sch != 6 && sch != 7) h->prev_e_valid = false;
@@ -3102,6 +3118,12 @@ ems_status ems_gpu_check(ems_gpu* h) {
 ems_status ems_gpu_test_wait_timeout(ems_gpu* h, uint64_t limit_ns) {
     if (!h || !limit_ns || limit_ns > 10000000000ull) return EMS_ERR_INVALID;
     h->test_wait_ns = limit_ns;
+    return EMS_OK;
+}
+
+ems_status ems_gpu_test_fail_alloc(ems_gpu* h, uint64_t n) {
+    if (!h) return EMS_ERR_INVALID;
+    h->test_fail_alloc = n;
     return EMS_OK;
 }
 

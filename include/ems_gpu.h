@@ -470,6 +470,10 @@ ems_status ems_gpu_check(ems_gpu* h);
  * EMS_ERR_TIMEOUT. The handle and the device context stay usable. */
 ems_status ems_gpu_test_wait_timeout(ems_gpu* h, uint64_t limit_ns);
 
+/* Test hook of running out of device memory: the handle's n-th allocation from
+ * now on fails (0: none). */
+ems_status ems_gpu_test_fail_alloc(ems_gpu* h, uint64_t n);
+
 /* The marching schedule's tile shape (0: 7 rows, 3 stages, two blocks per
  * SM; 1: 15 rows, 3 stages, one block; 2: 8 rows, 4 stages, one block; 3: 3
  * rows, 4 stages, three blocks) and the planes a block marches through (1

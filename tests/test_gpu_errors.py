@@ -125,3 +125,35 @@ def test_batch_wait_runs_out_and_every_read_reports_it(read):
     b.run(2)
     call()
     assert b.samples(1, probe).size == b.timestep(1)
+
+
+@pytest.mark.parametrize("schedule", [0, 4])
+@pytest.mark.parametrize("grown", [0, 1, 2, 3, 4])
+def test_no_room_for_samples_loses_none(schedule, grown):
+    """Memory runs out while the series grow (some of them moved already): the
+    run is refused before any of its steps, the counts stay, and steps that
+    need no more room go on with every sample in place."""
+    m, _, first = _resident()
+    amp = np.cos(0.1 * np.arange(50))
+    port = m.add_lumped_port_table(E.Y, [9, 9, 9], [9, 11, 9], 50.0, amp)
+    second = m.add_probe(E.CURRENT, [(E.X, (20, 15, 16), 1.0)])
+    series = [(first, 0), (port, 0), (port, 1), (port, 2), (second, 0)]
+    g, want = E.Engine(m), E.Engine(m)
+    for e in (g, want):
+        e.set_schedule(schedule)
+        e.run(1000)  # series hold 1024 samples
+    if schedule:
+        g.run(24)
+        want.run(24)
+    g.test_fail_alloc(1 + grown)
+    with pytest.raises(E.EngineError) as ei:
+        g.run(30)
+    assert ei.value.status == E.ERR_NOMEM
+    assert g.timestep == want.timestep and all(g.samples(*q).size == g.timestep for q in series)
+    for n in (20, 60):
+        g.run(n)
+        want.run(n)
+        for q in series:
+            x, y = g.samples(*q), want.samples(*q)
+            assert x.size == y.size == g.timestep and np.array_equal(x.view(np.uint64), y.view(np.uint64)), (n, q)
+    assert_fields_equal(g, want, "after running out of memory")
