@@ -234,6 +234,7 @@ struct ems_gpu {
     // split schedule on small grids, many steps per launch.
     struct Resident {
         bool ok = false;
+        uint64_t most = 0;                 // steps per launch
         std::vector<unsigned char> model;  // what the device table holds
         ResModel* d_model = nullptr;
         uint4* blocks = nullptr;
@@ -1350,7 +1351,15 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
 // split times before launch_next, which takes some 8 us off them.)
 constexpr size_t kResidentBytes = 256u << 20, kResidentPoleBytes = 32u << 20;
 constexpr size_t kResidentEdges = 4096;
-constexpr uint64_t kResidentSteps = 4096;  // most steps per launch
+// Most steps per launch, for models of up to 32 MB, and least ones: a launch
+// holds its SMs to the end, so that the kernels of other streams and engines
+// wait for it. With 4096 steps a small kernel waited 141 ms beside a 100^3 box
+// and 486 ms beside 180^3, now up to 5 ms; the launches more are not seen in the
+// time per step.
+constexpr uint64_t kResidentSteps = 128, kResidentLeast = 16;
+uint64_t resident_steps(size_t bytes) {
+    return std::min(kResidentSteps, std::max(kResidentLeast, kResidentSteps * (32u << 20) / (bytes + 1)));
+}
 
 size_t resident_bytes(const ems_gpu* h) {
     size_t b = 24 * h->g.np;
@@ -1705,6 +1714,7 @@ ems_status setup_resident(ems_gpu* h) {
     if (!h->status) h->status = h->alloc<int>(1);
     if (!r.blocks || !r.gangs || !r.list || !r.bars || !r.d_model || !h->status)
         return fail(h, EMS_ERR_NOMEM, "resident steps");
+    r.most = resident_steps(resident_bytes(h));
     r.ok = true;
     return check(h, cudaStreamSynchronize(h->stream), "resident steps");
 }
@@ -2581,7 +2591,7 @@ ems_status ems_gpu_run(ems_gpu* h, uint64_t n) {
     cudaSetDevice(h->device);
     for (uint64_t s = 0; s < n;) {
         const bool resident = use_resident(h);
-        const uint64_t k = resident ? std::min(n - s, kResidentSteps) : 1;
+        const uint64_t k = resident ? std::min(n - s, h->res.most) : 1;
         ems_status st = resident ? run_resident(h, k) : step_dumped(h, false);
         if (st) return st;
         s += k;
@@ -3232,6 +3242,8 @@ struct ems_batch {
     struct Resident {
         bool ok = false, stale = true;  // stale: the gangs are not those of the active models
         unsigned fit = 0, grid = 0;
+        uint64_t most = 0;              // steps per launch
+        size_t bytes = 0;               // of all models
         std::vector<uint64_t> quads;    // work of each model
         ResModel* models = nullptr;
         uint4* blocks = nullptr;
@@ -3573,6 +3585,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
             if (ems_status rs = resident_quads(h)) return rs;
         resident_model(h, rm[m]);
         b->res.quads.push_back(rm[m].quads);
+        b->res.bytes += resident_bytes(h);
         // Serial hooks: sources, probes, lumped elements (device tables).
         size_t op_i = 0;
         for (auto& op : h->ops) {
@@ -3691,6 +3704,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
         r.bars = b->alloc<uint32_t>((size_t)64 * r.fit);
         r.status = b->alloc<int>(1);
         if (!r.models || !r.blocks || !r.gangs || !r.list || !r.bars || !r.status) return EMS_ERR_NOMEM;
+        r.most = resident_steps(r.bytes);
         r.ok = true;
     }
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return EMS_ERR_CUDA;
@@ -3776,7 +3790,7 @@ ems_status ems_batch_run(ems_batch* b, uint64_t n) {
     cudaSetDevice(b->device);
     for (uint64_t q = 0; q < n; ++q) {
         if (b->res.ok && !b->tune.active) {
-            const uint64_t k = std::min(n - q, kResidentSteps);
+            const uint64_t k = std::min(n - q, b->res.most);
             ems_status st = batch_resident(b, k);
             if (st) return st;
             batch_count(b, k);

@@ -453,7 +453,7 @@ ems_status ems_gpu_set_interior_planes(ems_gpu* h, uint32_t planes);
  * reads and step_with_energy report the same at their end (the newest sample's
  * read the resident kernel's timeout alone, a series' count nothing). After a
  * timeout the fields and the samples of the launch that gave up are not
- * defined: for a resident launch up to 4096 steps, which the step and sample
+ * defined: for a resident launch up to 128 steps, which the step and sample
  * counts hold all the same. This is the
  * check at which device errors surface: stepping itself never fails, as in
  * the reference (src/engine/mod.rs:456-458; the run loop's Diverged outcome,

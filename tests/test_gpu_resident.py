@@ -169,6 +169,19 @@ def test_batch_of_more_models_than_blocks():
                 assert np.array_equal(b.field(q, f, a).view(np.uint32), g.field(f, a).view(np.uint32)), (q, f, a)
 
 
+def test_long_runs_are_cut_into_launches():
+    """A launch holds its SMs to its end: at most 128 steps each."""
+    m = _cavity((12, 9, 10))[0]
+    g, s = E.Engine(m), E.Engine(m)
+    for n, launches in ((1, 1), (128, 1), (129, 2), (1000, 8)):
+        before = g.launches
+        g.run(n)
+        assert g.launches - before == launches
+    s.set_schedule(4)
+    s.run(1258)
+    assert_fields_equal(g, s, "cut into launches")
+
+
 def test_large_grids_keep_the_split_kernels():
     w = W.vacuum_box(n=224, cpml=8, steps=10)
     g = E.Engine(w.model)
