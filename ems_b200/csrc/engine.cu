@@ -1341,15 +1341,26 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
 // ---- Resident steps (resident.cuh).
 
 // Most bytes of fields, dense coefficients, CPML and pole state a resident
-// model touches per step, and most edges of a source (or lumped element) that
-// one block applies alone. Measured on cubes, us per step resident / split:
-// vacuum with CPML 40 cells 22/35, 96 37/50, 160 (110 MB) 106/123, 200 (230
-// MB) 187/216; coefficients of every node 160 (260 MB) 129/141, 240 370/364.
-// The poles' correction runs better in its own kernel (trapezoidal media 64
-// cells 28/46, 96 (27 MB) 55/64, 128 (70 MB) 121/115), and so does the
-// openEMS PML's at nearly every size (24 34/26, 64 28/33, 96 68/59). (The
-// split times before launch_next, which takes some 8 us off them.)
-constexpr size_t kResidentBytes = 256u << 20, kResidentPoleBytes = 32u << 20;
+// model touches per step (with a CPML, without one, with poles; the poles'
+// correction runs better in its own kernel), most bytes of a batch's models
+// above the bound with poles, and most edges of a source (or lumped element)
+// that one block applies alone. Measured on cubes, us per step resident /
+// split:
+//   CPML   24 cells 20/24, 96 39/42, 160 (110 MB) 107/122, 208 (250 MB) 199/216,
+//          coefficients of every node 96 41/45, 160 136/143; beyond the bound
+//          still 1.05 at 240 to 256 cells, 0.98 at 288
+//   PEC    48 10/13, 96 19/22, 144 (73 MB) 41/47, 160 (100 MB) 75/70, 200 130/122
+//   poles  32 28/30, 64 27/38, 96 (27 MB) 55/56..61, 112 73/73..78, 120 97/85,
+//          128 (70 MB) 117/107; small ones 24 29/28, 16 33/27
+// and of batches as gangs / as graphs:
+//   CPML   8 x 96 241/338, 200 x 24 215/344, 4 x 200 dense 882/1040, 2 x 320
+//          1383/1460; PEC 8 x 160 530/592: gangs at every size measured
+//   poles  8 x 32 36/72, 40 x 64 795/884, 8 x 96 456/464, 2 x 128 (140 MB) 243/253;
+//          8 x 104 (272 MB) 568/550, 8 x 128 993/908, 2 x 160 447/412
+// openEMS's PML runs split at every size: 24 34/26, 64 28/33, 96 68/59 (the split
+// times before launch_next, which takes some 8 us off them).
+constexpr size_t kResidentBytes = 256u << 20, kResidentPecBytes = 96u << 20, kResidentPoleBytes = 32u << 20;
+constexpr size_t kGangPoleBytes = 160u << 20;
 constexpr size_t kResidentEdges = 4096;
 // Most steps per launch, for models of up to 32 MB, and least ones: a launch
 // holds its SMs to the end, so that the kernels of other streams and engines
@@ -1371,6 +1382,13 @@ size_t resident_bytes(const ems_gpu* h) {
         for (const PoleSideDev* p : {&op.poles.e, &op.poles.h}) b += 16 * p->n_poles + 21 * p->n_edges;
     }
     return b;
+}
+
+bool has_op(const ems_gpu* h, int kind) {
+    return std::any_of(h->ops.begin(), h->ops.end(), [=](const ems_gpu::Op& op) { return op.kind == kind; });
+}
+bool pole_model(const ems_gpu* h) {
+    return std::any_of(h->ops.begin(), h->ops.end(), [](const ems_gpu::Op& op) { return op.poles.e.n_edges || op.poles.h.n_edges; });
 }
 
 // Whether the model's operators can run resident: every hook one of those
@@ -1693,9 +1711,8 @@ ems_status setup_hooks(ems_gpu* h) {
 // that fit the device.
 ems_status setup_resident(ems_gpu* h) {
     auto& r = h->res;
-    bool poles = false;
-    for (const auto& op : h->ops) poles |= op.poles.e.n_edges || op.poles.h.n_edges;
-    if (!resident_ops(h) || resident_bytes(h) > (poles ? kResidentPoleBytes : kResidentBytes)) return EMS_OK;
+    const size_t bound = pole_model(h) ? kResidentPoleBytes : (has_op(h, EMS_OP_CPML) ? kResidentBytes : kResidentPecBytes);
+    if (!resident_ops(h) || resident_bytes(h) > bound) return EMS_OK;
     const unsigned fit = resident_blocks(h->device, kResThreads);
     if (!fit) return EMS_OK;
     const uint64_t quads = (uint64_t)h->g.nx * h->g.ny * ((h->g.nz + 3u) / 4u);
@@ -3513,6 +3530,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
     std::vector<BatchLumped> lum;
     std::vector<ResModel> rm(n_models);
     bool resident = true;
+    size_t pole_bytes = 0;  // of models with poles above the bound for an engine
     for (int k = 0; k < BK_KINDS; ++k) b->start[k].assign(1, 0u);
     int pf = -1;
     for (size_t m = 0; m < n_models; ++m) {
@@ -3580,12 +3598,10 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
         // Resident steps: the same tables; the saved values of the poles are
         // captured every step, as the batched kernels do.
         std::vector<ResOp> rops;
+        const size_t bytes = resident_bytes(h);
         resident = resident && resident_ops(h);
-        if (resident)
-            if (ems_status rs = resident_quads(h)) return rs;
-        resident_model(h, rm[m]);
-        b->res.quads.push_back(rm[m].quads);
-        b->res.bytes += resident_bytes(h);
+        b->res.bytes += bytes;
+        if (pole_model(h) && bytes > kResidentPoleBytes) pole_bytes += bytes;
         // Serial hooks: sources, probes, lumped elements (device tables).
         size_t op_i = 0;
         for (auto& op : h->ops) {
@@ -3658,6 +3674,13 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
         // The copies out of rops end before it goes.
         if (cudaStreamSynchronize(b->stream) != cudaSuccess) return EMS_ERR_CUDA;
     }
+    resident = resident && pole_bytes <= kGangPoleBytes;
+    for (size_t m = 0; m < n_models; ++m) {
+        if (resident)
+            if (ems_status rs = resident_quads(b->models[m])) return rs;
+        resident_model(b->models[m], rm[m]);
+        b->res.quads.push_back(rm[m].quads);
+    }
     b->poles_first = pf == 1;
     b->active.assign(n_models, 1);
     b->done.assign(n_models, 0);
@@ -3703,7 +3726,7 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
         r.list = b->alloc<uint32_t>(n_models);
         r.bars = b->alloc<uint32_t>((size_t)64 * r.fit);
         r.status = b->alloc<int>(1);
-        if (!r.models || !r.blocks || !r.gangs || !r.list || !r.bars || !r.status) return EMS_ERR_NOMEM;
+        if (!r.models || !r.blocks || !r.gangs || !r.list || !r.bars || !r.status) return EMS_ERR_NOMEM;  // below 1 MB
         r.most = resident_steps(r.bytes);
         r.ok = true;
     }

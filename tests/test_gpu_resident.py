@@ -190,6 +190,36 @@ def test_large_grids_keep_the_split_kernels():
     assert g.launches - before > 4 * 4
 
 
+@pytest.mark.parametrize("n,resident", [(138, True), (162, False)])
+def test_form_without_a_cpml(n, resident):
+    """96 MB of fields are the bound of PEC boxes (162^3: 100 MB)."""
+    g = E.Engine(_cavity((n, n, n))[0])
+    before = g.launches
+    g.run(4)
+    assert (g.launches - before == 1) == resident
+
+
+@pytest.mark.parametrize("n,gangs", [(72, True), (150, False)])
+def test_form_of_a_batch_with_poles(n, gangs):
+    """Large models with poles step by graph: no gang waits. Either way the
+    models equal the same ones alone."""
+    m = _poles((n, n, n), "electric", 1, 1)
+    b = E.Batch([m, m], max_steps=100)
+    s = E.Engine(m)
+    s.set_schedule(4)
+    b.run(7)
+    s.run(7)
+    for a in range(3):
+        assert np.array_equal(b.field(1, 0, a).view(np.uint32), s.field(0, a).view(np.uint32))
+    b.test_wait_timeout(5_000_000)
+    b.run(1)
+    if gangs:
+        with pytest.raises(E.EngineError):
+            b.field(0, 0, 2)
+    else:
+        b.field(0, 0, 2)
+
+
 def test_engines_on_several_threads():
     """Resident engines and a batch stepping at once from threads of their
     own (each launch fills the device): every result as when alone."""
