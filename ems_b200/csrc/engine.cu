@@ -1404,7 +1404,21 @@ bool resident_ops(const ems_gpu* h) {
     return true;
 }
 
-// The quad lists of a model whose CPML the resident updates apply.
+// Gives a model's quad lists back.
+void resident_drop(ems_gpu* h) {
+    cudaGetLastError();
+    cudaStreamSynchronize(h->stream);
+    for (int side = 0; side < 2; ++side) {
+        h->release((void*)h->cpml_layer[side]);
+        h->release((void*)h->cpml_inner[side]);
+        h->cpml_layer[side] = nullptr;
+        h->cpml_inner[side] = nullptr;
+        h->n_layer[side] = 0;
+    }
+}
+
+// The quad lists of a model whose CPML the resident updates apply. Without
+// room for them (EMS_ERR_NOMEM) nothing of them is kept.
 ems_status resident_quads(ems_gpu* h) {
     if (!h->cpml_first || h->cpml_inner[0]) return EMS_OK;
     const uint64_t nodes[3] = {h->g.nx, h->g.ny, h->g.nz};
@@ -1415,7 +1429,10 @@ ems_status resident_quads(ems_gpu* h) {
         h->n_layer[side] = (uint32_t)layer.size();
         h->cpml_layer[side] = h->upload(layer.data(), layer.size());
         h->cpml_inner[side] = h->upload(inner.data(), inner.size());
-        if (!h->cpml_layer[side] || !h->cpml_inner[side]) return fail(h, EMS_ERR_NOMEM, "resident steps");
+        if (!h->cpml_layer[side] || !h->cpml_inner[side]) {
+            resident_drop(h);
+            return fail(h, EMS_ERR_NOMEM, "resident steps");
+        }
         if (check(h, cudaStreamSynchronize(h->stream), "resident steps")) return EMS_ERR_CUDA;
     }
     return EMS_OK;
@@ -1716,7 +1733,8 @@ ems_status setup_resident(ems_gpu* h) {
     const unsigned fit = resident_blocks(h->device, kResThreads);
     if (!fit) return EMS_OK;
     const uint64_t quads = (uint64_t)h->g.nx * h->g.ny * ((h->g.nz + 3u) / 4u);
-    if (ems_status st = resident_quads(h)) return st;
+    // Without room for its tables the engine steps by the split kernels.
+    if (ems_status st = resident_quads(h)) return st == EMS_ERR_NOMEM ? EMS_OK : st;
     r.grid = (unsigned)std::min<uint64_t>(fit, std::max<uint64_t>(1, (quads + kResThreads - 1) / kResThreads));
     if (r.grid >= kHookGang) r.grid = std::min(fit, r.grid + 1u);  // one more for the hooks
     std::vector<uint4> blocks(r.grid);
@@ -1729,8 +1747,10 @@ ems_status setup_resident(ems_gpu* h) {
     r.bars = h->alloc<uint32_t>(64);
     r.d_model = h->alloc<ResModel>(1);
     if (!h->status) h->status = h->alloc<int>(1);
-    if (!r.blocks || !r.gangs || !r.list || !r.bars || !r.d_model || !h->status)
-        return fail(h, EMS_ERR_NOMEM, "resident steps");
+    if (!r.blocks || !r.gangs || !r.list || !r.bars || !r.d_model || !h->status) {
+        cudaGetLastError();
+        return EMS_OK;
+    }
     r.most = resident_steps(resident_bytes(h));
     r.ok = true;
     return check(h, cudaStreamSynchronize(h->stream), "resident steps");
@@ -3676,8 +3696,16 @@ ems_status ems_batch_create(const ems_engine_desc* const* descs, size_t n_models
     }
     resident = resident && pole_bytes <= kGangPoleBytes;
     for (size_t m = 0; m < n_models; ++m) {
-        if (resident)
-            if (ems_status rs = resident_quads(b->models[m])) return rs;
+        if (resident) {
+            const ems_status rs = resident_quads(b->models[m]);
+            if (rs == EMS_ERR_NOMEM) {
+                // No room: graphs, and the lists made so far are given back.
+                resident = false;
+                for (size_t q = 0; q < m; ++q) resident_drop(b->models[q]);
+            } else if (rs) {
+                return rs;
+            }
+        }
         resident_model(b->models[m], rm[m]);
         b->res.quads.push_back(rm[m].quads);
     }
