@@ -75,9 +75,9 @@ struct ems_gpu {
         bool active = false;
         std::string cache, key;
         std::vector<int> cand;
-        std::vector<double> ms;
+        std::vector<double> ms, steps;  // of each: timed steps and their time
         size_t at = 0;       // candidate being timed
-        int done = 0;        // steps of it run (the first is a warm-up)
+        uint64_t done = 0;   // steps of it run (the first is a warm-up)
         cudaEvent_t e0 = nullptr, e1 = nullptr;
     } tune;
     std::vector<std::unique_ptr<DevBuf>> bufs;
@@ -1756,12 +1756,12 @@ ems_status setup_resident(ems_gpu* h) {
     return check(h, cudaStreamSynchronize(h->stream), "resident steps");
 }
 
-// Whether the next steps (no energy, no dumps) run resident: the automatic
-// schedule, the plain step, and the step counter within the kernel's range.
-bool use_resident(const ems_gpu* h) {
-    return h->res.ok && h->schedule == 0 && !h->row_cpml_on && !h->profiling && !h->tune.active && h->dumps.empty() &&
-           h->tdumps.empty() && h->step < (1ull << 30);
+// Whether the next steps (no energy) can run resident: no dumps, and the step
+// counter within the kernel's range; and whether they do: the automatic schedule.
+bool can_resident(const ems_gpu* h) {
+    return h->res.ok && !h->row_cpml_on && !h->profiling && h->dumps.empty() && h->tdumps.empty() && h->step < (1ull << 30);
 }
+bool use_resident(const ems_gpu* h) { return h->schedule == 0 && !h->tune.active && can_resident(h); }
 
 ems_status run_resident(ems_gpu* h, uint64_t n) {
     auto& r = h->res;
@@ -2549,15 +2549,28 @@ static void tune_record(const std::string& path, const std::string& key, int val
     std::fclose(f);
 }
 
-constexpr int kTuneSteps = 4;  // per candidate: one warm-up step and three timed
+// Steps per candidate: one warm-up step, then the timed ones. The resident form
+// is timed over more, as it will run: many steps per launch.
+constexpr uint64_t kTuneSteps = 3, kTuneResident = 16;
 
-// One step of a tuning engine: the current candidate's schedule, timed.
-static ems_status tune_step(ems_gpu* h) {
+// The best candidate of a tuning by its time per step.
+static size_t tune_best(const std::vector<double>& ms, const std::vector<double>& steps) {
+    size_t best = 0;
+    for (size_t q = 1; q < ms.size(); ++q)
+        if (ms[q] / steps[q] < ms[best] / steps[best]) best = q;
+    return best;
+}
+
+// Up to `room` steps of a tuning engine in the current candidate's form (4: the
+// resident one where the automatic choice takes it), timed; *took: the steps.
+static ems_status tune_step(ems_gpu* h, uint64_t room, uint64_t* took) {
     auto& T = h->tune;
     h->schedule = T.cand[T.at];
-    const bool timed = T.done > 0;
+    const bool timed = T.done > 0, resident = h->schedule == 4 && can_resident(h);
+    const uint64_t last = 1 + (resident ? kTuneResident : kTuneSteps);
+    const uint64_t k = *took = timed && resident && T.done < last ? std::min(room, last - T.done) : 1;
     if (timed) cudaEventRecord(T.e0, h->stream);
-    ems_status st = run_step(h, false);
+    ems_status st = resident ? run_resident(h, k) : run_step(h, false);
     if (st) return st;
     if (timed) {
         cudaEventRecord(T.e1, h->stream);
@@ -2565,16 +2578,16 @@ static ems_status tune_step(ems_gpu* h) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, T.e0, T.e1);
         T.ms[T.at] += ms;
+        T.steps[T.at] += (double)k;
     }
-    if (++T.done == kTuneSteps) {
+    T.done += k;
+    if (T.done >= last) {
         T.done = 0;
         if (++T.at == T.cand.size()) {
-            size_t best = 0;
-            for (size_t q = 1; q < T.cand.size(); ++q)
-                if (T.ms[q] < T.ms[best]) best = q;
+            const size_t best = tune_best(T.ms, T.steps);
             // The split schedule: its resident form too, where the automatic choice takes it.
             h->schedule = T.cand[best] == 4 ? 0 : T.cand[best];
-            tune_record(T.cache, T.key, T.cand[best], T.ms[best] / (kTuneSteps - 1));
+            tune_record(T.cache, T.key, T.cand[best], T.ms[best] / T.steps[best]);
             T.active = false;
             cudaEventDestroy(T.e0);
             cudaEventDestroy(T.e1);
@@ -2616,9 +2629,10 @@ static ems_status dumps_sample(ems_gpu* h, uint64_t m, bool first) {
 // every step (Cursor::post_e).
 static ems_status step_dumped(ems_gpu* h, bool energy) {
     const bool any = !h->dumps.empty() || !h->tdumps.empty();
+    uint64_t took;
     ems_status st = any ? dumps_sample(h, h->step, true) : EMS_OK;
     if (st) return st;
-    st = (!energy && h->tune.active) ? tune_step(h) : run_step(h, energy);
+    st = (!energy && h->tune.active) ? tune_step(h, 1, &took) : run_step(h, energy);
     if (st) return st;
     return any ? dumps_sample(h, h->step, false) : EMS_OK;
 }
@@ -2628,8 +2642,10 @@ ems_status ems_gpu_run(ems_gpu* h, uint64_t n) {
     cudaSetDevice(h->device);
     for (uint64_t s = 0; s < n;) {
         const bool resident = use_resident(h);
-        const uint64_t k = resident ? std::min(n - s, h->res.most) : 1;
-        ems_status st = resident ? run_resident(h, k) : step_dumped(h, false);
+        uint64_t k = resident ? std::min(n - s, h->res.most) : 1;
+        ems_status st = resident                            ? run_resident(h, k)
+                        : h->tune.active && can_resident(h) ? tune_step(h, n - s, &k)
+                                                            : step_dumped(h, false);
         if (st) return st;
         s += k;
     }
@@ -2813,8 +2829,8 @@ ems_status ems_gpu_autotune(ems_gpu* h, const char* cache_path) {
     if (!h || !cache_path) return EMS_ERR_INVALID;
     auto& T = h->tune;
     char key[256];
-    std::snprintf(key, sizeof key, "engine %ux%ux%u ops=%zu tables=%d curl=%d", h->g.nx, h->g.ny, h->g.nz,
-                  h->ops.size(), h->tables_ok ? 1 : 0, h->oe_curl ? 1 : 0);
+    std::snprintf(key, sizeof key, "engine %ux%ux%u ops=%zu tables=%d curl=%d resident=%d", h->g.nx, h->g.ny, h->g.nz,
+                  h->ops.size(), h->tables_ok ? 1 : 0, h->oe_curl ? 1 : 0, h->res.ok ? 1 : 0);
     std::string k(key);
     for (auto& op : h->ops) k += "," + std::to_string(op.kind);
     T.key = k;
@@ -2835,6 +2851,7 @@ ems_status ems_gpu_autotune(ems_gpu* h, const char* cache_path) {
     if (h->tables_ok && h->march_why.empty()) T.cand.push_back(7);
     T.cand.push_back(1);
     T.ms.assign(T.cand.size(), 0.0);
+    T.steps.assign(T.cand.size(), 0.0);
     T.at = 0;
     T.done = 0;
     if (check(h, cudaEventCreate(&T.e0), "autotune") || check(h, cudaEventCreate(&T.e1), "autotune"))
@@ -3262,15 +3279,16 @@ struct ems_batch {
     unsigned grid[BK_KINDS] = {0, 0, 0, 0, 0};  // persistent grid per kind
     uint64_t resident[BK_KINDS] = {0, 0, 0, 0, 0};  // blocks resident at once per kind
     cudaGraphExec_t step_graph = nullptr, energy_graph = nullptr;
-    // Autotuning of the persistent grids (ems_batch_autotune): code 0 one
-    // block per work item, 1 the resident blocks, 2 half of them.
+    // Autotuning (ems_batch_autotune): the persistent grids of the step graph,
+    // code 0 one block per work item, 1 the resident blocks, 2 half of them; 3
+    // the gangs (recorded as 3 + the grid of the energy steps).
     struct Tune {
         bool active = false;
         std::string cache, key;
         std::vector<int> cand;
-        std::vector<double> ms;
+        std::vector<double> ms, steps;
         size_t at = 0;
-        int done = 0;
+        uint64_t done = 0;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
     } tune;
     int grid_code = 1;
@@ -3278,6 +3296,7 @@ struct ems_batch {
     // Resident steps (resident.cuh): a gang of blocks per active model.
     struct Resident {
         bool ok = false, stale = true;  // stale: the gangs are not those of the active models
+        bool use = true;                // plain steps run as gangs (autotuning may pick a graph)
         unsigned fit = 0, grid = 0;
         uint64_t most = 0;              // steps per launch
         size_t bytes = 0;               // of all models
@@ -3398,6 +3417,7 @@ ems_status batch_capture(ems_batch* b, bool energy, cudaGraphExec_t* out) {
     return EMS_OK;
 }
 
+constexpr int kTuneGangs = 3;          // autotuning's code of the gangs
 constexpr unsigned kGangThreads = 256;  // two blocks per SM: gangs of half an SM's grain
 
 // Gangs for the active models: with no more models than blocks, each block in
@@ -3780,36 +3800,52 @@ ems_status ems_batch_destroy(ems_batch* b) {
     return EMS_OK;
 }
 
-// One step of a tuning batch: the current candidate's graph, timed.
-static ems_status batch_tune_step(ems_batch* b) {
+// Up to `room` steps of a tuning batch in the current candidate's form, timed;
+// *took: the steps.
+static ems_status batch_tune_step(ems_batch* b, uint64_t room, uint64_t* took) {
     auto& T = b->tune;
-    if (b->grid_code != T.cand[T.at]) {
-        batch_grids(b, T.cand[T.at]);
+    const int cand = T.cand[T.at];
+    const bool timed = T.done > 0, gangs = cand == kTuneGangs;
+    if (!gangs && b->grid_code != cand) {
+        batch_grids(b, cand);
         ems_status st = batch_graphs(b);
         if (st) return st;
     }
-    const bool timed = T.done > 0;
+    const uint64_t last = 1 + (gangs ? kTuneResident : kTuneSteps);
+    const uint64_t k = *took = timed && gangs ? std::min(room, last - T.done) : 1;
     if (timed) cudaEventRecord(T.e0, b->stream);
-    if (cudaGraphLaunch(b->step_graph, b->stream) != cudaSuccess) return bfail(b, EMS_ERR_CUDA, "graph launch");
+    if (gangs) {
+        if (ems_status st = batch_resident(b, k)) return st;
+    } else if (cudaGraphLaunch(b->step_graph, b->stream) != cudaSuccess) {
+        return bfail(b, EMS_ERR_CUDA, "graph launch");
+    }
     if (timed) {
         cudaEventRecord(T.e1, b->stream);
         cudaEventSynchronize(T.e1);
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, T.e0, T.e1);
         T.ms[T.at] += ms;
+        T.steps[T.at] += (double)k;
     }
-    if (++T.done == kTuneSteps) {
+    T.done += k;
+    if (T.done >= last) {
         T.done = 0;
         if (++T.at == T.cand.size()) {
-            size_t best = 0;
-            for (size_t q = 1; q < T.cand.size(); ++q)
-                if (T.ms[q] < T.ms[best]) best = q;
-            tune_record(T.cache, T.key, T.cand[best], T.ms[best] / (kTuneSteps - 1));
+            const size_t best = tune_best(T.ms, T.steps);
+            b->res.use = T.cand[best] == kTuneGangs;
+            // The energy steps' grid: the best graph's, also beside gangs.
+            int grid = T.cand[best];
+            if (b->res.use) {
+                std::vector<double> graphs = T.ms;
+                graphs[best] = 1e30;
+                grid = T.cand[tune_best(graphs, T.steps)];
+            }
+            tune_record(T.cache, T.key, b->res.use ? kTuneGangs + grid : grid, T.ms[best] / T.steps[best]);
             T.active = false;
             cudaEventDestroy(T.e0);
             cudaEventDestroy(T.e1);
-            if (b->grid_code != T.cand[best]) {
-                batch_grids(b, T.cand[best]);
+            if (b->grid_code != grid) {
+                batch_grids(b, grid);
                 return batch_graphs(b);
             }
         }
@@ -3840,7 +3876,7 @@ ems_status ems_batch_run(ems_batch* b, uint64_t n) {
     if (!b) return EMS_ERR_INVALID;
     cudaSetDevice(b->device);
     for (uint64_t q = 0; q < n; ++q) {
-        if (b->res.ok && !b->tune.active) {
+        if (b->res.ok && b->res.use && !b->tune.active) {
             const uint64_t k = std::min(n - q, b->res.most);
             ems_status st = batch_resident(b, k);
             if (st) return st;
@@ -3849,8 +3885,12 @@ ems_status ems_batch_run(ems_batch* b, uint64_t n) {
             continue;
         }
         if (b->tune.active) {
-            ems_status st = batch_tune_step(b);
+            uint64_t k = 1;
+            ems_status st = batch_tune_step(b, n - q, &k);
             if (st) return st;
+            batch_count(b, k);
+            q += k - 1;
+            continue;
         } else if (cudaGraphLaunch(b->step_graph, b->stream) != cudaSuccess) {
             return bfail(b, EMS_ERR_CUDA, "graph launch");
         }
@@ -3865,20 +3905,23 @@ ems_status ems_batch_autotune(ems_batch* b, const char* cache_path) {
     cudaSetDevice(b->device);
     auto& T = b->tune;
     char key[256];
-    std::snprintf(key, sizeof key, "batch n=%zu blocks=%u,%u,%u,%u,%u", b->models.size(), b->start[0].back(),
-                  b->start[1].back(), b->start[2].back(), b->start[3].back(), b->start[4].back());
+    std::snprintf(key, sizeof key, "batch n=%zu blocks=%u,%u,%u,%u,%u gangs=%d", b->models.size(), b->start[0].back(),
+                  b->start[1].back(), b->start[2].back(), b->start[3].back(), b->start[4].back(), b->res.ok ? 1 : 0);
     T.key = key;
     T.cache = cache_path;
     int v = 0;
-    if (tune_lookup(T.cache, T.key, &v) && v >= 0 && v <= 2) {
+    if (tune_lookup(T.cache, T.key, &v) && v >= 0 && v < (b->res.ok ? 2 * kTuneGangs : kTuneGangs)) {
+        b->res.use = v >= kTuneGangs;
+        v %= kTuneGangs;
         if (v != b->grid_code) {
             batch_grids(b, v);
             return batch_graphs(b);
         }
         return EMS_OK;
     }
-    T.cand = {1, 0, 2};
+    T.cand = b->res.ok ? std::vector<int>{kTuneGangs, 1, 0, 2} : std::vector<int>{1, 0, 2};
     T.ms.assign(T.cand.size(), 0.0);
+    T.steps.assign(T.cand.size(), 0.0);
     T.at = 0;
     T.done = 0;
     if (cudaEventCreate(&T.e0) != cudaSuccess || cudaEventCreate(&T.e1) != cudaSuccess)

@@ -618,8 +618,9 @@ ems_status ems_batch_samples(ems_batch* b, size_t model, size_t op, int which, d
  * copy, if a wait of the resident kernel ran out since the last check). */
 ems_status ems_batch_download_field(ems_batch* b, size_t model, int field, int axis, float* host);
 
-/* Picks the persistent grid of the batched kernels (one block per work
- * item, the resident blocks, or half of them) for this batch's shape: from
+/* Picks gangs of blocks or the step graph for the plain steps, and the
+ * persistent grid of the batched kernels (one block per work item, the
+ * resident blocks, or half of them), for this batch's shape: from
  * `cache_path` if it holds the key, else by timing each candidate over the
  * next steps ems_batch_run takes (results do not depend on the grid) and
  * appending the pick to the file. No counterpart in the reference. */

@@ -258,3 +258,47 @@ def test_engines_on_several_threads():
     for q, e in enumerate(alone):
         assert b.timestep(q) == 600 and b.samples(q, 2).size == 200
         assert np.array_equal(b.field(q, 0, 2).view(np.uint32), e.field(0, 2).view(np.uint32))
+
+
+def test_autotuning_times_the_resident_form(tmp_path):
+    """The candidate of the split schedule is timed in the form that will run:
+    one warm-up step, then many steps per launch; the same for a batch."""
+    cache = str(tmp_path / "tune.txt")
+    m = _cavity((33, 20, 17), layers=4)[0]
+    g, s = E.Engine(m), E.Engine(m)
+    s.set_schedule(4)
+    g.autotune(cache)
+    for n, launches in ((1, 1), (9, 1), (7, 1)):
+        before = g.launches
+        g.run(n)
+        assert g.launches - before == launches
+    g.run(60)
+    s.run(77)
+    assert_fields_equal(g, s, "tuned")
+    key, pick, _ = open(cache).read().strip().rsplit(" ", 2)
+    assert key.startswith("engine ") and "resident=1" in key
+    h = E.Engine(m)
+    h.autotune(cache)
+    assert h.schedule == int(pick) == g.schedule
+    before = h.launches
+    h.run(40)
+    assert (h.launches - before == 1) == (int(pick) == 4)
+    b = E.Batch([m, m], max_steps=200)
+    b.autotune(cache)
+    b.test_wait_timeout(5_000_000)
+    b.run(1)
+    with pytest.raises(E.EngineError):
+        b.field(0, 0, 2)
+    b = E.Batch([m, m], max_steps=200)
+    b.autotune(cache)
+    for n in (20, 57):
+        b.run(n)
+    assert b.timestep(1) == 77
+    for a in range(3):
+        assert np.array_equal(b.field(1, 0, a).view(np.uint32), s.field(0, a).view(np.uint32))
+    line = open(cache).read().splitlines()[-1]
+    assert line.startswith("batch ") and "gangs=1" in line and 0 <= int(line.split()[-2]) < 6
+    c = E.Batch([m, m], max_steps=200)
+    c.autotune(cache)
+    c.run(77)
+    assert np.array_equal(c.field(0, 1, 2).view(np.uint32), s.field(1, 2).view(np.uint32))
