@@ -1531,7 +1531,7 @@ bool resident_op(const ems_gpu::Op& op, ResOp& o) {
         o.kind = ResOp::PROBE;
         o.electric = p.quantity == EMS_PROBE_VOLTAGE;
         o.probe = p.d;
-        o.interval = (uint32_t)std::min<uint64_t>(p.interval, ~0u);
+        o.interval = p.interval;
     } else if (op.kind == EMS_OP_LUMPED) {
         const auto& l = op.lumped;
         o.kind = ResOp::LUMPED;
@@ -1600,7 +1600,7 @@ ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
             k.stale |= was != op.source.amp_dev.p;
         } else if (op.kind == EMS_OP_PROBE) {
             auto& p = op.probe;
-            const uint64_t end = (h->step + n + p.interval - 1) / p.interval;
+            const uint64_t end = (h->step + n - 1) / p.interval + 1;
             k.stale |= end > p.cap;
             st = grow(h, &p.values, p.count, &p.cap, end);
         } else if (op.kind == EMS_OP_LUMPED) {
@@ -1621,7 +1621,7 @@ ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
         if (st) return st;
     }
     for (auto& op : h->ops) {
-        if (op.kind == EMS_OP_PROBE) op.probe.count = (h->step + n + op.probe.interval - 1) / op.probe.interval;
+        if (op.kind == EMS_OP_PROBE) op.probe.count = (h->step + n - 1) / op.probe.interval + 1;
         if (op.kind == EMS_OP_LUMPED && op.lumped.record) op.lumped.count = h->step + n;
     }
     if (!k.stale) {
@@ -1639,18 +1639,18 @@ ems_status prepare_hooks(ems_gpu* h, uint64_t n) {
         o.mail = k.mail + 3 * q;
         if (op.kind == EMS_OP_SOURCE) {
             o.amp = op.source.amp_dev.p;
-            o.n_amp = (uint32_t)op.source.amp_dev.cap;
+            o.n_amp = op.source.amp_dev.cap;
         } else if (op.kind == EMS_OP_PROBE) {
             o.values = op.probe.values;
-            o.cap = (uint32_t)std::min<size_t>(op.probe.cap, ~0u);
+            o.cap = op.probe.cap;
         } else {
             const auto& l = op.lumped;
             o.amp_l = l.amp_dev.p;
-            o.n_amp = (uint32_t)l.amp_dev.cap;
+            o.n_amp = l.amp_dev.cap;
             o.rec = l.record ? l.rec : nullptr;
             o.pv = l.columns ? l.pv : nullptr;
             o.pi = l.columns ? l.pi : nullptr;
-            o.cap = (uint32_t)std::min<size_t>(l.cap, ~0u);
+            o.cap = l.cap;
         }
         ops.insert(ops.end(), raw, raw + sizeof(ResOp));
     }
@@ -2076,7 +2076,7 @@ ems_status setup_sheet(ems_gpu* h, const ems_sheet* t, ems_gpu::Op& op) {
 // sides bit 0 the magnetic ones, bit 1 the electric ones.
 void run_hooks(ems_gpu* h, const Fields& f, int& lo, int hi, int sides, bool& acts) {
     if (acts && hi > lo) {
-        launch_next(h->stream, k_hooks, 1, 256, f, h->dt, h->hooks.dev + lo, (uint32_t)(hi - lo), (uint32_t)h->step, sides);
+        launch_next(h->stream, k_hooks, 1, 256, f, h->dt, h->hooks.dev + lo, (uint32_t)(hi - lo), h->step, sides);
         ++h->launches;
     }
     lo = hi;

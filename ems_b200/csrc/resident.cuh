@@ -43,8 +43,8 @@ __device__ __forceinline__ uint32_t quotient(const FastDiv& f, uint32_t n) { ret
 struct ResOp {
     enum Kind : int32_t { SOURCE = 0, PROBE = 1, LUMPED = 2 };
     int32_t kind, electric;      // of the field (SOURCE, PROBE)
-    uint32_t n, hard, n_amp, cap;
-    uint32_t interval, axis_l, has_src, pad;
+    uint32_t n, hard, axis_l, has_src;
+    uint64_t n_amp, cap, interval;
     const uint32_t* node;
     const uint8_t* axis;
     const float* weight;
@@ -172,9 +172,11 @@ __device__ __forceinline__ void probe_warp(const Fields& f, bool electric, const
 
 // The serial hooks of one field side at step `step`, by one block, in
 // registration order (probes: the probes; writers: the others); consecutive
-// probes take a warp each.
+// probes take a warp each. STEP: the resident kernel counts below 2^31 (and
+// takes probe intervals below that), the other steps in 64 bits.
+template <class STEP>
 __device__ __forceinline__ void serial_hooks(const Fields& f, double dt, const ResOp* ops, uint32_t n_ops, bool electric,
-                                             uint32_t step, bool probes, bool writers) {
+                                             STEP step, bool probes, bool writers) {
     for (uint32_t q = 0; q < n_ops;) {
         const ResOp& o = ops[q];
         const bool mine = (o.electric != 0) == electric && (o.kind == ResOp::PROBE ? probes : writers);
@@ -187,8 +189,8 @@ __device__ __forceinline__ void serial_hooks(const Fields& f, double dt, const R
             while (end < n_ops && ops[end].kind == ResOp::PROBE) ++end;
             for (uint32_t r = q + (threadIdx.x >> 5); r < end; r += blockDim.x >> 5) {
                 const ResOp& p = ops[r];
-                if ((p.electric != 0) != electric || step % p.interval) continue;
-                const uint32_t at = step / p.interval;
+                if ((p.electric != 0) != electric || step % (STEP)p.interval) continue;
+                const STEP at = step / (STEP)p.interval;
                 if (at < p.cap) probe_warp(f, electric, p.probe, p.values + at, p.mail);
             }
             q = end;
@@ -227,7 +229,7 @@ __device__ __forceinline__ void serial_pre(const Fields& f, const ResOp* ops, ui
 // the electric ones) instead of one each: six launches of 2.5 us on a box with
 // a source and five probes.
 __global__ void __launch_bounds__(256) k_hooks(const __grid_constant__ Fields f, double dt, const ResOp* ops, uint32_t n_ops,
-                                               uint32_t step, int sides) {
+                                               uint64_t step, int sides) {
     after_previous();
     if (sides & 1) serial_hooks(f, dt, ops, n_ops, false, step, true, true);
     if (sides & 2) serial_hooks(f, dt, ops, n_ops, true, step, true, true);

@@ -1065,3 +1065,37 @@ extern "C" int emu_resident_run(const ems_engine_desc* d, unsigned blocks, int d
             std::memcpy(fields[c] + r * g.nz, &buf[c][r * g.pitch], g.nz * 4);
     return 0;
 }
+
+// One launch of the serial hooks (k_hooks) at step `step` on a field of eight
+// zeros: a soft source of amplitudes 1..8 on node 2 and a probe of it with the
+// given interval and room for eight samples. values: the probe's samples (8).
+// Returns the field at node 2.
+extern "C" float emu_hooks_at(uint64_t step, uint64_t interval, double* values) {
+    float u[8] = {}, weight = 1.0f, amp[8];
+    for (int q = 0; q < 8; ++q) amp[q] = (float)(q + 1);
+    const uint32_t node = 2;
+    const uint8_t axis = 0;
+    const double w = 1.0;
+    ResOp ops[2] = {};
+    ops[0].kind = ResOp::SOURCE;
+    ops[0].electric = 1;
+    ops[0].n = 1;
+    ops[0].node = &node;
+    ops[0].axis = &axis;
+    ops[0].weight = &weight;
+    ops[0].amp = amp;
+    ops[0].n_amp = 8;
+    ops[1].kind = ResOp::PROBE;
+    ops[1].electric = 1;
+    ops[1].interval = interval;
+    ops[1].cap = 8;
+    ops[1].values = values;
+    ops[1].probe.n = 1;
+    ops[1].probe.axis = &axis;
+    ops[1].probe.node = &node;
+    ops[1].probe.weight = &w;
+    Fields f{};
+    f.u[0] = u;
+    emu_launch(1, 1, 1, 32, 1, [&] { k_hooks(f, 1.0, ops, 2, step, 3); });
+    return u[2];
+}

@@ -45,6 +45,8 @@ def emu_lib(asan=False):
     lib.emu_march_timeout.argtypes = [C.c_void_p, C.c_void_p, C.c_uint64]
     lib.emu_resident_run.restype = C.c_int
     lib.emu_resident_run.argtypes = [C.c_void_p, C.c_uint, C.c_int, C.c_int, C.c_uint64, C.c_void_p]
+    lib.emu_hooks_at.restype = C.c_float
+    lib.emu_hooks_at.argtypes = [C.c_uint64, C.c_uint64, C.c_void_p]
     lib.emu_pole_prev_fold.restype = C.c_int
     lib.emu_pole_prev_fold.argtypes = [C.c_void_p, C.c_int]
     lib.emu_error.restype = C.c_char_p
@@ -300,6 +302,20 @@ def test_resident_gang_equals_oracle(cpml, sides, fold):
         for name, a, b in zip(["u_x", "u_y", "u_z", "i_x", "i_y", "i_z"], arrs, want):
             bad = np.argwhere(a.view(np.uint32) != b.view(np.uint32))
             assert bad.size == 0, f"{blocks} blocks, down {down}, {name}: {len(bad)} differ, first {tuple(bad[0])}"
+
+
+@pytest.mark.parametrize("step", [0, 3, 7, 8, 2**31 + 1, 2**32, 2**32 + 3, 5 * 2**32 + 6])
+@pytest.mark.parametrize("interval", [1, 3, 2**32 - 1, 2**32, 2**32 + 3, 2**63])
+def test_serial_hooks_count_steps_in_64_bits(step, interval):
+    """After 2^32 steps no source starts again and no probe writes over its
+    first samples."""
+    values = np.full(8, -1.0)
+    u = emu_lib().emu_hooks_at(step, interval, values.ctypes.data)
+    assert u == (step + 1 if step < 8 else 0.0)
+    want = np.full(8, -1.0)
+    if step % interval == 0 and step // interval < 8:
+        want[step // interval] = u
+    assert np.array_equal(values, want)
 
 
 def test_pole_capture_fold_decision():
