@@ -1343,8 +1343,8 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
 // Most bytes of fields, dense coefficients, CPML and pole state a resident
 // model touches per step (with a CPML, without one, with poles; the poles'
 // correction runs better in its own kernel), most bytes of a batch's models
-// above the bound with poles, and most edges of a source (or lumped element)
-// that one block applies alone. Measured on cubes, us per step resident /
+// above the bound with poles, and most edges of a source that one block applies
+// alone (as many as a lumped element may have). Measured on cubes, us per step resident /
 // split:
 //   CPML   24 cells 20/24, 96 39/42, 160 (110 MB) 107/122, 208 (250 MB) 199/216,
 //          coefficients of every node 96 41/45, 160 136/143; beyond the bound
@@ -1398,7 +1398,6 @@ bool resident_ops(const ems_gpu* h) {
     for (const auto& op : h->ops) {
         if (op.kind == EMS_OP_MUR || op.kind == EMS_OP_SHEET || op.kind == EMS_OP_UPML) return false;
         if (op.kind == EMS_OP_SOURCE && op.source.n > kResidentEdges) return false;
-        if (op.kind == EMS_OP_LUMPED && op.lumped.n_edges > kResidentEdges) return false;
         if (op.kind == EMS_OP_PROBE && op.probe.interval >= (1ull << 31)) return false;
     }
     return true;
@@ -1706,16 +1705,15 @@ bool upml_own(const ems_engine_desc* d, int side) {
     return true;
 }
 
-// The table of the serial hooks one block can run (every probe; sources and
-// lumped elements of few edges), and the host mirror of the newest samples.
+// The table of the serial hooks one block can run (every probe and lumped
+// element; sources of few edges), and the host mirror of the newest samples.
 ems_status setup_hooks(ems_gpu* h) {
     auto& k = h->hooks;
     int n = 0;
     k.late_h = true;
     for (const auto& op : h->ops) {
         const bool fits = (op.kind == EMS_OP_SOURCE && op.source.n <= kResidentEdges) ||
-                          (op.kind == EMS_OP_LUMPED && op.lumped.n_edges <= kResidentEdges) ||
-                          op.kind == EMS_OP_PROBE;
+                          op.kind == EMS_OP_LUMPED || op.kind == EMS_OP_PROBE;
         k.place.push_back(fits ? n++ : -1);
         if (op.kind == EMS_OP_SHEET || (op.kind == EMS_OP_SOURCE && (op.source.kind == EMS_SOFT_H || op.source.kind == EMS_HARD_H)))
             k.late_h = false;
@@ -2135,13 +2133,8 @@ ems_status serial_pre_e(ems_gpu* h, const Fields& f) {
     bool acts = false;
     for (size_t q = 0; q < h->ops.size(); ++q) {
         auto& op = h->ops[q];
-        if (op.kind == EMS_OP_LUMPED && (op.lumped.record || op.lumped.has_branch)) {
-            if (h->hooks.place[q] >= 0) {
-                acts = true;
-                continue;
-            }
-            k_lumped_pre_e<<<blocks_for(op.lumped.n_edges, 128), 128, 0, h->stream>>>(f.u[op.lumped.axis], op.lumped.d);
-            ++h->launches;
+        if (op.kind == EMS_OP_LUMPED) {
+            acts |= op.lumped.record || op.lumped.has_branch;
         } else if (op.kind == EMS_OP_MUR && op.mur.n) {
             k_mur_save<<<blocks_for(op.mur.n, 256), 256, 0, h->stream>>>(f.u[0], f.u[1], f.u[2], op.mur);
             ++h->launches;
@@ -2181,15 +2174,6 @@ ems_status serial_post_e(ems_gpu* h, const Fields& f) {
                                                                                m.n_edges, m.n);
                 ++h->launches;
             }
-        } else if (op.kind == EMS_OP_LUMPED) {
-            run_hooks(h, f, lo, hi, sides, acts);
-            const ems_gpu::LumpedDev& L = op.lumped;
-            const double val = (L.has_src && h->step < L.amp.size()) ? L.amp[h->step] : 0.0;
-            const bool active = L.has_src && val != 0.0;
-            k_lumped_post_e<<<1, 256, 0, s>>>(f.u[L.axis], L.d, val, active ? 1 : 0, h->dt,
-                                              L.record ? L.rec + h->step : nullptr, L.columns ? L.pv + h->step : nullptr,
-                                              L.columns ? L.pi + h->step : nullptr, h->hooks.mail + 3 * q);
-            ++h->launches;
         } else if (op.kind == EMS_OP_SOURCE && !h_side) {
             run_hooks(h, f, lo, hi, sides, acts);
             run_source(h, op.source, f.u);
@@ -2299,7 +2283,7 @@ static ems_status create_engine(const ems_engine_desc* d, int device, bool alone
             const auto* l = (const ems_lumped*)t;
             auto& L = op.lumped;
             size_t ne = l->n_edges;
-            if (l->axis < 0 || l->axis > 2 || !ne || !l->node || !l->cb || !l->g_src || ne > 4096) return EMS_ERR_INVALID;
+            if (l->axis < 0 || l->axis > 2 || !ne || !l->node || !l->cb || !l->g_src || ne > kResidentEdges) return EMS_ERR_INVALID;
             std::vector<uint32_t> node(ne);
             for (size_t e = 0; e < ne; ++e) {
                 if (l->node[e] >= g.n) return EMS_ERR_INVALID;

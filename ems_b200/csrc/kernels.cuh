@@ -326,12 +326,6 @@ __device__ __forceinline__ void lumped_pre_e_edge(const float* u, const LumpedDe
     if (d.record) d.ru_prev[e] = x;
 }
 
-__global__ void k_lumped_pre_e(const float* u, LumpedDevT d) {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= d.n) return;
-    lumped_pre_e_edge(u, d, e);
-}
-
 // Lumped element post_e (src/engine/lumped.rs:1123-1236) and, for a port,
 // V = Σu/columns, I = −record (src/engine/port.rs:276-290). One block: the
 // per-edge updates and the terms of the sums in parallel, the sums in edge
@@ -421,11 +415,6 @@ __device__ __forceinline__ void lumped_post_e_block(float* u, const LumpedDevT& 
             mail[2] = -rec;
         }
     }
-}
-
-__global__ void __launch_bounds__(256) k_lumped_post_e(float* u, LumpedDevT d, double val, int active, double dt,
-                                                       double* rec_out, double* pv_out, double* pi_out, double* mail) {
-    lumped_post_e_block(u, d, val, active, dt, rec_out, pv_out, pi_out, mail);
 }
 
 // Σ ½·L·j² + ½·q²/C_p of the electric then the magnetic poles

@@ -76,3 +76,34 @@ def test_two_port_bit_exact():
     for p in (p1, p2):
         for which in (1, 2):
             _equal(g.samples(p, which), o.samples(p, which), f"port {p} {which}")
+
+
+@pytest.mark.parametrize("schedule", [0, 1])
+def test_large_sources_between_small_hooks(schedule):
+    """A source too large for the one launch of the serial hooks (4096 edges)
+    and an element of 3600 edges, registered between small ones: the hooks
+    before and behind them keep their places, and the newest samples follow the
+    series."""
+    n = (78, 76, 9)
+    m = E.Model.uniform(n, [1e-3] * 3)
+    m.build(courant=0.95)
+    amp = np.sin(0.2 * np.arange(120))
+    edges = [(E.X, (i, j, 6), 0.1 + 0.01 * ((i * j) % 7)) for i in range(2, 74) for j in range(2, 70)]
+    small = m.add_lumped(E.Z, [4, 4, 4], [4, 5, 6], r=40.0, record=True, amp=amp)
+    sheet = m.add_lumped_port_table(E.Z, [3, 3, 4], [62, 62, 5], 60.0, 0.5 * amp)
+    after = m.add_lumped(E.Z, [40, 30, 6], [40, 32, 7], r=70.0, l=3e-9, record=True)
+    m.add_source_table(E.SOFT_E, [(E.Z, (30, 30, 4), 1.0)], amp)
+    m.add_source_table(E.SOFT_E, edges, amp)
+    m.add_source_table(E.HARD_E, [(E.X, (20, 20, 6), 0.5)], amp)
+    v = m.add_probe(E.VOLTAGE, [(E.X, (20, 20, 6), 1.0), (E.Z, (30, 30, 4), -1.0)])
+    i = m.add_probe(E.CURRENT, [(E.X, (30, 29, 4), 1.0)], interval=2)
+    g, o = E.Engine(m), OracleEngine(m, threads=4)
+    g.set_schedule(schedule)
+    for steps in (1, 30, 1):
+        g.run(steps)
+        o.run(steps)
+    assert_fields_equal(g, o, "large hooks")
+    for op, which in [(small, 0), (sheet, 0), (sheet, 1), (sheet, 2), (after, 0), (v, 0), (i, 0)]:
+        x = g.samples(op, which)
+        _equal(x, o.samples(op, which), (op, which))
+        assert g.last_sample(op, which) == x[-1]
