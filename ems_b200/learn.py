@@ -282,7 +282,7 @@ class Net:
         self.forward(x)
         self._mse[0].p[1] = self._ptr(y)
         self._run(self._mse)
-        self.backward(self.grad)
+        self.backward(self.grad.view(x.shape[0], -1))
         self.adam(lr)
         return self.loss
 

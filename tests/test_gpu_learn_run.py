@@ -239,3 +239,4 @@ def test_backward_takes_gradients_of_other_types_and_places():
     for bad in (d[:4], d[:, :-1], t.cat([d, d])):
         with pytest.raises(RuntimeError):
             net.backward(bad)
+    net.train_step(t.zeros(3, L.K_IN, 2, device="cuda"), t.zeros(3, 2 * L.T_OUT, device="cuda"))
