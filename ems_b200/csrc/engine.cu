@@ -1362,14 +1362,14 @@ void launch_split_rows(ems_gpu* h, const FusedParams& P0, bool oe, cudaStream_t 
 constexpr size_t kResidentBytes = 256u << 20, kResidentPecBytes = 96u << 20, kResidentPoleBytes = 32u << 20;
 constexpr size_t kGangPoleBytes = 160u << 20;
 constexpr size_t kResidentEdges = 4096;
-// Most steps per launch, for models of up to 32 MB, and least ones: a launch
+// Most steps per launch, for models of up to 64 MB, and least ones: a launch
 // holds its SMs to the end, so that the kernels of other streams and engines
 // wait for it. With 4096 steps a small kernel waited 141 ms beside a 100^3 box
 // and 486 ms beside 180^3, now up to 5 ms; the launches more are not seen in the
 // time per step.
-constexpr uint64_t kResidentSteps = 128, kResidentLeast = 16;
+constexpr uint64_t kResidentSteps = 128, kResidentLeast = 32;
 uint64_t resident_steps(size_t bytes) {
-    return std::min(kResidentSteps, std::max(kResidentLeast, kResidentSteps * (32u << 20) / (bytes + 1)));
+    return std::min(kResidentSteps, std::max(kResidentLeast, kResidentSteps * (64u << 20) / (bytes + 1)));
 }
 
 size_t resident_bytes(const ems_gpu* h) {
@@ -2475,8 +2475,8 @@ static ems_status create_engine(const ems_engine_desc* d, int device, bool alone
     }
     if (alone) {
         if (h->has_upml)
-        for (int side = 0; side < 2; ++side) h->upml_fold[side] = upml_own(d, side);
-    if (ems_status st = setup_hooks(h.get())) return st;
+            for (int side = 0; side < 2; ++side) h->upml_fold[side] = upml_own(d, side);
+        if (ems_status st = setup_hooks(h.get())) return st;
         if (ems_status st = setup_resident(h.get())) return st;
     }
     if (check(h.get(), cudaStreamSynchronize(h->stream), "create")) return EMS_ERR_CUDA;

@@ -639,7 +639,10 @@ int gemm_job(Operand A, Operand B, Epilogue E, int M, int N, int K, Job& J) {
     E.wide = E.ldc % 8 == 0 && !(((uintptr_t)E.C | (uintptr_t)E.outf | (uintptr_t)E.outb) & 15);
     A.mode = operand_mode(A);
     B.mode = operand_mode(B);
-    const int ra = M >= TM ? TM : (M + 15) / 16 * 16, tn = N >= 128 ? 128 : (N + 15) / 16 * 16;
+    const int ra = M >= TM ? TM : (M + 15) / 16 * 16;
+    // Narrower tiles while half of the SMs have none.
+    int tn = N >= 128 ? 128 : (N + 15) / 16 * 16;
+    while (tn > 32 && tn % 32 == 0 && ((M - 1) / TM + 1) * (int64_t)((N - 1) / tn + 1) < 74) tn /= 2;
     const int chunks = (K - 1) / TK + 1, fit = (int)(kStageBytes / (chunk_bytes(ra) + chunk_bytes(tn)));
     // A stage holds up to four chunks, where three stages of it fit: handing one
     // over costs as much as the copies and products of a small chunk.
