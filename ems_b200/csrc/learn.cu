@@ -31,11 +31,10 @@ namespace {
 // other sizes: a batch's rows come out bit for bit as each would alone, and K
 // is not shared out over the chip. Shares added in f32 gave other bits, with an
 // error against f64 up to 3 % larger. The chain of one CTA bounds the small
-// matrices: 0.18 us per chunk for the products, and about as much again for
-// copies and hand-over that they do not hide (32x16 over 32704 rows: 158 us,
-// 64x256 over 8064: 54 us, 32x64 over 3840: 25 us; with two stages filled
-// through registers 1100, 300 and 160 us). The weight gradients therefore share
-// a launch (Jobs).
+// matrices: 0.25 us per chunk for the products alone, 0.27 with copies and
+// hand-over (32x16 over 32704 rows: 138 us, 64x256 over 8064: 39 us, 32x64 over
+// 3840: 21 us; with two stages filled through registers 1100, 300 and 160 us).
+// The weight gradients therefore share a launch (Jobs).
 //
 // An operand is copied in vectors along whichever index is contiguous (mode 1:
 // k; mode 2: the row or column), into 8×8 core matrices without swizzle that
@@ -386,7 +385,20 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_tc(const __grid_consta
         ok = feeders(J.B, n0, N, tn, t, smem_addr(smem) + size_a, size, K, stages, deep, full, empty);
     } else if (lane == 0) {
         const uint32_t id = inst_desc((uint32_t)tn, J.A.mode == 2, J.B.mode == 2);
-        const uint32_t step_a = k_step(ra), step_b = k_step(tn);
+        // The descriptors of stage 0; places further on are added in units of 16
+        // bytes (all of shared memory fits the address field).
+        const uint32_t a0 = smem_addr(smem), step_a = k_step(ra) >> 3, step_b = k_step(tn) >> 3;
+        const uint64_t da0 = smem_desc(a0, k_step(ra), kGroup), db0 = smem_desc(a0 + size_a, k_step(tn), kGroup);
+        uint32_t acc = 0;
+        auto product = [&](uint32_t a, uint32_t b) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                "l"(da0 + a), "l"(db0 + b), "r"(id), "r"(acc)
+                : "memory");
+            acc = 1u;
+        };
         int sg = 0;
         uint32_t round = 0;
         for (int ch = 0; ch < chunks;) {
@@ -400,18 +412,13 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_tc(const __grid_consta
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int d = 0; d < deep && ch < chunks; ++d, ++ch) {
-                const uint32_t a0 = smem_addr(smem) + (uint32_t)(sg * deep + d) * size, b0 = a0 + size_a;
-                const int steps = (min(TK, K - ch * TK) + 15) / 16;
-                for (int s = 0; s < steps; ++s) {
-                    const uint64_t da = smem_desc(a0 + s * 2 * step_a, step_a, kGroup);
-                    const uint64_t db = smem_desc(b0 + s * 2 * step_b, step_b, kGroup);
-                    const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                        "l"(da), "l"(db), "r"(id), "r"(acc)
-                        : "memory");
+                const uint32_t at = (uint32_t)(sg * deep + d) * (size >> 4);
+                const int left = K - ch * TK;
+                if (left >= TK) {
+#pragma unroll
+                    for (uint32_t s = 0; s < TK / 16; ++s) product(at + s * step_a, at + s * step_b);
+                } else {
+                    for (uint32_t s = 0; s < (uint32_t)(left + 15) / 16; ++s) product(at + s * step_a, at + s * step_b);
                 }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
