@@ -1365,7 +1365,7 @@ constexpr size_t kResidentEdges = 4096;
 // Most steps per launch, for models of up to 64 MB, and least ones: a launch
 // holds its SMs to the end, so that the kernels of other streams and engines
 // wait for it. With 4096 steps a small kernel waited 141 ms beside a 100^3 box
-// and 486 ms beside 180^3, now up to 5 ms; the launches more are not seen in the
+// and 486 ms beside 180^3, now up to 7 ms; the launches more are not seen in the
 // time per step.
 constexpr uint64_t kResidentSteps = 128, kResidentLeast = 32;
 uint64_t resident_steps(size_t bytes) {

@@ -581,10 +581,11 @@ ems_status ems_gpu_freq_dump_read(ems_gpu* h, size_t id, size_t k, double* out, 
  * Simulation::run (src/sim/mod.rs:1044) once per model. A batch builds
  * every model as ems_gpu_create does and steps them together on one device:
  * many steps per launch, a gang of blocks per model sized by its cells, or,
- * for energy steps and models with more edges in a source than one block can
- * drive, one CUDA graph per step (each kernel kind of the split schedule once
- * over all models, a packed per-model block table walked by a persistent
- * grid). The serial hooks run from device-side step counters. Each model's fields, probe and port series equal those of the
+ * for energy steps, large models with poles and models with more edges in a
+ * source than one block can drive, one CUDA graph per step (each kernel kind
+ * of the split schedule once over all models, a packed per-model block table
+ * walked by a persistent grid). The serial hooks run from device-side step
+ * counters. Each model's fields, probe and port series equal those of the
  * same model run alone bit for bit. A model needs the split schedule's
  * tables, its post_e hooks in the order lumped elements, E sources, voltage
  * probes and its post_h hooks in the order H sources, current probes, and
