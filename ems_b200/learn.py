@@ -150,7 +150,7 @@ class Net:
         self.W = param_views(self.p, k_in, t_out)
         self.Wb = param_views(self.pb, k_in, t_out)
         self.G = param_views(self.g, k_in, t_out)
-        self.dy = []  # the layers' gradients in f32
+        self.dy = []  # the layers' gradients in f32 and their partial column sums
         self._buf_b = -1
 
     # -- plumbing
@@ -185,11 +185,13 @@ class Net:
         return self._cmd(GEMM, (M, N, K, act, pa, pb, int(join)), (*sa, *sb, N if ldc is None else ldc, ba, bb),
                          (A, B, C, bias, outb, outf))
 
-    def _dy(self, y, da, dyb, db, rows, cols, act, conv=None):
-        """bf16(da·act'(y)) and the bias gradient; conv (T, k, s): da through the adjoint of im2col."""
+    def _dy(self, y, da, dyb, db, rows, cols, act, conv=None, later=False):
+        """bf16(da·act'(y)) and the bias gradient (later: at the end of the list); conv (T, k, s): da through the
+        adjoint of im2col."""
         T, k, st = conv or (0, 0, 0)
-        self.dy.append(self.torch.empty(rows * cols, dtype=self.torch.float32, device=self.dev))
-        return self._cmd(DY, (rows, cols, act, T, k, st), (), (y, da, dyb, self.dy[-1], db))
+        f32 = dict(dtype=self.torch.float32, device=self.dev)
+        self.dy.append((self.torch.empty(rows * cols, **f32), self.torch.empty(256 * cols, **f32)))
+        return self._cmd(DY, (rows, cols, act, T, k, st, int(later)), (), (y, da, dyb, self.dy[-1][0], db, self.dy[-1][1]))
 
     def _bufs(self, B: int):
         """Activation buffers and the launch lists for batch size B."""
@@ -221,14 +223,14 @@ class Net:
                               outf=self.out))
 
         # The gradients of the layers' outputs, last to first: fc2 (identity activation), fc1, the convolutions.
-        bwd = [self._dy(None, None, self.dy5_b, self.G[4][1], B, no, 0),
+        bwd = [self._dy(None, None, self.dy5_b, self.G[4][1], B, no, 0, later=True),
                self._gemm(self.dy5_b, (no, 1), self.Wb[4][0], (HIDDEN, 1), B, HIDDEN, no, self.da4),
-               self._dy(self.y4, self.da4, self.dy4_b, self.G[3][1], B, HIDDEN, 1),
+               self._dy(self.y4, self.da4, self.dy4_b, self.G[3][1], B, HIDDEN, 1, later=True),
                self._gemm(self.dy4_b, (HIDDEN, 1), self.Wb[3][0], (flat, 1), B, flat, HIDDEN, self.da3)]
         da, conv = self.da3, None
         for q in range(len(CONVS) - 1, -1, -1):
             ci, co, k, st = CONVS[q]
-            bwd.append(self._dy(self.ys[q], da, self.dyb[q], self.G[q][1], rows[q], co, 1, conv))
+            bwd.append(self._dy(self.ys[q], da, self.dyb[q], self.G[q][1], rows[q], co, 1, conv, later=True))
             if q:
                 bwd.append(self._gemm(self.dyb[q], (co, 1), self.Wb[q][0], (k * ci, 1), rows[q], k * ci, co,
                                       self.dcols[q]))

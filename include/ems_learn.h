@@ -50,7 +50,8 @@ int ems_learn_gemm_bf16(const uint16_t* A, int64_t sa0, int64_t sa1, const uint1
  *  DY       dy = da (p[1]) * act'(y (p[0])) (i[2] as above) to p[3], bf16(dy) to
  *           p[2] and its column sums (as ems_learn_bias_grad) to p[4]; rows i[0],
  *           cols i[1]. i[4] > 0: da is the adjoint of im2col of p[1] (kernel i[4],
- *           stride i[5], T = i[3]; rows = B*T).
+ *           stride i[5], T = i[3]; rows = B*T). p[5]: 256 * cols floats of its own.
+ *           i[6] != 0: the sums may come last in the list.
  *  MSE      as ems_learn_mse: p out, target, grad, loss; s n.
  * Every element of a GEMM is one sum over k in order, so the rows of a batch
  * come out as each would alone. */

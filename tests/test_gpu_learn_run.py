@@ -174,6 +174,21 @@ def test_bias_gradient_is_summed_as_bias_grad(net, rows, cols):
     assert np.array_equal(_bits(S), _bits(want))
 
 
+def test_bias_gradients_put_off_to_the_end_of_the_list(net):
+    """Eight of them: six in one launch, two in the next; uneven matrices."""
+    t = net.torch
+    rng = np.random.default_rng(3)
+    shapes = [(1, 1), (300, 33), (64, 768), (4097, 64), (255, 8), (256, 31), (1000, 7), (513, 129)]
+    d = [t.from_numpy(rng.standard_normal(s).astype(np.float32)).cuda() for s in shapes]
+    S = [t.empty(s[1], device="cuda") for s in shapes]
+    H = [t.empty(s, dtype=t.int16, device="cuda") for s in shapes]
+    _run(net, *[net._dy(None, d[q], H[q], S[q], *shapes[q], 0, later=True) for q in range(8)])
+    for q, (rows, cols) in enumerate(shapes):
+        want = t.empty(cols, device="cuda")
+        assert net.lib.ems_learn_bias_grad(net._ptr(d[q]), net._ptr(want), rows, cols, net._s()) == 0
+        assert np.array_equal(_bits(S[q]), _bits(want)), (rows, cols)
+
+
 @pytest.mark.parametrize("n", [1, 1025, 49152, 100001])
 def test_loss_is_summed_as_mse(net, n):
     from ems_b200 import learn as L
